@@ -24,6 +24,7 @@
 #include "cxg_kernels.h"
 #include "cxg_layout.h"
 #include "cxg_tc.cuh"
+#include "cxg_tiles.cuh"
 
 namespace cxg {
 
@@ -421,455 +422,28 @@ static __device__ double kktResidual(Ctx& c, const DevSettings& st, const double
 // ------------------------------------------------------------------------------------------
 // dense LDL' of the tiled root (no pivoting) and its solve
 // ------------------------------------------------------------------------------------------
-// Right-looking over 32-wide tile columns J:
-//   (1) one warp factors the diagonal tile (rows in registers, shuffles), stores L (lower),
-//       D (diagonal) and Linv^T (upper half) of the tile;
-//   (2) warps compute the off-diagonal tiles L_IJ = A_IJ Linv_JJ^T D_J^-1;
-//   (3) warps apply the trailing updates A_IK -= L_IJ D_J L_KJ^T, one tile pair per warp.
-// Three barriers per tile column. Pivot rules: QDLDL (qdldl_ldlt.cpp:64-68) fails on an exact
-// zero pivot; REGULARIZED (regularized_ldlt.cpp:132-139, 251-253) corrects a pivot below eps with
-// the expected sign (+ on x rows, - on Zero-cone rows) and fails if > 5% were corrected.
+// Right-looking over 32-wide tile columns J (tile operations in cxg_tiles.cuh). Pivot rules: QDLDL
+// (qdldl_ldlt.cpp:64-68) fails on an exact zero pivot; REGULARIZED (regularized_ldlt.cpp:132-139,
+// 251-253) corrects a pivot below eps with the expected sign (+ on x rows, - on Zero-cone rows)
+// and fails if > 5% were corrected.
 
-// Pivot statistics written by the factoring warp (shared memory, read after a barrier).
-struct PivotStats {
-  int nreg, zero, wrong, pad;
-  double minAbs;
-};
+// Warps that factor the diagonal tile together in a block of nw warps; with eight warps the other
+// four start on the trailing products at once.
+__device__ __forceinline__ int diagWarps(int nw) { return nw >= 8 ? 4 : min(nw, 2); }
 
-template <typename T>
-__device__ __forceinline__ T shflT(T v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-__device__ __forceinline__ df64 shflT(df64 v, int src) {
-  return df64(__shfl_sync(0xffffffffu, v.hi, src), __shfl_sync(0xffffffffu, v.lo, src));
-}
-// c + a b and c - a b in the tile arithmetic (one FMA for float/double, the fused double-float form)
-template <typename T>
-__device__ __forceinline__ T madT(T c, T a, T b) { return c + a * b; }
-__device__ __forceinline__ df64 madT(df64 c, df64 a, df64 b) { return dfMad(c, a, b); }
-template <typename T>
-__device__ __forceinline__ T msubT(T c, T a, T b) { return c - a * b; }
-__device__ __forceinline__ df64 msubT(df64 c, df64 a, df64 b) { return dfMad(c, -a, b); }
-// Accumulation inside tile products: accT (no renormalisation for double-float), then accEnd.
-template <typename T>
-__device__ __forceinline__ T accT(T c, T a, T b) { return c + a * b; }
-__device__ __forceinline__ df64 accT(df64 c, df64 a, df64 b) { return dfMadLoose(c, a, b); }
-template <typename T>
-__device__ __forceinline__ T accEnd(T c) { return c; }
-__device__ __forceinline__ df64 accEnd(df64 c) { return dfNorm(c); }
-
-// A row of 32 values held in registers (indices are compile-time after unrolling). The
-// double-float row is kept as two float arrays so that it stays in registers.
-template <typename T>
-struct Row32 {
-  T v[32];
-  __device__ __forceinline__ T get(int k) const { return v[k]; }
-  __device__ __forceinline__ void set(int k, T x) { v[k] = x; }
-};
-template <>
-struct Row32<df64> {
-  float h[32], l[32];
-  __device__ __forceinline__ df64 get(int k) const { return df64(h[k], l[k]); }
-  __device__ __forceinline__ void set(int k, df64 x) {
-    h[k] = x.hi;
-    l[k] = x.lo;
-  }
-};
-
-// 1/d for a pivot. FP32: the IEEE reciprocal intrinsic. FP64 and double-float: Newton-Raphson
-// iteration r <- r + r (1 - d r) from the FP32 reciprocal of the leading part (each step doubles
-// the correct bits: 23 -> 46 -> full; two steps for FP64, one for double-float), falling back to
-// a division when d is outside the float range or not finite.
-__device__ __forceinline__ float recipT(float d) { return __frcp_rn(d); }
-__device__ __forceinline__ double recipT(double d) {
-  const float f = __double2float_rn(d);
-  const float af = fabsf(f);
-  if (!(af >= 1e-37f && af <= 1e37f)) return 1.0 / d;
-  double r = (double)__frcp_rn(f);
-  double e = fma(-d, r, 1.0);
-  r = fma(r, e, r);
-  e = fma(-d, r, 1.0);
-  return fma(r, e, r);
-}
-__device__ __forceinline__ df64 recipT(df64 d) {
-  const float af = fabsf(d.hi);
-  if (!(af >= 1e-37f && af <= 1e37f)) return df64(1.0f, 0.0f) / d;
-  // one step from the 23-bit seed gives ~46 bits, the double-float rounding level
-  const df64 r(__frcp_rn(d.hi), 0.0f);
-  const df64 one(1.0f, 0.0f);
-  return r + r * (one - d * r);
-}
-
-// Factors diagonal tile J in place (one warp), FP32 form. Global row of tile row r is J*32 + r.
-// Lane r keeps row r of the tile in registers (entries right of the diagonal mirrored from the
-// lower triangle) and the 32 elimination steps broadcast pivot column j by shuffles. The same
-// steps applied to the identity (Gauss-Jordan) give row r of the inverse of the unit-lower
-// factor, which is stored transposed in the upper half: Linv(r, c) at r*ld + c. Only the
-// per-pivot regularisation test runs inside the loop, in the tile's own arithmetic; the pivot
-// statistics (exact zero, wrong sign, smallest |D|) are taken once from the final D.
-template <typename T>
-__device__ void tileFactorDiagRegs(T* A, int J, int nr, int nx, const DevSettings& st, PivotStats* ps) {
-  const int r = threadIdx.x & 31;
-  const bool regularized = st.linear_solver == 2;
-  const T epsT = (T)st.dynamic_reg_eps, deltaT = (T)st.dynamic_reg_delta;
-  Row32<T> a, e;
-#pragma unroll
-  for (int col = 0; col < 32; ++col) {
-    a.set(col, (col <= r) ? A[col * kTileLd + r] : A[r * kTileLd + col]);
-    e.set(col, (col == r) ? (T)1 : (T)0);
-  }
-  int nreg = 0;
-  T dr = (T)0;
-#pragma unroll
-  for (int j = 0; j < 32; ++j) {
-    T dj = shflT(a.get(j), j);
-    if (regularized) {
-      const int g = J * 32 + j;
-      if (g < nr) {
-        const T sg = (g < nx) ? (T)1 : (T)-1;
-        if (dj * sg < epsT) {
-          dj = dj + sg * deltaT;
-          if (dj * sg < epsT) dj = sg * deltaT;
-          ++nreg;
-        }
-      }
-    }
-    const T inv = recipT(dj);
-    const T lj = a.get(j) * inv;
-#pragma unroll
-    for (int k = j + 1; k < 32; ++k) {
-      const T akj = shflT(a.get(j), k);
-      a.set(k, msubT(a.get(k), lj, akj));
-    }
-    // Gauss-Jordan on the identity: row j of the inverse is final at step j
-#pragma unroll
-    for (int c = 0; c <= j; ++c) {
-      const T ejc = shflT(e.get(c), j);
-      if (r > j) e.set(c, msubT(e.get(c), lj, ejc));
-    }
-    if (r > j) a.set(j, lj);
-    if (r == j) {
-      a.set(j, dj);
-      dr = dj;
-    }
-  }
-  // pivot statistics of the real rows of this tile
-  {
-    const int g = J * 32 + r;
-    const bool real = g < nr;
-    const double d = (double)dr;
-    const double sgn = (g < nx) ? 1.0 : -1.0;
-    const unsigned zeroMask = __ballot_sync(0xffffffffu, real && d == 0.0);
-    const unsigned wrongMask = __ballot_sync(0xffffffffu, real && !(d * sgn > 0.0));
-    double ad = real ? fabs(d) : INFINITY;
-    if (real && !isfinite(ad)) ad = NAN;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const double o = __shfl_xor_sync(0xffffffffu, ad, off);
-      ad = (isnan(ad) || isnan(o)) ? NAN : fmin(ad, o);
-    }
-    if (r == 0) {
-      ps->nreg += nreg;
-      if (!regularized && zeroMask) ps->zero = 1;
-      if (wrongMask) ps->wrong = 1;
-      ps->minAbs = (isnan(ad) || isnan(ps->minAbs)) ? NAN : fmin(ps->minAbs, ad);
-    }
-  }
-  __syncwarp();
-#pragma unroll
-  for (int col = 0; col < 32; ++col) {
-    if (col <= r) A[col * kTileLd + r] = a.get(col);
-    if (col < r) A[r * kTileLd + col] = e.get(col);
-  }
-  __syncwarp();
-}
-
-// Factors diagonal tile J in place (one warp), form for 8-byte arithmetic (FP64, double-float),
-// whose fully unrolled register version would be too large. Global row of tile row r is J*32 + r.
-// Blocked right-looking LDL' in 8-column blocks, in shared memory (entry (i, k) at k*ld + i):
-//  (1) leaf: the 8x8 diagonal block, rows in registers of its 8 lanes, pivots by shuffle;
-//  (2) panel: every row below finishes its 8 entries of the block by substitution with the leaf
-//      (unscaled values kept in registers for (3)) and scales them by the pivot reciprocals;
-//  (3) trailing: rows below subtract the block's rank-8 product from their remaining entries.
-// Only the per-pivot regularisation test runs inside the pivot loop, in the tile's own
-// arithmetic; the pivot statistics (exact zero, wrong sign, smallest |D|) are taken once from D.
-// Then the inverse of the unit-lower factor, blocked the same way (four 8x8 leaf inverses, then
-// the blocks below the diagonal by distance), is stored transposed in the upper half:
-// Linv(R, C) at R*ld + C for C < R.
-template <typename T>
-__device__ void tileFactorDiagBlocked(T* A, int J, int nr, int nx, const DevSettings& st, PivotStats* ps) {
-  const int r = threadIdx.x & 31;
-  const bool regularized = st.linear_solver == 2;
-  const T epsT = (T)st.dynamic_reg_eps, deltaT = (T)st.dynamic_reg_delta;
-  int nreg = 0;
-  T invMine = (T)0;  // 1 / D(r), kept by lane r
-  for (int b = 0; b < 4; ++b) {
-    const int c0 = 8 * b;
-    const int li = r - c0;
-    const bool leaf = li >= 0 && li < 8;
-    // (1) leaf
-    T a[8];
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      const int ct = c0 + t;
-      a[t] = leaf ? ((t <= li) ? A[ct * kTileLd + r] : A[r * kTileLd + ct]) : (T)0;
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      T dj = shflT(a[j], c0 + j);
-      if (regularized) {
-        const int g = J * 32 + c0 + j;
-        if (g < nr) {
-          const T sg = (g < nx) ? (T)1 : (T)-1;
-          if (dj * sg < epsT) {
-            dj = dj + sg * deltaT;
-            if (dj * sg < epsT) dj = sg * deltaT;
-            ++nreg;
-          }
-        }
-      }
-      const T inv = recipT(dj);
-      if (li == j) invMine = inv;
-      const T lj = a[j] * inv;
-#pragma unroll
-      for (int k = j + 1; k < 8; ++k) {
-        const T akj = shflT(a[j], c0 + k);
-        a[k] = msubT(a[k], lj, akj);
-      }
-      if (li > j) a[j] = lj;
-      if (li == j) a[j] = dj;
-    }
-    if (leaf) {
-#pragma unroll
-      for (int t = 0; t < 8; ++t)
-        if (t <= li) A[(c0 + t) * kTileLd + r] = a[t];
-    }
-    __syncwarp();
-    if (c0 + 8 >= 32) break;
-    // (2) panel
-    const bool below = r >= c0 + 8;
-    T u[8];
-#pragma unroll
-    for (int t = 0; t < 8; ++t) u[t] = below ? A[(c0 + t) * kTileLd + r] : (T)0;
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-#pragma unroll
-      for (int s2 = t + 1; s2 < 8; ++s2) u[s2] = msubT(u[s2], u[t], A[(c0 + t) * kTileLd + c0 + s2]);
-    }
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      const T idt = shflT(invMine, c0 + t);
-      if (below) A[(c0 + t) * kTileLd + r] = u[t] * idt;
-    }
-    __syncwarp();
-    // (3) trailing
-    if (below) {
-      int k = c0 + 8;
-      for (; k + 3 <= r; k += 4) {
-        T acc0 = A[k * kTileLd + r], acc1 = A[(k + 1) * kTileLd + r];
-        T acc2 = A[(k + 2) * kTileLd + r], acc3 = A[(k + 3) * kTileLd + r];
-#pragma unroll
-        for (int t = 0; t < 8; ++t) {
-          const T* Lc = A + (c0 + t) * kTileLd;
-          const T nu = -u[t];
-          acc0 = accT(acc0, nu, Lc[k]);
-          acc1 = accT(acc1, nu, Lc[k + 1]);
-          acc2 = accT(acc2, nu, Lc[k + 2]);
-          acc3 = accT(acc3, nu, Lc[k + 3]);
-        }
-        A[k * kTileLd + r] = accEnd(acc0);
-        A[(k + 1) * kTileLd + r] = accEnd(acc1);
-        A[(k + 2) * kTileLd + r] = accEnd(acc2);
-        A[(k + 3) * kTileLd + r] = accEnd(acc3);
-      }
-      for (; k <= r; ++k) {
-        T acc = A[k * kTileLd + r];
-#pragma unroll
-        for (int t = 0; t < 8; ++t) acc = accT(acc, -u[t], A[(c0 + t) * kTileLd + k]);
-        A[k * kTileLd + r] = accEnd(acc);
-      }
-    }
-    __syncwarp();
-  }
-  // pivot statistics of the real rows of this tile
-  {
-    const int g = J * 32 + r;
-    const bool real = g < nr;
-    const double d = (double)A[r * kTileLd + r];
-    const double sgn = (g < nx) ? 1.0 : -1.0;
-    const unsigned zeroMask = __ballot_sync(0xffffffffu, real && d == 0.0);
-    const unsigned wrongMask = __ballot_sync(0xffffffffu, real && !(d * sgn > 0.0));
-    double ad = real ? fabs(d) : INFINITY;
-    if (real && !isfinite(ad)) ad = NAN;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const double o = __shfl_xor_sync(0xffffffffu, ad, off);
-      ad = (isnan(ad) || isnan(o)) ? NAN : fmin(ad, o);
-    }
-    if (r == 0) {
-      ps->nreg += nreg;
-      if (!regularized && zeroMask) ps->zero = 1;
-      if (wrongMask) ps->wrong = 1;
-      ps->minAbs = (isnan(ad) || isnan(ps->minAbs)) ? NAN : fmin(ps->minAbs, ad);
-    }
-  }
-  // (a) inverses of the four 8x8 unit-lower leaf blocks, lane r -> block r/8, column r%8
-  {
-    const int o = r & ~7, c = r & 7;
-    T y[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      T acc = (T)0;
-#pragma unroll
-      for (int k = 0; k < i; ++k) acc = accT(acc, A[(o + k) * kTileLd + o + i], y[k]);
-      y[i] = (i < c) ? (T)0 : ((i == c) ? (T)1 : -accEnd(acc));
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (i > c) A[(o + i) * kTileLd + o + c] = y[i];
-  }
-  __syncwarp();
-  // (b) blocks (I, J) = (Jb + d, Jb): Linv(I,J) = -Linv(I,I) sum_{K=J}^{I-1} L(I,K) Linv(K,J)
-  for (int d = 1; d < 4; ++d) {
-    const int nb = 4 - d;
-    for (int e = r; e < nb * 64; e += 32) {
-      const int Jb = e >> 6, i = (e >> 3) & 7, j = e & 7;
-      const int R = 8 * (Jb + d) + i, C = 8 * Jb + j;
-      T acc0 = (T)0, acc1 = (T)0;
-      for (int kk = 8 * Jb; kk < 8 * (Jb + d); kk += 2) {
-        const T lv0 = (kk > C) ? A[kk * kTileLd + C] : ((kk == C) ? (T)1 : (T)0);
-        const T lv1 = (kk + 1 > C) ? A[(kk + 1) * kTileLd + C] : ((kk + 1 == C) ? (T)1 : (T)0);
-        acc0 = accT(acc0, A[kk * kTileLd + R], lv0);
-        acc1 = accT(acc1, A[(kk + 1) * kTileLd + R], lv1);
-      }
-      A[R * kTileLd + C] = accEnd(acc0) + accEnd(acc1);
-    }
-    __syncwarp();
-    if (r < nb * 8) {
-      const int Jb = r >> 3, j = r & 7;
-      const int o = 8 * (Jb + d), C = 8 * Jb + j;
-      for (int i = 7; i >= 0; --i) {
-        T acc = A[(o + i) * kTileLd + C];
-        for (int i2 = 0; i2 < i; ++i2) acc = accT(acc, A[(o + i) * kTileLd + o + i2], A[(o + i2) * kTileLd + C]);
-        A[(o + i) * kTileLd + C] = -accEnd(acc);
-      }
-    }
-    __syncwarp();
-  }
-}
-
-// Diagonal tile factorisation: the register form for FP32, the blocked form for 8-byte types.
-template <typename T>
-__device__ __forceinline__ void tileFactorDiag(T* A, int J, int nr, int nx, const DevSettings& st, PivotStats* ps) {
-  if constexpr (sizeof(T) == 4)
-    tileFactorDiagRegs<T>(A, J, nr, nx, st, ps);
-  else
-    tileFactorDiagBlocked<T>(A, J, nr, nx, st, ps);
-}
-
-// L_IJ = A_IJ Linv_JJ^T D_J^-1 for one off-diagonal tile (one warp), in place. Column c of the
-// result needs columns k <= c of A only, so the right half (c >= 16) is produced first.
-template <typename T>
-__device__ void tileOffDiag(T* Aij, const T* Ajj) {
-  const int lane = threadIdx.x & 31, lr = lane & 7, lc = lane >> 3;
-#pragma unroll
-  for (int pass = 1; pass >= 0; --pass) {
-    const int c0 = pass * 16 + lc * 4;
-    T acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = (T)0;
-#pragma unroll 2
-    for (int k = 0; k < 32; ++k) {
-      T av[4], cv[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = Aij[k * kTileLd + lr * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int col = c0 + j;
-        cv[j] = (k < col) ? Ajj[col * kTileLd + k] : ((k == col) ? (T)1 : (T)0);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = accT(acc[i][j], av[i], cv[j]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int col = c0 + j;
-      const T dinv = recipT(Ajj[col * kTileLd + col]);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) Aij[col * kTileLd + lr * 4 + i] = accEnd(acc[i][j]) * dinv;
-    }
-    __syncwarp();
-  }
-}
-
-// C -= A diag(d) B^T for 32x32 tiles (one warp); d = diagonal of the factored tile Ajj.
-template <typename T>
-__device__ void tileSyrk(T* C, const T* A, const T* B, const T* Ajj) {
-  const int lane = threadIdx.x & 31, lr = lane & 7, lc = lane >> 3;
-#pragma unroll
-  for (int pass = 0; pass < 2; ++pass) {
-    const int c0 = pass * 16 + lc * 4;
-    T acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = (T)0;
-#pragma unroll 2
-    for (int k = 0; k < 32; ++k) {
-      const T dk = Ajj[k * kTileLd + k];
-      T av[4], bv[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = A[k * kTileLd + lr * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bv[j] = B[k * kTileLd + c0 + j] * dk;
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = accT(acc[i][j], av[i], bv[j]);
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) C[(c0 + j) * kTileLd + lr * 4 + i] -= accEnd(acc[i][j]);
-  }
-}
-
-// One 16x16 quadrant (qr, qc) of tileSyrk's C -= A diag(d) B^T, one warp: lane (r4, c2) takes
-// rows qr*16 + 4 r4 + {0..3} and columns qc*16 + 2 c2 + {0, 1}. Every entry gets tileSyrk's
-// operations in its order, so the result is the same.
-template <typename T>
-__device__ void tileSyrkQuad(T* C, const T* A, const T* B, const T* Ajj, int qr, int qc) {
-  const int lane = threadIdx.x & 31, r0 = qr * 16 + (lane & 3) * 4, c0 = qc * 16 + (lane >> 2) * 2;
-  T acc[4][2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = (T)0;
-#pragma unroll 4
-  for (int k = 0; k < 32; ++k) {
-    const T dk = Ajj[k * kTileLd + k];
-    T av[4], bv[2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) av[i] = A[k * kTileLd + r0 + i];
-#pragma unroll
-    for (int j = 0; j < 2; ++j) bv[j] = B[k * kTileLd + c0 + j] * dk;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 2; ++j) acc[i][j] = accT(acc[i][j], av[i], bv[j]);
-  }
-#pragma unroll
-  for (int j = 0; j < 2; ++j)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) C[(c0 + j) * kTileLd + r0 + i] -= accEnd(acc[i][j]);
-}
-
+// The root's LDL' by one CTA, right-looking by tile column J with a one-column lookahead:
+//  (1) the off-diagonal tiles of column J, each split over one, two or four warps by columns;
+//  (2) the next diagonal tile's product on up to six warps, then its factorisation by
+//      diagWarps() warps while the others take the other products of column J from a queue
+//      (half a tile each), joined by the factoring warps when they are done.
+// The order in which warps take products does not change a result: each is one warp's own.
 template <typename T>
 __device__ __noinline__ void denseLdlt(Ctx& c, T* M, const DevSettings& st, int& fail, int& wrongSign, double& minAbsD) {
   const int nr = c.nr, nx = c.n, Tn = rootTiles(nr);
-  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int gw = diagWarps(nw), lw = min(nw, 6);
   PivotStats* ps = reinterpret_cast<PivotStats*>(c.sc + SC_COUNT);
+  T* invD = reinterpret_cast<T*>(c.red);  // pivot reciprocals of the current tile column
   if (threadIdx.x == 0) {
     ps->nreg = 0;
     ps->zero = 0;
@@ -877,45 +451,62 @@ __device__ __noinline__ void denseLdlt(Ctx& c, T* M, const DevSettings& st, int&
     ps->minAbs = INFINITY;
   }
   __syncthreads();
-  // Right-looking by tile column with a one-column lookahead: warp 0 applies column J's update
-  // to the next diagonal tile and factors it while the other warps apply the rest of column J.
-  if (warp == 0) tileFactorDiag<T>(M, 0, nr, nx, st, ps);
+  if (warp < gw) tileFactorDiag<T>(M, 0, nr, nx, st, ps, invD, gw);
   __syncthreads();
   for (int J = 0; J + 1 < Tn; ++J) {
     T* Ajj = M + tileBase(Tn, J, J);
-    for (int I = J + 1 + warp; I < Tn; I += nw) tileOffDiag<T>(M + tileBase(Tn, I, J), Ajj);
-    __syncthreads();
     const int rem = Tn - J - 1;
-    const int npairs = rem * (rem + 1) / 2;
-    if (nw >= 4 && warp < 3) {
-      // the next diagonal tile's update, the head of the critical path, on three warps: the
-      // quadrants the factorisation reads (the upper-right one is overwritten by Linv anyway)
-      T* Anext = M + tileBase(Tn, J + 1, J + 1);
-      const T* Lnext = M + tileBase(Tn, J + 1, J);
-      tileSyrkQuad<T>(Anext, Lnext, Lnext, Ajj, warp == 0 ? 0 : 1, warp == 2 ? 1 : 0);
-      asm volatile("bar.sync 1, 96;" ::: "memory");
-    }
-    if (warp == 0 || nw == 1) {
-      T* Anext = M + tileBase(Tn, J + 1, J + 1);
-      const T* Lnext = M + tileBase(Tn, J + 1, J);
-      if (nw < 4) tileSyrk<T>(Anext, Lnext, Lnext, Ajj);
-      if (nw == 1) {
-        for (int t = 1; t < npairs; ++t) {
-          int K = J + 1, tt = t, len = rem;
-          while (tt >= len) { tt -= len; --len; ++K; }
-          const int I = K + tt;
-          tileSyrk<T>(M + tileBase(Tn, I, K), M + tileBase(Tn, I, J), M + tileBase(Tn, K, J), Ajj);
-        }
+    if (threadIdx.x == 0) ps->next = 0;
+    if (2 * rem > nw) {
+      for (int I = J + 1 + warp; I < Tn; I += nw) tileOffDiag<T>(M + tileBase(Tn, I, J), Ajj, invD);
+    } else if (4 * rem > nw) {
+      // two warps a tile: columns 0-7 and 24-31, or 8-23 (five units of 8x8 products each)
+      T* Aij = M + tileBase(Tn, J + 1 + (warp >> 1), J);
+      const bool on = (warp >> 1) < rem;
+      const int g0 = (warp & 1) ? 1 : 0, g1 = (warp & 1) ? 2 : 3;
+      T o0[8], o1[8];
+      if (on) {
+        tileOffDiagGroup(Aij, Ajj, invD, g0, o0);
+        tileOffDiagGroup(Aij, Ajj, invD, g1, o1);
       }
-      tileFactorDiag<T>(Anext, J + 1, nr, nx, st, ps);
+      __syncthreads();
+      if (on) {
+        tileOffDiagStore(Aij, g0, o0);
+        tileOffDiagStore(Aij, g1, o1);
+      }
     } else {
-      // pairs t >= 1: (I, K) with J < K <= I < Tn, enumerated column by column (t = 0 is the
-      // next diagonal tile)
-      for (int t = warp; t < npairs; t += nw - 1) {
-        int K = J + 1, tt = t, len = rem;
-        while (tt >= len) { tt -= len; --len; ++K; }
-        const int I = K + tt;
-        tileSyrk<T>(M + tileBase(Tn, I, K), M + tileBase(Tn, I, J), M + tileBase(Tn, K, J), Ajj);
+      T* Aij = M + tileBase(Tn, J + 1 + (warp >> 2), J);
+      const bool on = (warp >> 2) < rem;
+      T o0[8];
+      if (on) tileOffDiagGroup(Aij, Ajj, invD, warp & 3, o0);
+      __syncthreads();
+      if (on) tileOffDiagStore(Aij, warp & 3, o0);
+    }
+    __syncthreads();
+    const int ntask = rem * (rem + 1) - 2;  // halves of the pairs (I, K), J < K <= I, but the first
+    T* Anext = M + tileBase(Tn, J + 1, J + 1);
+    const T* Lnext = M + tileBase(Tn, J + 1, J);
+    for (int u = warp; u < 6 && warp < lw; u += lw) tileSyrkDiagUnit<T>(Anext, Lnext, Ajj, u);
+    if (nw <= 6) __syncthreads();
+    else if (warp < lw) asm volatile("bar.sync 3, %0;" ::"r"(32 * lw) : "memory");
+    if (warp < gw) tileFactorDiag<T>(Anext, J + 1, nr, nx, st, ps, invD, gw);
+    for (;;) {
+      int q = 0;
+      if (lane == 0) q = atomicAdd(&ps->next, 1);
+      q = __shfl_sync(0xffffffffu, q, 0);
+      if (q >= ntask) break;
+      // pairs column by column, (J + 1, J + 1) first
+      int K = J + 1, t = 1 + (q >> 1), len = rem;
+      while (t >= len) { t -= len; --len; ++K; }
+      const int I = K + t;
+      const T *Lik = M + tileBase(Tn, I, J), *Lkj = M + tileBase(Tn, K, J);
+      T* C = M + tileBase(Tn, I, K);
+      if (I == K && (q & 1)) {
+        // the upper right quadrant of a diagonal tile is never read
+        tileSyrkDiagUnit<T>(C, Lik, Ajj, 4);
+        tileSyrkDiagUnit<T>(C, Lik, Ajj, 5);
+      } else {
+        tileSyrkHalf<T>(C, Lik, Lkj, Ajj, q & 1);
       }
     }
     __syncthreads();
@@ -1502,16 +1093,18 @@ __device__ __forceinline__ float pow2Scale(float x, int ex) {
   return scalbnf(x, ex);
 }
 
-// Writes the slices (A and B) of the 32 rows of tile row I over the tile columns J0, J0 + 1 and
-// their exponents; one warp, lane rr takes row 32 I + rr. L_I,J0 and L_I,J0+1 must be complete
-// in M (the second written by this warp, the first before the last grid barrier).
-static __device__ __noinline__ void sliceRowPair(const df64* M, int Tn, int I, int J0, unsigned char* slices) {
-  __syncwarp();
+// Writes the slices of the 32 rows of tile row I over the tile columns J0, J0 + 1 and their
+// exponents, from the finished tiles L0 = L_I,J0 and L1 = L_I,J0+1 and the diagonal tiles A0, A1 of
+// the two columns (all in shared memory); part q of f (f = 1, 2, 4 warps a tile row: both operands,
+// one each, or half of one operand's k-groups), one warp, lane rr takes row 32 I + rr.
+static __device__ __noinline__ void sliceRowPair(const df64* L0, const df64* L1, const df64* A0, const df64* A1, int Tn,
+                                                 int I, unsigned char* slices, int q, int f) {
   const int rr = threadIdx.x & 31;
   const int64_t rows = (int64_t)Tn * kTile, m = (int64_t)I * kTile + rr;
-  const df64* src[2] = {M + tileBase(Tn, I, J0) + rr, M + tileBase(Tn, I, J0 + 1) + rr};
-  const df64* dg[2] = {M + tileBase(Tn, J0, J0), M + tileBase(Tn, J0 + 1, J0 + 1)};
-  for (int o = 0; o < 2; ++o) {
+  const df64* src[2] = {L0 + rr, L1 + rr};
+  const df64* dg[2] = {A0, A1};
+  const int kgLo = (f == 4 && q >= 2) ? kDfK / 16 : 0, kgHi = (f == 4 && q < 2) ? kDfK / 16 : kDfK / 8;
+  for (int o = (f == 1) ? 0 : (q & 1); o < ((f == 1) ? 2 : (q & 1) + 1); ++o) {
     auto value = [&](int k) -> df64 {
       const int t = k >> 5, kk = k & 31;
       df64 x = src[t][kk * kTileLd];
@@ -1524,7 +1117,7 @@ static __device__ __noinline__ void sliceRowPair(const df64* M, int Tn, int I, i
     const int e = (mx > 0.0f && mx <= 3.0e38f) ? ilogbf(mx) + 1 : 0;
     reinterpret_cast<int*>(slices + 1536 * rows)[o * rows + m] = e;
 #pragma unroll 1
-    for (int kg = 0; kg < kDfK / 8; ++kg) {
+    for (int kg = kgLo; kg < kgHi; ++kg) {
       uint32_t w[kDfSlices][4];
 #pragma unroll
       for (int t = 0; t < 8; ++t) {
@@ -1725,17 +1318,18 @@ constexpr int64_t kF32StageBytes = (int64_t)kF32OpBytes + 16 * (int64_t)kTileByt
 static_assert(kF32StageBytes + 128 <= kGridTcStageBytes, "FP32 pair staging exceeds the stage area");
 static_assert(2 * kF32Parts * kF32Groups * 16 <= 2 * kDfSlices * (kDfK / 8) * 16, "FP32 panels exceed the slice area");
 
-// Writes the TF32 parts (A and B) of the 32 rows of tile row I over the tile columns J0, J0 + 1;
-// one warp, lane rr takes row 32 I + rr. L_I,J0 and L_I,J0+1 must be complete in M.
-static __device__ __noinline__ void sliceRowPair(const float* M, int Tn, int I, int J0, unsigned char* slices) {
-  __syncwarp();
+// Writes the TF32 parts of the 32 rows of tile row I over the tile columns J0, J0 + 1; arguments as
+// for the double-float form.
+static __device__ __noinline__ void sliceRowPair(const float* L0, const float* L1, const float* A0, const float* A1,
+                                                 int Tn, int I, unsigned char* slices, int q, int f) {
   const int rr = threadIdx.x & 31;
   const int64_t rows = (int64_t)Tn * kTile, m = (int64_t)I * kTile + rr;
-  const float* src[2] = {M + tileBase(Tn, I, J0) + rr, M + tileBase(Tn, I, J0 + 1) + rr};
-  const float* dg[2] = {M + tileBase(Tn, J0, J0), M + tileBase(Tn, J0 + 1, J0 + 1)};
-  for (int o = 0; o < 2; ++o) {
+  const float* src[2] = {L0 + rr, L1 + rr};
+  const float* dg[2] = {A0, A1};
+  const int kgLo = (f == 4 && q >= 2) ? kF32Groups / 2 : 0, kgHi = (f == 4 && q < 2) ? kF32Groups / 2 : kF32Groups;
+  for (int o = (f == 1) ? 0 : (q & 1); o < ((f == 1) ? 2 : (q & 1) + 1); ++o) {
 #pragma unroll 2
-    for (int kg = 0; kg < kF32Groups; ++kg) {
+    for (int kg = kgLo; kg < kgHi; ++kg) {
       float hi[4], lo[4];
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
@@ -1886,46 +1480,181 @@ static __device__ __noinline__ bool tcF32PairTrailingStep(float* M, int Tn, int 
   return true;
 }
 
+// Copies one tile between global and shared memory (16-byte vectors), thread t of nt.
+template <typename T>
+__device__ __forceinline__ void copyTile(T* dst, const T* src, int t, int nt) {
+  constexpr int nv = kTileElems * (int)sizeof(T) / 16;
+#pragma unroll 4
+  for (int v = t; v < nv; v += nt) reinterpret_cast<uint4*>(dst)[v] = reinterpret_cast<const uint4*>(src)[v];
+}
+
+// Shared-memory tiles of a CTA in the whole-GPU factor's column phases: the pivot reciprocals of
+// the diagonal tile(s), up to three tiles for the whole CTA, then two per team of warps.
+template <typename T>
+struct ColStage {
+  T *inv0, *inv1, *t0, *t1, *t2, *team;
+};
+template <typename T>
+__device__ __forceinline__ ColStage<T> colStage(T* stage) {
+  T* t = stage + 64;
+  return {stage, stage + 32, t, t + kTileElems, t + 2 * kTileElems, t + 3 * kTileElems};
+}
+
+// Warps per tile in a column phase with `rem` tiles on GW warps: four, two or one, as many as fit.
+__device__ __forceinline__ int teamWarps(int rem, int GW) { return 4 * rem <= GW ? 4 : (2 * rem <= GW ? 2 : 1); }
+
+// Named barrier of one team of f warps (ids 4 ..; f is 2 or 4, eight warps a CTA).
+__device__ __forceinline__ void teamSync(int team, int f) {
+  if (f == 1) __syncwarp();
+  else asm volatile("bar.sync %0, %1;" ::"r"(4 + team), "r"(32 * f) : "memory");
+}
+
+// The column groups of warp q in a team of f: one (f = 4), two of together five units (f = 2) or
+// all four, last first (f = 1); src and dst may be the same tile only for f = 1.
+template <typename T>
+__device__ __forceinline__ void teamOffDiag(const T* src, T* dst, const T* Ajj, const T* invD, int q, int f) {
+#pragma unroll 1
+  for (int i = 0; i < 4 / f; ++i) {
+    const int g = (f == 4) ? q : (f == 2) ? (q ? 1 + i : 3 * i) : 3 - i;
+    T o[8];
+    tileOffDiagGroup(src, Ajj, invD, g, o);
+    if (f == 1) __syncwarp();
+    tileOffDiagStore(dst, g, o);
+    if (f == 1) __syncwarp();
+  }
+}
+
+// Column J's off-diagonal tiles I >= I0 on warps w0 .. GW-1 of the grid (gw this warp's number):
+// the CTA's tiles are read into shared memory and the results written to global memory.
+template <typename T>
+__device__ __noinline__ void gridOffDiag(T* M, int Tn, int I0, int J, int w0, int gw, int GW, const ColStage<T>& cs) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int f = teamWarps(Tn - I0, GW - w0), first = (gw - warp - w0) / f;  // this CTA's first team
+  if (gw - warp < w0 || I0 + first >= Tn) return;
+  const T* Ajj = M + tileBase(Tn, J, J);
+  copyTile(cs.t0, Ajj, (int)threadIdx.x, (int)blockDim.x);
+  if (warp == 0) cs.inv0[lane] = recipT(Ajj[lane * kTileLd + lane]);
+  const int team = warp / f, q = warp % f;
+  T* A = cs.team + 2 * team * kTileElems;
+  int I = I0 + first + team;
+  if (I < Tn) copyTile(A, M + tileBase(Tn, I, J), q * 32 + lane, 32 * f);
+  __syncthreads();
+  for (; I < Tn; I += (GW - w0) / f) {
+    T* dst = M + tileBase(Tn, I, J);
+    if (f == 1) {
+      for (int g = 3; g >= 0; --g) {
+        T o[8];
+        tileOffDiagGroup(A, cs.t0, cs.inv0, g, o);
+        tileOffDiagStore(dst, g, o);
+      }
+      __syncwarp();
+      const int In = I + (GW - w0);
+      if (In < Tn) copyTile(A, M + tileBase(Tn, In, J), lane, 32);
+      __syncwarp();
+    } else {
+      teamOffDiag(A, dst, cs.t0, cs.inv0, q, f);
+    }
+  }
+  tc::fenceProxyAsyncShared();  // these accesses before the trailing update's bulk copies into the area
+}
+
+// CTA 0 with its eight warps: tile (J, J) of the root into cs.t2, updated by the columns whose
+// off-diagonal tiles L_J,K and diagonal tiles A_KK are given (global; the second may be null),
+// factored and written back.
+template <typename T>
+__device__ __noinline__ void gridNextDiag(T* M, int Tn, int J, const T* L0, const T* A0, const T* L1, const T* A1,
+                                          int nr, int nx, const DevSettings& st, PivotStats* ps,
+                                          const ColStage<T>& cs) {
+  const int warp = threadIdx.x >> 5, tid = threadIdx.x, nt = blockDim.x;
+  T* An = M + tileBase(Tn, J, J);
+  copyTile(cs.t2, An, tid, nt);
+  __syncthreads();
+  for (int h = 0; h < 2; ++h) {
+    const T* L = h ? L1 : L0;
+    if (!L) break;
+    copyTile(cs.t1, L, tid, nt);
+    copyTile(cs.t0, h ? A1 : A0, tid, nt);
+    __syncthreads();
+    if (warp < 6) tileSyrkDiagUnit<T>(cs.t2, cs.t1, cs.t0, warp);
+    __syncthreads();
+  }
+  if (warp < 4) tileFactorDiag<T>(cs.t2, J, nr, nx, st, ps, cs.inv0, 4);
+  __syncthreads();
+  copyTile(An, cs.t2, tid, nt);
+  __syncthreads();
+}
+
 // Whole-GPU FP32 and double-float LDL' over pairs of tile columns (J0, J1 = J0 + 1), three grid
-// barriers per pair:
-//  (A0) the off-diagonal tiles of column J0, one warp each; CTA 0's warp 0 takes L_J1,J0, then
-//       updates the diagonal tile (J1, J1) with it and factors it;
-//  (A1) column J1's tiles I > J1, one warp each: the update by column J0 (tile routine),
-//       L_I,J1, and the tensor-core operands of the row pair (sliceRowPair: TF32 parts for FP32,
-//       BF16 slices for double-float);
+// barriers per pair; in the column phases a tile's work is shared by up to four warps, on copies
+// in shared memory:
+//  (A0) the off-diagonal tiles of column J0; CTA 0 takes L_J1,J0, then updates the diagonal tile
+//       (J1, J1) with it and factors it;
+//  (A1) column J1's tiles I > J1: the update by column J0 (tile routine), L_I,J1, and the
+//       tensor-core operands of the row pair (sliceRowPair: TF32 parts for FP32, BF16 slices for
+//       double-float);
 //  (B)  the trailing update of both columns at once (tcF32PairTrailingStep / tcDfTrailingStep,
-//       CTAs 1..), while CTA 0's warp 0 updates the diagonal tile (J1 + 1, J1 + 1) with both
-//       columns and factors it.
-// Only CTA 0's warp 0 factors diagonal tiles, so the pivot statistics stay in its shared memory.
+//       CTAs 1..), while CTA 0 updates the diagonal tile (J1 + 1, J1 + 1) with both columns and
+//       factors it.
+// Only CTA 0 factors diagonal tiles, so the pivot statistics stay in its shared memory.
 template <typename T>
 __device__ __noinline__ bool gridLdltPairs(GridCtl* g, int nr, int nx, const DevSettings& st, T* M, PivotStats* ps,
-                                           unsigned char* slices, int Tn, int warp, int gw, int GW, bool cta0,
+                                           T* stage, unsigned char* slices, int Tn, int warp, int gw, int GW, bool cta0,
                                            TcState& tcs) {
-  if (cta0 && warp == 0) tileFactorDiag<T>(M, 0, nr, nx, st, ps);
+  const ColStage<T> cs = colStage(stage);
+  const int W = blockDim.x >> 5, tid = threadIdx.x, lane = tid & 31;
+  if (cta0) gridNextDiag<T>(M, Tn, 0, nullptr, nullptr, nullptr, nullptr, nr, nx, st, ps, cs);
   if (!gridSync(g)) return false;
   for (int J0 = 0; J0 + 1 < Tn; J0 += 2) {
     const int J1 = J0 + 1;
     const T* A0 = M + tileBase(Tn, J0, J0);
-    T* A1 = M + tileBase(Tn, J1, J1);
+    const T* A1 = M + tileBase(Tn, J1, J1);
     // (A0)
-    if (cta0 && warp == 0) {
+    if (cta0) {
       T* L10 = M + tileBase(Tn, J1, J0);
-      tileOffDiag<T>(L10, A0);
-      __syncwarp();
-      tileSyrk<T>(A1, L10, L10, A0);
-      __syncwarp();
-      tileFactorDiag<T>(A1, J1, nr, nx, st, ps);
+      copyTile(cs.t0, A0, tid, (int)blockDim.x);
+      copyTile(cs.t1, L10, tid, (int)blockDim.x);
+      if (warp == 0) cs.inv0[lane] = recipT(A0[lane * kTileLd + lane]);
+      __syncthreads();
+      if (warp < 4) teamOffDiag(cs.t1, L10, cs.t0, cs.inv0, warp, 4);
+      __syncthreads();
+      gridNextDiag<T>(M, Tn, J1, L10, A0, nullptr, nullptr, nr, nx, st, ps, cs);
     } else {
-      for (int I = J1 + 1 + (gw - 1); I < Tn; I += GW - 1) tileOffDiag<T>(M + tileBase(Tn, I, J0), A0);
+      gridOffDiag<T>(M, Tn, J1 + 1, J0, W, gw, GW, cs);
     }
     if (!gridSync(g)) return false;
     // (A1)
-    for (int I = J1 + 1 + gw; I < Tn; I += GW) {
-      T* C = M + tileBase(Tn, I, J1);
-      tileSyrk<T>(C, M + tileBase(Tn, I, J0), M + tileBase(Tn, J1, J0), A0);
-      __syncwarp();
-      tileOffDiag<T>(C, A1);
-      sliceRowPair(M, Tn, I, J0, slices);
+    const int f = teamWarps(Tn - J1 - 1, GW), team = warp / f, q = warp % f, first = (gw - warp) / f;
+    if (J1 + 1 + first < Tn) {
+      T *C = cs.team + 2 * team * kTileElems, *L0 = C + kTileElems;
+      copyTile(cs.t0, A0, tid, (int)blockDim.x);
+      copyTile(cs.t1, A1, tid, (int)blockDim.x);
+      copyTile(cs.t2, M + tileBase(Tn, J1, J0), tid, (int)blockDim.x);
+      if (warp == 0) cs.inv1[lane] = recipT(A1[lane * kTileLd + lane]);
+      __syncthreads();
+      for (int I = J1 + 1 + first + team; I < Tn; I += GW / f) {
+        T* dst = M + tileBase(Tn, I, J1);
+        copyTile(C, dst, q * 32 + lane, 32 * f);
+        copyTile(L0, M + tileBase(Tn, I, J0), q * 32 + lane, 32 * f);
+        teamSync(team, f);
+        for (int h = q; h < 2; h += f) tileSyrkHalf<T>(C, L0, cs.t2, cs.t0, h);
+        teamSync(team, f);
+        T o0[8], o1[8];
+        if (f == 1) {
+          teamOffDiag(C, C, cs.t1, cs.inv1, 0, 1);
+        } else {
+          const int g0 = (f == 4) ? q : (q ? 1 : 0), g1 = q ? 2 : 3;
+          tileOffDiagGroup(C, cs.t1, cs.inv1, g0, o0);
+          if (f == 2) tileOffDiagGroup(C, cs.t1, cs.inv1, g1, o1);
+          teamSync(team, f);
+          tileOffDiagStore(C, g0, o0);
+          if (f == 2) tileOffDiagStore(C, g1, o1);
+          teamSync(team, f);
+        }
+        copyTile(dst, C, q * 32 + lane, 32 * f);
+        sliceRowPair(L0, C, cs.t0, cs.t1, Tn, I, slices, q, f);
+        teamSync(team, f);
+      }
+      tc::fenceProxyAsyncShared();  // these accesses before the trailing update's bulk copies into the area
     }
     if (!gridSync(g)) return false;
     if (J1 + 1 >= Tn) break;
@@ -1934,14 +1663,8 @@ __device__ __noinline__ bool gridLdltPairs(GridCtl* g, int nr, int nx, const Dev
     const int nb = (rem + 3) >> 2;
     const long long nsb = (long long)nb * (nb + 1) / 2;
     if (cta0) {
-      if (warp == 0) {
-        T* An = M + tileBase(Tn, J1 + 1, J1 + 1);
-        tileSyrk<T>(An, M + tileBase(Tn, J1 + 1, J0), M + tileBase(Tn, J1 + 1, J0), A0);
-        __syncwarp();
-        tileSyrk<T>(An, M + tileBase(Tn, J1 + 1, J1), M + tileBase(Tn, J1 + 1, J1), A1);
-        __syncwarp();
-        tileFactorDiag<T>(An, J1 + 1, nr, nx, st, ps);
-      }
+      gridNextDiag<T>(M, Tn, J1 + 1, M + tileBase(Tn, J1 + 1, J0), A0, M + tileBase(Tn, J1 + 1, J1), A1, nr, nx, st, ps,
+                      cs);
     } else {
       bool okT;
       if constexpr (sizeof(T) == 4)
@@ -1961,14 +1684,14 @@ __device__ __noinline__ bool gridLdltPairs(GridCtl* g, int nr, int nx, const Dev
 }
 
 // Tiled right-looking LDL' of the root over the whole grid. Per tile column J:
-//  (A) the off-diagonal tiles of column J, one warp each; barrier;
+//  (A) the off-diagonal tiles of column J, up to four warps each; barrier;
 //  (B) the trailing update C_IK -= L_IJ D_J L_KJ^T, J < K <= I, in super-blocks of 4x4 tiles, one
 //      CTA each (CTAs 1..: FP32 on the tensor cores, tcTrailingStep; FP64 and double-float on the
-//      CUDA cores, superSyrk), while warp 0 of CTA 0 updates the tile (J+1, J+1) with the tile
-//      routine and factors it (one-column lookahead); barrier.
+//      CUDA cores, superSyrk), while CTA 0 updates the tile (J+1, J+1) with the tile routine and
+//      factors it (one-column lookahead); barrier.
 // In FP64 every root entry receives its updates in increasing J with the same operations and
-// rounding as the single-CTA factor, so both give the same bits. Only warp 0 of CTA 0 factors
-// diagonal tiles, so the pivot statistics stay in CTA 0's shared memory (ps). `stage` holds
+// rounding as the single-CTA factor, so both give the same bits. Only CTA 0 factors diagonal
+// tiles, so the pivot statistics stay in its shared memory (ps). `stage` holds
 // gridStageBytes. Large FP32 and double-float roots run over column pairs instead (gridLdltPairs).
 template <typename T>
 __device__ __noinline__ bool gridLdltSteps(GridCtl* g, int nr, int nx, const DevSettings& st, T* M, PivotStats* ps,
@@ -2015,7 +1738,7 @@ __device__ __noinline__ bool gridLdlt(GridCtl* g, int nr, int nx, const DevSetti
   }
   bool ok = false;
   if constexpr (kTc) {
-    if (Tn >= pairMinTiles<T>()) ok = gridLdltPairs<T>(g, nr, nx, st, M, ps, slices, Tn, warp, gw, GW, cta0, tcs);
+    if (Tn >= pairMinTiles<T>()) ok = gridLdltPairs<T>(g, nr, nx, st, M, ps, stage, slices, Tn, warp, gw, GW, cta0, tcs);
   }
   if (!kTc || Tn < pairMinTiles<T>())
     ok = gridLdltSteps<T>(g, nr, nx, st, M, ps, stage, slices, Tn, warp, gw, GW, cta0, tcs);
@@ -2033,25 +1756,21 @@ template <typename T>
 __device__ __noinline__ bool gridLdltSteps(GridCtl* g, int nr, int nx, const DevSettings& st, T* M, PivotStats* ps,
                                            T* stage, unsigned char* slices, int Tn, int warp, int gw, int GW, bool cta0,
                                            TcState& tcs) {
-  if (cta0 && warp == 0) tileFactorDiag<T>(M, 0, nr, nx, st, ps);
+  const ColStage<T> cs = colStage(stage);
+  if (cta0) gridNextDiag<T>(M, Tn, 0, nullptr, nullptr, nullptr, nullptr, nr, nx, st, ps, cs);
   if (!gridSync(g)) return false;
   for (int J = 0; J + 1 < Tn; ++J) {
     T* Ajj = M + tileBase(Tn, J, J);
-    for (int I = J + 1 + gw; I < Tn; I += GW) tileOffDiag<T>(M + tileBase(Tn, I, J), Ajj);
+    gridOffDiag<T>(M, Tn, J + 1, J, 0, gw, GW, cs);
     if (!gridSync(g)) return false;
     const int rem = Tn - J - 1;
     const int nb = (rem + 3) >> 2;
     const long long nsb = (long long)nb * (nb + 1) / 2;
-    // CTA 0's warp 0 updates and factors the next diagonal tile (J+1, J+1), the critical path of
-    // the next column; the super-blocks (row order: sb = r (r + 1) / 2 + k, tile rows J+1+4r..,
-    // tile columns J+1+4k..) go to CTAs 1.. cyclically, super-block 0 without that tile
+    // CTA 0 updates and factors the next diagonal tile (J+1, J+1), the critical path of the next
+    // column; the super-blocks (row order: sb = r (r + 1) / 2 + k, tile rows J+1+4r.., tile
+    // columns J+1+4k..) go to CTAs 1.. cyclically, super-block 0 without that tile
     if (cta0) {
-      if (warp == 0) {
-        T* An = M + tileBase(Tn, J + 1, J + 1);
-        const T* Ln = M + tileBase(Tn, J + 1, J);
-        tileSyrk<T>(An, Ln, Ln, Ajj);
-        tileFactorDiag<T>(An, J + 1, nr, nx, st, ps);
-      }
+      gridNextDiag<T>(M, Tn, J + 1, M + tileBase(Tn, J + 1, J), Ajj, nullptr, nullptr, nr, nx, st, ps, cs);
       if (!gridSync(g)) return false;
       continue;
     }

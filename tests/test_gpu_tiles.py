@@ -1,0 +1,31 @@
+"""GPU tests of the root factor's tile operations at the edges of their splits: sizes around the
+8-row leaf blocks and the 32-row tiles, every number of warps that splits the work differently.
+
+However the work is spread, every entry takes one order of operations, so L and D are the same bits
+for every block size; and they agree with numpy's LDL' within test_gpu_dense's tolerances."""
+import numpy as np
+import pytest
+
+from test_gpu_dense import TOL, ldlt_ref, probe, quasi_definite
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("arith", ["fp64", "fp32", "df64"])
+@pytest.mark.parametrize("nr", [1, 7, 8, 9, 24, 25, 31, 33, 41, 65, 96, 129, 161, 190])
+def test_factor_is_the_same_for_every_split(nr, arith):
+    nx = max(1, nr - nr // 8)
+    K = quasi_definite(nr, nx, seed=nr)
+    b = np.random.default_rng(nr).standard_normal(nr)
+    ref = None
+    # 32 .. 256 threads: one warp; two; an odd number; four; more than four; eight
+    for threads in (32, 64, 96, 128, 160, 256):
+        L, D, x, _, flags = probe(K, nx, b, arith, threads)
+        assert flags[0] == 0 and flags[1] == 0
+        if ref is None:
+            ref = (L, D)
+            L0, D0 = ldlt_ref(K)
+            tol = TOL[arith]
+            assert np.max(np.abs(D - D0)) <= tol * np.max(np.abs(D0))
+            assert np.max(np.abs(L - L0)) <= tol * max(1.0, np.max(np.abs(L0)))
+        assert np.array_equal(L, ref[0]) and np.array_equal(D, ref[1]), threads
