@@ -15,7 +15,52 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include "cxg_layout.h"
+
 namespace cxg {
+
+// Finiteness and sign from the bits (integer tests: an FP64 comparison holds the FP64 unit of its
+// sub-partition for 64 cycles).
+__device__ __forceinline__ bool finiteBits(double v) {
+  return ((__double_as_longlong(v) >> 52) & 0x7ff) != 0x7ff;
+}
+__device__ __forceinline__ bool negBits(double v) {  // v < 0
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  return b > 0x8000000000000000ull && b <= 0xfff0000000000000ull;
+}
+
+// Order of doubles as integers (NaN outside both infinities), and minima / maxima on it with fmin's
+// and fmax's treatment of NaN.
+__device__ __forceinline__ long long orderKey(double v) {
+  const long long b = __double_as_longlong(v);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ bool nanBits(double v) {
+  return (__double_as_longlong(v) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+}
+__device__ __forceinline__ double minBits(double a, double b) {
+  if (nanBits(a)) return b;
+  if (nanBits(b)) return a;
+  return orderKey(b) < orderKey(a) ? b : a;
+}
+__device__ __forceinline__ double maxBits(double a, double b) {
+  if (nanBits(a)) return b;
+  if (nanBits(b)) return a;
+  return orderKey(b) > orderKey(a) ? b : a;
+}
+__device__ __forceinline__ bool zeroBits(double v) { return (__double_as_longlong(v) << 1) == 0; }
+// a < b (false when either is NaN)
+__device__ __forceinline__ bool lessBits(double a, double b) {
+  return !nanBits(a) && !nanBits(b) && orderKey(a) < orderKey(b) && !(zeroBits(a) && zeroBits(b));
+}
+__device__ __forceinline__ bool posBits(double v) {  // v > 0
+  const long long b = __double_as_longlong(v);
+  return b > 0 && b <= 0x7ff0000000000000ll;
+}
+__device__ __forceinline__ bool nonNegBits(double v) {  // v >= 0
+  const long long b = __double_as_longlong(v);
+  return (b >= 0 && b <= 0x7ff0000000000000ll) || b == (long long)0x8000000000000000ull;
+}
 
 constexpr double kTiny = 1e-12;                    // second_order_cone.cpp:23
 constexpr double kDblMin = 2.2250738585072014e-308;
@@ -28,88 +73,106 @@ constexpr double kWMax = 1e8;                      // second_order_cone.cpp:152
 // reference dense form below
 constexpr double kHsRes = 2.220446049250313e-16;
 
-// Per-SOC-block scaling parameters (8 doubles in shared memory):
-// [0] kind (0 identity fallback, 1 diagonal, 2 plane, 3 plane with the small eigenvalue of Hs held
-// at the dense form's resolution, hsSmall), [1] beta, [2] lambda (plane) or
-// a = 2v0^2-1 (diagonal), [3] q1c, [4] q1s (in-plane eigenvector of lambda), [5..7] the three
-// eigenvalues of G = (Hs + eps I)^-1 prepared at factorisation time (socPrepareG).
+// Per-SOC-block scaling parameters (9 doubles in shared memory): kind (0 identity fallback, 1
+// diagonal, 2 plane, 3 plane with the small eigenvalue of Hs held at the dense form's resolution,
+// hsSmall), beta, lam = lambda (plane) or a = 2v0^2-1 (diagonal), w2 = beta / lambda (plane), the
+// small in-plane eigenvalue of W, kept since a division costs as much as nine multiply-adds and
+// every application needs it, qc, qs (in-plane eigenvector of lambda), and the three eigenvalues of
+// G = (Hs + eps I)^-1 prepared at factorisation time (socPrepareG).
 // The unit vector u is kept in a row-indexed array at rows off+1 .. off+dim-1.
 struct SocScale {
-  double kind, beta, lam, qc, qs, r0, r1, r2;
+  long long kind;
+  double beta, lam, w2, qc, qs, r0, r1, r2;
 };
+static_assert(sizeof(SocScale) == 8 * kSocScaleDoubles, "SocScale is kept in arrays of doubles");
 
 // Computes the NT scaling of one SOC block from (s, z) (second_order_cone.cpp:70-159): the same
 // clamps (margin floors, beta clamp, c floor, v0 floor) and the same identity fallback test on
-// the entries of W = beta (2 v v' - J).
-__device__ __forceinline__ void socUpdateScaling(const double* s, const double* z, int d,
-                                                 SocScale& sc, double* u) {
+// the entries of W = beta (2 v v' - J). DIM: the block's dimension where it is known when
+// compiling (registers instead of loops), else 0. The sums are written as fused multiply-adds: an
+// unrolled sum's first two products could otherwise be fused either way round.
+template <int DIM>
+__device__ __forceinline__ void socUpdateScalingDim(const double* s, const double* z, int dim, SocScale& sc, double* u) {
+  const int d = DIM ? DIM : dim;
   double s1sq = 0, z1sq = 0, sz = 0;
+#pragma unroll
   for (int i = 1; i < d; ++i) {
-    s1sq += s[i] * s[i];
-    z1sq += z[i] * z[i];
+    s1sq = fma(s[i], s[i], s1sq);
+    z1sq = fma(z[i], z[i], z1sq);
   }
-  for (int i = 0; i < d; ++i) sz += s[i] * z[i];
+#pragma unroll
+  for (int i = 0; i < d; ++i) sz = fma(s[i], z[i], sz);
   const double s0 = s[0], z0 = z[0];
-  const double a = sqrt(fmax(fmax(s0 * s0 - s1sq, kTinyRel * s0 * s0), kAbsFloor));
-  const double b = sqrt(fmax(fmax(z0 * z0 - z1sq, kTinyRel * z0 * z0), kAbsFloor));
-  const double beta = fmin(fmax(sqrt(a / b), 1.0 / kBetaMax), kBetaMax);
-  const double c = sqrt(fmax((sz / (a * b) + 1.0) / 2.0, kTiny));
+  const double a = sqrt(maxBits(maxBits(s0 * s0 - s1sq, kTinyRel * s0 * s0), kAbsFloor));
+  const double b = sqrt(maxBits(maxBits(z0 * z0 - z1sq, kTinyRel * z0 * z0), kAbsFloor));
+  const double beta = minBits(maxBits(sqrt(a / b), 1.0 / kBetaMax), kBetaMax);
+  const double c = sqrt(maxBits((sz / (a * b) + 1.0) / 2.0, kTiny));
   // v = (s/a + J z / b) / (2c); v0 += 1; v0 = max(v0, tiny); v /= sqrt(2 v0)
-  const double inv2c = 1.0 / (2.0 * c);
   double v0 = (z0 / b + s0 / a) / (2.0 * c);
   v0 += 1.0;
-  v0 = fmax(v0, kTiny);
+  v0 = maxBits(v0, kTiny);
   const double nrm = sqrt(2.0 * v0);
   v0 /= nrm;
   double n1sq = 0.0, vmax1 = 0.0, vmax2 = 0.0, vdiagmax = 0.0;
-  bool finite = isfinite(v0) && isfinite(beta);
+  bool finite = finiteBits(v0) && finiteBits(beta);
+#pragma unroll
   for (int i = 1; i < d; ++i) {
     const double vi = ((-z[i] / b + s[i] / a) / (2.0 * c)) / nrm;
-    (void)inv2c;
     u[i] = vi;
-    n1sq += vi * vi;
+    n1sq = fma(vi, vi, n1sq);
     const double av = fabs(vi);
-    if (av > vmax1) { vmax2 = vmax1; vmax1 = av; } else if (av > vmax2) { vmax2 = av; }
-    vdiagmax = fmax(vdiagmax, fabs(2.0 * vi * vi + 1.0));
-    finite = finite && isfinite(vi);
+    if (lessBits(vmax1, av)) { vmax2 = vmax1; vmax1 = av; } else if (lessBits(vmax2, av)) { vmax2 = av; }
+    vdiagmax = maxBits(vdiagmax, fabs(2.0 * vi * vi + 1.0));
+    finite = finite && finiteBits(vi);
   }
   // max |W_ij| / beta over the explicit W = beta (2 v v' - J)
   double wmax = fabs(2.0 * v0 * v0 - 1.0);
-  wmax = fmax(wmax, vdiagmax);
-  wmax = fmax(wmax, 2.0 * fabs(v0) * vmax1);
-  if (d > 2) wmax = fmax(wmax, 2.0 * vmax1 * vmax2);
+  wmax = maxBits(wmax, vdiagmax);
+  wmax = maxBits(wmax, 2.0 * fabs(v0) * vmax1);
+  if (d > 2) wmax = maxBits(wmax, 2.0 * vmax1 * vmax2);
   wmax *= beta;
   // Hs = W W has entries up to ~dim * wmax^2: finite whenever W is finite and wmax <= 1e8.
-  if (!finite || !(wmax <= kWMax)) {
-    sc.kind = 0.0;
+  if (!finite || nanBits(wmax) || lessBits(kWMax, wmax)) {
+    sc.kind = 0;
     sc.beta = 1.0;
     sc.lam = 1.0;
+    sc.w2 = 1.0;
     sc.qc = 1.0;
     sc.qs = 0.0;
     return;
   }
   const double n1 = sqrt(n1sq);
   sc.beta = beta;
-  if (n1 == 0.0 || d == 1) {
-    sc.kind = 1.0;
+  if (zeroBits(n1) || d == 1) {
+    sc.kind = 1;
     sc.lam = 2.0 * v0 * v0 - 1.0;
+    sc.w2 = beta;
     sc.qc = 1.0;
     sc.qs = 0.0;
+#pragma unroll
     for (int i = 1; i < d; ++i) u[i] = 0.0;
     return;
   }
+#pragma unroll
   for (int i = 1; i < d; ++i) u[i] /= n1;
   const double A = 2.0 * v0 * v0 - 1.0, C = 2.0 * v0 * n1, E = 2.0 * n1 * n1 + 1.0;
   const double h = 0.5 * (A + E);
   const double r = hypot(0.5 * (A - E), C);
   const double l1 = h + r;
   double qa, qb;
-  if (A >= E) { qa = l1 - E; qb = C; } else { qa = C; qb = l1 - A; }
+  if (!lessBits(A, E)) { qa = l1 - E; qb = C; } else { qa = C; qb = l1 - A; }
   const double qn = hypot(qa, qb);
-  sc.kind = 2.0;
+  sc.kind = 2;
   sc.lam = l1;
+  sc.w2 = beta / l1;
   sc.qc = qa / qn;
   sc.qs = qb / qn;
+}
+
+__device__ __forceinline__ void socUpdateScaling(const double* s, const double* z, int d, SocScale& sc, double* u) {
+  if (d == 3) socUpdateScalingDim<3>(s, z, d, sc, u);
+  else if (d == 4) socUpdateScalingDim<4>(s, z, d, sc, u);
+  else socUpdateScalingDim<0>(s, z, d, sc, u);
 }
 
 // Scalar functions of W used by the method.
@@ -125,21 +188,39 @@ __device__ __forceinline__ double wfun(int f, double w, double eps) {
   }
 }
 
+// w^2 + eps, fused or with the square rounded first. Which of the two an expression takes is written
+// out below, so that it does not depend on what the compiler finds in one basic block.
+__device__ __forceinline__ double sqEps(double w, double eps, bool fused) {
+  return fused ? __fma_rn(w, w, eps) : __dadd_rn(__dmul_rn(w, w), eps);
+}
+// wfun for an eigenvalue of a SOC block's W.
+__device__ __forceinline__ double wfunSoc(int f, double w, double eps, bool fused) {
+  switch (f) {
+    case kW: return w;
+    case kWinv: return 1.0 / w;
+    case kHs: return w * w;
+    case kHsEps: return sqEps(w, eps, fused);
+    default: return 1.0 / sqEps(w, eps, fused);
+  }
+}
+
 // Functions of Hs given one of its eigenvalues h (f = kHs, kHsEps, kGinv).
 __device__ __forceinline__ double hsfun(int f, double h, double eps) {
-  return f == kHs ? h : (f == kHsEps ? h + eps : 1.0 / (h + eps));
+  return f == kHs ? h : (f == kHsEps ? __dadd_rn(h, eps) : 1.0 / __dadd_rn(h, eps));
 }
 
 // The small in-plane eigenvalue of Hs of a kind-3 block: (beta / lambda)^2, held at no less than
 // kHsRes (beta lambda)^2.
 __device__ __forceinline__ double hsSmall(const SocScale& sc) {
-  const double w1 = sc.beta * sc.lam, w2 = sc.beta / sc.lam;
-  return fmax(w2 * w2, kHsRes * (w1 * w1));
+  const double w1 = sc.beta * sc.lam, w2 = sc.w2;
+  return maxBits(__dmul_rn(w2, w2), __dmul_rn(kHsRes, __dmul_rn(w1, w1)));
 }
 
 // y = f(W) x for one SOC block (x, y may alias only if identical).
-__device__ __forceinline__ void socApply(const SocScale& sc, const double* u, int d, int f, double eps,
-                                         const double* x, double* y) {
+template <int DIM>
+__device__ __forceinline__ void socApplyDim(const SocScale& sc, const double* u, int dim, int f, double eps,
+                                            const double* x, double* y) {
+  const int d = DIM ? DIM : dim;
   const int kind = (int)sc.kind;
   if (kind == 0) {
     const double g = wfun(f, 1.0, eps);
@@ -155,16 +236,24 @@ __device__ __forceinline__ void socApply(const SocScale& sc, const double* u, in
   }
   const double x0 = x[0];
   double xf = 0.0;
-  for (int i = 1; i < d; ++i) xf += u[i] * x[i];
+#pragma unroll
+  for (int i = 1; i < d; ++i) xf = fma(u[i], x[i], xf);
   const double c1 = sc.qc * x0 + sc.qs * xf;
   const double c2 = -sc.qs * x0 + sc.qc * xf;
-  const double f1 = wfun(f, sc.beta * sc.lam, eps);
-  const double f2 = (kind == 3 && f >= kHs) ? hsfun(f, hsSmall(sc), eps) : wfun(f, sc.beta / sc.lam, eps);
-  const double f3 = wfun(f, sc.beta, eps);
+  const double f1 = wfunSoc(f, sc.beta * sc.lam, eps, true);
+  const double f2 = (kind == 3 && f >= kHs) ? hsfun(f, hsSmall(sc), eps) : wfunSoc(f, sc.w2, eps, false);
+  const double f3 = wfunSoc(f, sc.beta, eps, true);
   const double y0 = f1 * c1 * sc.qc - f2 * c2 * sc.qs;
   const double yF = f1 * c1 * sc.qs + f2 * c2 * sc.qc;
+#pragma unroll
   for (int i = 1; i < d; ++i) y[i] = f3 * (x[i] - xf * u[i]) + yF * u[i];
   y[0] = y0;
+}
+__device__ __forceinline__ void socApply(const SocScale& sc, const double* u, int d, int f, double eps,
+                                         const double* x, double* y) {
+  if (d == 3) socApplyDim<3>(sc, u, d, f, eps, x, y);
+  else if (d == 4) socApplyDim<4>(sc, u, d, f, eps, x, y);
+  else socApplyDim<0>(sc, u, d, f, eps, x, y);
 }
 
 // G = (Hs + eps I)^-1 of one SOC block as its three eigenvalues (stored in sc.r0..r2).
@@ -178,15 +267,17 @@ __device__ __forceinline__ void socPrepareG(SocScale& sc, double eps) {
     sc.r0 = 1.0 / (w0 * w0 + eps);
     sc.r1 = sc.r2 = 1.0 / (w * w + eps);
   } else {
-    const double w1 = sc.beta * sc.lam, w2 = sc.beta / sc.lam, w3 = sc.beta;
-    sc.r0 = 1.0 / (w1 * w1 + eps);
-    sc.r1 = 1.0 / ((kind == 3 ? hsSmall(sc) : w2 * w2) + eps);
-    sc.r2 = 1.0 / (w3 * w3 + eps);
+    const double w1 = sc.beta * sc.lam, w2 = sc.w2, w3 = sc.beta;
+    sc.r0 = 1.0 / sqEps(w1, eps, false);
+    sc.r1 = 1.0 / (kind == 3 ? __dadd_rn(hsSmall(sc), eps) : sqEps(w2, eps, false));
+    sc.r2 = 1.0 / sqEps(w3, eps, true);
   }
 }
 
 // y = G x with the eigenvalues prepared by socPrepareG (same structure as socApply).
-__device__ __forceinline__ void socApplyG(const SocScale& sc, const double* u, int d, const double* x, double* y) {
+template <int DIM>
+__device__ __forceinline__ void socApplyGDim(const SocScale& sc, const double* u, int dim, const double* x, double* y) {
+  const int d = DIM ? DIM : dim;
   const int kind = (int)sc.kind;
   if (kind == 0) {
     for (int i = 0; i < d; ++i) y[i] = sc.r0 * x[i];
@@ -200,13 +291,20 @@ __device__ __forceinline__ void socApplyG(const SocScale& sc, const double* u, i
   }
   const double x0 = x[0];
   double xf = 0.0;
-  for (int i = 1; i < d; ++i) xf += u[i] * x[i];
+#pragma unroll
+  for (int i = 1; i < d; ++i) xf = fma(u[i], x[i], xf);
   const double c1 = sc.qc * x0 + sc.qs * xf;
   const double c2 = -sc.qs * x0 + sc.qc * xf;
   const double y0 = sc.r0 * c1 * sc.qc - sc.r1 * c2 * sc.qs;
   const double yF = sc.r0 * c1 * sc.qs + sc.r1 * c2 * sc.qc;
+#pragma unroll
   for (int i = 1; i < d; ++i) y[i] = sc.r2 * (x[i] - xf * u[i]) + yF * u[i];
   y[0] = y0;
+}
+__device__ __forceinline__ void socApplyG(const SocScale& sc, const double* u, int d, const double* x, double* y) {
+  if (d == 3) socApplyGDim<3>(sc, u, d, x, y);
+  else if (d == 4) socApplyGDim<4>(sc, u, d, x, y);
+  else socApplyGDim<0>(sc, u, d, x, y);
 }
 
 // Jordan product (second_order_cone.cpp:43-48); out may alias neither u nor v.
@@ -227,8 +325,8 @@ __device__ __forceinline__ void socInverseProduct(const double* u, const double*
     nu += u[i] * w[i];
   }
   double rho = u0 * u0 - u1sq;
-  if (fabs(rho) < kTiny) rho = (rho >= 0 ? kTiny : -kTiny);
-  if (fabs(u0) < kTiny) u0 = kTiny;
+  if (lessBits(fabs(rho), kTiny)) rho = (nonNegBits(rho) ? kTiny : -kTiny);
+  if (lessBits(fabs(u0), kTiny)) u0 = kTiny;
   const double w0 = w[0];
   const double k1 = (nu / u0 - w0), k2 = (rho / u0);
   for (int i = 1; i < d; ++i) out[i] = (k1 * u[i] + k2 * w[i]) / rho;
@@ -248,26 +346,26 @@ __device__ __forceinline__ double socMaxStep(const double* x, const double* dx, 
   const double b = 2.0 * (p0 * d0 - p1d1);
   const double c = p0 * p0 - p1sq;
   double alpha = amax;
-  if (fabs(a) < kStepDegenerateEps) {
-    if (fabs(b) > kStepDegenerateEps) {
+  if (lessBits(fabs(a), kStepDegenerateEps)) {
+    if (lessBits(kStepDegenerateEps, fabs(b))) {
       const double r = -c / b;
-      if (r > 0 && (p0 + r * d0) >= 0) alpha = fmin(alpha, r);
+      if (posBits(r) && nonNegBits(p0 + r * d0)) alpha = minBits(alpha, r);
     }
     return alpha;
   }
   const double disc = b * b - 4.0 * a * c;
-  if (disc < 0) return alpha;
+  if (negBits(disc)) return alpha;
   const double sq = sqrt(disc);
-  const double q = (b >= 0) ? -0.5 * (b + sq) : -0.5 * (b - sq);
+  const double q = nonNegBits(b) ? -0.5 * (b + sq) : -0.5 * (b - sq);
   double r1, r2;
-  if (fabs(q) > kStepDegenerateEps) {
+  if (lessBits(kStepDegenerateEps, fabs(q))) {
     r1 = q / a;
     r2 = c / q;
   } else {
     r1 = r2 = -b / (2.0 * a);
   }
-  if (r1 > 0 && (p0 + r1 * d0) >= 0) alpha = fmin(alpha, r1);
-  if (r2 > 0 && (p0 + r2 * d0) >= 0) alpha = fmin(alpha, r2);
+  if (posBits(r1) && nonNegBits(p0 + r1 * d0)) alpha = minBits(alpha, r1);
+  if (posBits(r2) && nonNegBits(p0 + r2 * d0)) alpha = minBits(alpha, r2);
   return alpha;
 }
 
@@ -303,87 +401,139 @@ __host__ __device__ __forceinline__ double ladderBump(int level, double delta) {
 }
 
 // Dense Hs of one block (row-major d x d, d <= kRefDenseMaxDim) in the reference's arithmetic;
-// false for the identity fallback (W non-finite or max |W_ij| > 1e8), where Hs = I.
-static __device__ __noinline__ bool socRefHs(const double* s, const double* z, int d, double* Hs) {
-  double v[kRefDenseMaxDim];
+// false for the identity fallback (W non-finite or max |W_ij| > 1e8), where Hs = I (not written).
+// W and Hs are symmetric to the last bit here (doubling is exact, products commute and the sums run
+// over the same terms in the same order), so only their lower triangles are formed.
+template <int DIM>
+static __device__ __forceinline__ bool socRefHs(const double* s, const double* z, int dim, double* Hs) {
+  constexpr int kMax = DIM ? DIM : kRefDenseMaxDim;
+  const int d = DIM ? DIM : dim;
+  double v[kMax];
   double s1sq = 0.0, z1sq = 0.0, sz = 0.0;
+#pragma unroll
   for (int i = 1; i < d; ++i) {
     s1sq = __dadd_rn(s1sq, __dmul_rn(s[i], s[i]));
     z1sq = __dadd_rn(z1sq, __dmul_rn(z[i], z[i]));
   }
+#pragma unroll
   for (int i = 0; i < d; ++i) sz = __dadd_rn(sz, __dmul_rn(s[i], z[i]));
   const double s0 = s[0], z0 = z[0];
-  const double a =
-      __dsqrt_rn(fmax(fmax(__dsub_rn(__dmul_rn(s0, s0), s1sq), __dmul_rn(__dmul_rn(kTinyRel, s0), s0)), kAbsFloor));
-  const double b =
-      __dsqrt_rn(fmax(fmax(__dsub_rn(__dmul_rn(z0, z0), z1sq), __dmul_rn(__dmul_rn(kTinyRel, z0), z0)), kAbsFloor));
-  const double beta = fmin(fmax(__dsqrt_rn(__ddiv_rn(a, b)), __ddiv_rn(1.0, kBetaMax)), kBetaMax);
-  const double c = __dsqrt_rn(fmax(__ddiv_rn(__dadd_rn(__ddiv_rn(sz, __dmul_rn(a, b)), 1.0), 2.0), kTiny));
+  const double a = __dsqrt_rn(
+      maxBits(maxBits(__dsub_rn(__dmul_rn(s0, s0), s1sq), __dmul_rn(__dmul_rn(kTinyRel, s0), s0)), kAbsFloor));
+  const double b = __dsqrt_rn(
+      maxBits(maxBits(__dsub_rn(__dmul_rn(z0, z0), z1sq), __dmul_rn(__dmul_rn(kTinyRel, z0), z0)), kAbsFloor));
+  const double beta = minBits(maxBits(__dsqrt_rn(__ddiv_rn(a, b)), 1.0 / kBetaMax), kBetaMax);
+  const double c = __dsqrt_rn(maxBits(__dmul_rn(__dadd_rn(__ddiv_rn(sz, __dmul_rn(a, b)), 1.0), 0.5), kTiny));
   v[0] = __dadd_rn(__ddiv_rn(z0, b), __ddiv_rn(s0, a));
+#pragma unroll
   for (int i = 1; i < d; ++i) v[i] = __dadd_rn(__ddiv_rn(-z[i], b), __ddiv_rn(s[i], a));
   const double c2 = __dmul_rn(2.0, c);
+#pragma unroll
   for (int i = 0; i < d; ++i) v[i] = __ddiv_rn(v[i], c2);
-  v[0] = fmax(__dadd_rn(v[0], 1.0), kTiny);
+  v[0] = maxBits(__dadd_rn(v[0], 1.0), kTiny);
   const double nrm = __dsqrt_rn(__dmul_rn(2.0, v[0]));
+#pragma unroll
   for (int i = 0; i < d; ++i) v[i] = __ddiv_rn(v[i], nrm);
-  auto W = [&](int r, int cc) {
-    double w = __dmul_rn(__dmul_rn(2.0, v[r]), v[cc]);
-    if (r == cc) w = (r == 0) ? __dsub_rn(w, 1.0) : __dadd_rn(w, 1.0);
-    return __dmul_rn(w, beta);
-  };
+  double W[kMax * kMax];
   double wmax = 0.0;
   bool finite = true;
+#pragma unroll
   for (int r = 0; r < d; ++r)
-    for (int cc = 0; cc < d; ++cc) {
-      const double w = W(r, cc);
-      finite = finite && isfinite(w);
-      wmax = fmax(wmax, fabs(w));
+#pragma unroll
+    for (int cc = 0; cc <= r; ++cc) {
+      double w = __dmul_rn(__dmul_rn(2.0, v[r]), v[cc]);
+      if (r == cc) w = (r == 0) ? __dsub_rn(w, 1.0) : __dadd_rn(w, 1.0);
+      w = __dmul_rn(w, beta);
+      finite = finite && finiteBits(w);
+      wmax = maxBits(wmax, fabs(w));
+      W[r * kMax + cc] = W[cc * kMax + r] = w;
     }
-  if (finite && wmax <= kWMax) {
-    for (int r = 0; r < d; ++r)
-      for (int cc = 0; cc < d; ++cc) {
-        double acc = 0.0;
-        for (int k = 0; k < d; ++k) acc = __dadd_rn(acc, __dmul_rn(W(r, k), W(k, cc)));
-        finite = finite && isfinite(acc);
-        Hs[r * d + cc] = acc;
-      }
-    if (finite) return true;
-  }
+  if (!finite || lessBits(kWMax, wmax)) return false;
+#pragma unroll
   for (int r = 0; r < d; ++r)
-    for (int cc = 0; cc < d; ++cc) Hs[r * d + cc] = (r == cc) ? 1.0 : 0.0;
-  return false;
+#pragma unroll
+    for (int cc = 0; cc <= r; ++cc) {
+      double acc = 0.0;
+#pragma unroll
+      for (int k = 0; k < d; ++k) acc = __dadd_rn(acc, __dmul_rn(W[r * kMax + k], W[k * kMax + cc]));
+      finite = finite && finiteBits(acc);
+      Hs[r * kMax + cc] = acc;
+    }
+  return finite;
+}
+
+// Whether every dense pivot of a block passes at level 0 whatever the rounding, from a bound in
+// FP32: the largest eigenvalue of Hs is at most (a / b)(s0 / a + z0 / b)^2, a^2 = s0^2 - |s1|^2, b^2 =
+// z0^2 - |z1|^2. The dense entries and the LDL' of d <= 8 rows together change Hs by less than
+// 1000 eps times it, and every pivot of an exact Hs + sregA I is at least sregA; so while 1000 eps
+// |Hs| < sregA / 4 and deps < sregA / 4 the pivots pass. The FP32 values carry relative errors of
+// about 1e-6 (the margins s0 - |s1| are used only above 1e-3 s0), far inside the factor four.
+__device__ __forceinline__ bool socPivotsPass(const double* s, const double* z, int d, double sregA, double deps) {
+  const float s0 = (float)s[0], z0 = (float)z[0];
+  float s1 = 0.0f, z1 = 0.0f;
+  for (int i = 1; i < d; ++i) {
+    const float si = (float)s[i], zi = (float)z[i];
+    s1 = fmaf(si, si, s1);
+    z1 = fmaf(zi, zi, z1);
+  }
+  s1 = sqrtf(s1);
+  z1 = sqrtf(z1);
+  const float sm = s0 - s1, zm = z0 - z1;
+  if (!(sm > 1e-3f * s0) || !(zm > 1e-3f * z0) || !(s0 > 1e-15f) || !(z0 > 1e-15f) || !(s0 < 1e15f) || !(z0 < 1e15f))
+    return false;
+  const float a = sqrtf(sm * (s0 + s1)), b = sqrtf(zm * (z0 + z1));
+  const float t = s0 / a + z0 / b;
+  const float hs = (a / b) * t * t, reg = (float)sregA;
+  return hs * (1000.0f * 2.22e-16f) < 0.25f * reg && (float)deps < 0.25f * reg;
 }
 
 // The first ladder level (attempt index, 0..17) at which the block's dense pivots all pass, or
 // 18 when none does; the search starts at startLevel (a block that passes there returns
 // startLevel). Blocks of one row or above kRefDenseMaxDim rows: 0.
-static __device__ __noinline__ int socRefLadderLevel(const double* s, const double* z, int d, double sregA,
-                                                     double deps, double delta, int startLevel) {
-  if (d > kRefDenseMaxDim || d < 2) return 0;
-  double Hs[kRefDenseMaxDim * kRefDenseMaxDim];
-  if (!socRefHs(s, z, d, Hs)) return 0;  // Hs = I: every pivot passes
+template <int DIM>
+static __device__ __noinline__ int socRefLadderDim(const double* s, const double* z, int dim, double sregA, double deps,
+                                                   double delta, int startLevel) {
+  constexpr int kMax = DIM ? DIM : kRefDenseMaxDim;
+  const int d = DIM ? DIM : dim;
+  double Hs[kMax * kMax];
+  if (!socRefHs<DIM>(s, z, d, Hs)) return 0;  // Hs = I: every pivot passes
   for (int level = startLevel; level < kLadderLevels; ++level) {
     const double ea = ladderBump(level, delta);
     // up-looking LDL' of -(Hs + sregA I) - ea I in natural order, QDLDL's operation order
-    double L[kRefDenseMaxDim * kRefDenseMaxDim], Dinv[kRefDenseMaxDim], y[kRefDenseMaxDim];
+    double L[kMax * kMax], Dinv[kMax], y[kMax];
     bool ok = true;
-    for (int k = 0; k < d && ok; ++k) {
-      double Dk = __dsub_rn(-Hs[k * d + k], sregA);
-      if (ea != 0.0) Dk = __dsub_rn(Dk, ea);
-      for (int r = 0; r < k; ++r) y[r] = -Hs[k * d + r];
+#pragma unroll
+    for (int k = 0; k < d; ++k) {
+      if (!ok) break;
+      double Dk = __dsub_rn(-Hs[k * kMax + k], sregA);
+      if (!zeroBits(ea)) Dk = __dsub_rn(Dk, ea);
+#pragma unroll
+      for (int r = 0; r < k; ++r) y[r] = -Hs[k * kMax + r];
+#pragma unroll
       for (int cc = 0; cc < k; ++cc) {
         const double yc = y[cc];
-        for (int r = cc + 1; r < k; ++r) y[r] = __dsub_rn(y[r], __dmul_rn(L[r * kRefDenseMaxDim + cc], yc));
+#pragma unroll
+        for (int r = cc + 1; r < k; ++r) y[r] = __dsub_rn(y[r], __dmul_rn(L[r * kMax + cc], yc));
         const double l = __dmul_rn(yc, Dinv[cc]);
-        L[k * kRefDenseMaxDim + cc] = l;
+        L[k * kMax + cc] = l;
         Dk = __dsub_rn(Dk, __dmul_rn(yc, l));
       }
-      ok = isfinite(Dk) && fabs(Dk) > deps;
-      Dinv[k] = __ddiv_rn(1.0, Dk);
+      ok = finiteBits(Dk) && lessBits(deps, fabs(Dk));
+      if (k + 1 < d) Dinv[k] = __ddiv_rn(1.0, Dk);
     }
     if (ok) return level;
   }
   return kLadderLevels;
+}
+
+__device__ __forceinline__ int socRefLadderLevel(const double* s, const double* z, int d, double sregA, double deps,
+                                                 double delta, int startLevel) {
+  if (d > kRefDenseMaxDim || d < 2) return 0;
+  if (socPivotsPass(s, z, d, sregA, deps)) return startLevel;
+  if (d == 2) return socRefLadderDim<2>(s, z, d, sregA, deps, delta, startLevel);
+  if (d == 3) return socRefLadderDim<3>(s, z, d, sregA, deps, delta, startLevel);
+  if (d == 4) return socRefLadderDim<4>(s, z, d, sregA, deps, delta, startLevel);
+  return socRefLadderDim<0>(s, z, d, sregA, deps, delta, startLevel);
 }
 
 __device__ __forceinline__ double socMargin(const double* x, int d) {

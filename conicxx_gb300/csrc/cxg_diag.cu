@@ -87,7 +87,7 @@ __global__ void coneEvalKernel(int op, int zero, int nn, int nsoc, const int* of
   }
   if (params) {
     for (int b = threadIdx.x; b < nsoc; b += blockDim.x) {
-      params[8 * b + 0] = sp[b].kind;
+      params[8 * b + 0] = (double)sp[b].kind;
       params[8 * b + 1] = sp[b].beta;
       params[8 * b + 2] = sp[b].lam;
       params[8 * b + 3] = sp[b].qc;
@@ -161,7 +161,7 @@ extern "C" int cxg_cones_eval(int op, int zero_dim, int nonneg_dim, int n_soc, c
   DG_CUDA(cudaMemcpy(dZ, z, sizeof(double) * (size_t)m, cudaMemcpyHostToDevice));
   DG_CUDA(cudaMemcpy(dU, u, sizeof(double) * (size_t)m, cudaMemcpyHostToDevice));
   DG_CUDA(cudaMemcpy(dV, v ? v : u, sizeof(double) * (size_t)m, cudaMemcpyHostToDevice));
-  const size_t shBytes = sizeof(double) * (2 * (size_t)m + 8 * (size_t)n_soc);
+  const size_t shBytes = sizeof(double) * (2 * (size_t)m + kSocScaleDoubles * (size_t)n_soc);
   if (shBytes > 200 * 1024) {
     for (void* p : bufs) cudaFree(p);
     lastErrorRef() = "cxg_cones_eval: cone set too large";

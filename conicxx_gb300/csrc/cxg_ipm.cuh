@@ -58,66 +58,101 @@ __device__ __forceinline__ double csrDot(const double* __restrict__ val, const i
   return (a0 + a1) + (a2 + a3);
 }
 
-// Finiteness by the exponent bits (an integer test; FP64 compares run on the scarce FP64 pipe).
-__device__ __forceinline__ bool finiteBits(double v) {
-  return ((__double_as_longlong(v) >> 52) & 0x7ff) != 0x7ff;
-}
 
 // ------------------------------------------------------------------------------------------
 // block reductions (deterministic: fixed summation order, identical result in every thread)
 // ------------------------------------------------------------------------------------------
+// An FP64 instruction holds its sub-partition's FP64 unit for 64 cycles whatever the number of
+// active lanes, so the trees below pack the additions of several values (and of several warps'
+// partials) into one instruction's lanes, and comparisons run on the integer pipe. Six sums over
+// 256 threads take 14 FP64 instructions a warp where one tree per value took 72.
+
+// Lane of warpSums' result k of K: the bit pattern of k, lowest bit in lane bit 4.
+__device__ __forceinline__ int sumLane(int k) { return ((k & 1) << 4) | ((k & 2) << 2) | (k & 4); }
+
+// Sums of K values (K <= 8) over the warp: v_k = ((v_k[0] + v_k[16]) + (v_k[8] + v_k[24])) + ..., the
+// shuffle-down tree's order (additions commute), in lane sumLane(k) of the result.
+template <int K>
+__device__ __forceinline__ double warpSums(const double (&v)[K]) {
+  const int lane = threadIdx.x & 31;
+  double w[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) w[k] = v[k];
+  int n = K;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < (K + 1) / 2; ++i) {
+      if (2 * i + 1 < n) {  // two values: the lower half of the lanes goes on with the first
+        const double keep = up ? w[2 * i + 1] : w[2 * i], give = up ? w[2 * i] : w[2 * i + 1];
+        w[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      } else if (2 * i < n) {
+        w[i] = w[2 * i] + __shfl_xor_sync(0xffffffffu, w[2 * i], o);
+      }
+    }
+    n = (n + 1) / 2;
+  }
+  return w[0];
+}
+
+// Totals of the warps' partials red[k * 16 + w], w < nw, pairwise over the warps, of the (up to
+// 32 / nw) values from k0 on: value k0 + i's in the lanes i * nw .. of the calling warp. Block
+// sizes of 1, 2, 4 or 8 warps.
+__device__ __forceinline__ double warpTotals(const double* red, int k0, int nw) {
+  const int lane = threadIdx.x & 31;
+  double t = red[min(k0 + lane / nw, 7) * 16 + lane % nw];
+  for (int o = 1; o < nw; o <<= 1) t = t + __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
+}
+
+template <int K>
+__device__ __forceinline__ void blockPartials(const double (&v)[K], double* red) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const double p = warpSums<K>(v);
+  const int k = ((lane >> 4) & 1) | ((lane >> 2) & 2) | (lane & 4);
+  __syncthreads();  // the last reduction's readers are done with red
+  if (lane == sumLane(k) && k < K) red[k * 16 + w] = p;
+  __syncthreads();
+}
+
 template <int K>
 __device__ __forceinline__ void blockSum(double (&v)[K], double* red) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int nw = blockDim.x >> 5;
+  blockPartials<K>(v, red);
+  if (nw & (nw - 1)) {  // a number of warps that is no power of two: in sequence
 #pragma unroll
-  for (int k = 0; k < K; ++k)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-  __syncthreads();
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < K; ++k) red[k * 16 + w] = v[k];
-  __syncthreads();
-  // pairwise over the warps' partials (depth log2(nw), not nw: FP64 adds are long-latency here)
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const double* r = red + k * 16;
-    double t;
-    if (nw == 1) t = r[0];
-    else if (nw == 2) t = r[0] + r[1];
-    else if (nw == 4) t = (r[0] + r[1]) + (r[2] + r[3]);
-    else if (nw == 8) t = ((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7]));
-    else {
-      t = 0.0;
-      for (int j = 0; j < nw; ++j) t += r[j];
+    for (int k = 0; k < K; ++k) {
+      double t = 0.0;
+      for (int j = 0; j < nw; ++j) t += red[k * 16 + j];
+      v[k] = t;
     }
-    v[k] = t;
+    return;
+  }
+#pragma unroll
+  for (int k0 = 0; k0 < K; k0 += 4) {
+    const double t = warpTotals(red, k0, nw);
+#pragma unroll
+    for (int k = k0; k < min(k0 + 4, K); ++k) v[k] = __shfl_sync(0xffffffffu, t, (k - k0) * nw);
   }
 }
 
 __device__ __forceinline__ double blockMin(double v, double* red) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_down_sync(0xffffffffu, v, o));
+  for (int o = 16; o > 0; o >>= 1) v = minBits(v, __shfl_xor_sync(0xffffffffu, v, o));
   __syncthreads();
   if (lane == 0) red[w] = v;
   __syncthreads();
   double t = red[0];
-  for (int j = 1; j < nw; ++j) t = fmin(t, red[j]);
+  for (int j = 1; j < nw; ++j) t = minBits(t, red[j]);
   return t;
 }
 
-__device__ __forceinline__ int blockOrInt(int v, int* redi) {
-  __syncthreads();
-  if (threadIdx.x == 0) redi[0] = 0;
-  __syncthreads();
-  if (v) atomicOr(redi, v);
-  __syncthreads();
-  return redi[0];
-}
+__device__ __forceinline__ bool blockAny(int v) { return __syncthreads_or(v) != 0; }
 
 __device__ __forceinline__ int blockMaxInt(int v, int* redi) {
-  __syncthreads();
+  if (!__syncthreads_or(v > 0)) return 0;
   if (threadIdx.x == 0) redi[0] = 0;
   __syncthreads();
   if (v) atomicMax(redi, v);
@@ -154,7 +189,7 @@ struct Ctx {
 // scalar slots in Ctx::sc
 enum {
   SC_TAU = 0, SC_KAPPA, SC_EXTRA_P, SC_EXTRA_A, SC_USE64, SC_NFB, SC_RSTEPS, SC_MAXREL,
-  SC_ATTEMPTS, SC_FACTOK, SC_GMRES, SC_ITREL, SC_FAULTF, SC_FAULTS, SC_ESC, SC_SOCLVL, SC_HSFLOOR, SC_COUNT
+  SC_ATTEMPTS, SC_FACTOK, SC_GMRES, SC_ITREL, SC_FAULTF, SC_FAULTS, SC_ESC, SC_SOCLVL, SC_HSFLOOR, SC_PXOK, SC_COUNT
 };
 
 
@@ -209,24 +244,34 @@ static __device__ __noinline__ void loadInstance(Ctx& c, const LaunchArgs& a) {
 // (kind 3, hsSmall; flag SC_HSFLOOR).
 static __device__ __noinline__ void coneUpdateScaling(Ctx& c, const DevSettings& st, const double* s, const double* z) {
   int lvl = 0;
-  FOR_T(t, c.l + c.nsoc) {
-    if (t < c.l) {
-      const int r = c.p + t;
-      c.cw[r] = sqrt(s[r] / z[r]);  // nonnegative_cone.cpp:24
-    } else {
-      const int b = t - c.l;
-      const int off = c.socOff[b], d = c.socDim[b];
-      socUpdateScaling(s + off, z + off, d, c.sp[b], c.cu + off);
-      if (st.soc_ref_dense && st.linear_solver != 2)
+  // three lists of work, one after another over the threads: the SOC blocks' scaling, their pivot
+  // tests and the NN rows; each list starts at a warp of its own (a warp with lanes of two lists
+  // would run both, one after the other)
+  constexpr int al = 31;
+  const bool test = st.soc_ref_dense && st.linear_solver != 2;
+  const int o1 = (c.nsoc + al) & ~al, o2 = o1 + (test ? ((c.nsoc + al) & ~al) : 0);
+  FOR_T(t, o2 + c.l) {
+    if (t < o1) {
+      if (t < c.nsoc) {
+        const int off = c.socOff[t], d = c.socDim[t];
+        socUpdateScaling(s + off, z + off, d, c.sp[t], c.cu + off);
+      }
+    } else if (t < o2) {
+      if (t - o1 < c.nsoc) {
+        const int off = c.socOff[t - o1], d = c.socDim[t - o1];
         lvl = max(lvl, socRefLadderLevel(s + off, z + off, d, st.static_reg_A, st.dynamic_reg_eps,
                                          st.dynamic_reg_delta, lvl));
+      }
+    } else {
+      const int r = c.p + (t - o2);
+      c.cw[r] = sqrt(s[r] / z[r]);  // nonnegative_cone.cpp:24
     }
   }
   const int mx = blockMaxInt(lvl, c.redi);
   // once a block's dense form has lost its small eigenvalue (the reference's pivot test fails),
   // the instance's blocks take Hs at the dense form's resolution, from this iteration on (sticky)
   const bool floorHs = c.sc[SC_HSFLOOR] != 0.0 || mx > 0;
-  if (floorHs) FOR_T(b, c.nsoc) if (c.sp[b].kind == 2.0) c.sp[b].kind = 3.0;
+  if (floorHs) FOR_T(b, c.nsoc) if (c.sp[b].kind == 2) c.sp[b].kind = 3;
   __syncthreads();
   if (threadIdx.x == 0) {
     c.sc[SC_SOCLVL] = (double)mx;
@@ -238,12 +283,12 @@ static __device__ __noinline__ void coneUpdateScaling(Ctx& c, const DevSettings&
 // out = f(W) x on every cone row (Zero rows: 0, or eps * x for kHsEps).
 static __device__ __noinline__ void coneApply(Ctx& c, int f, double eps, const double* x, double* out) {
   FOR_T(r, c.p) out[r] = (f == kHsEps) ? eps * x[r] : 0.0;
-  FOR_T(t, c.l + c.nsoc) {
-    if (t < c.l) {
-      const int r = c.p + t;
+  FOR_T(t, c.l + c.nsoc) {  // the longer SOC units first, packed into as few warps as they fill
+    if (t >= c.nsoc) {
+      const int r = c.p + (t - c.nsoc);
       out[r] = wfun(f, c.cw[r], eps) * x[r];
     } else {
-      const int b = t - c.l;
+      const int b = t;
       const int off = c.socOff[b], d = c.socDim[b];
       socApply(c.sp[b], c.cu + off, d, f, eps, x + off, out + off);
     }
@@ -255,11 +300,11 @@ static __device__ __noinline__ void coneApply(Ctx& c, int f, double eps, const d
 static __device__ __noinline__ void coneApplyG(Ctx& c, const double* x, double* out) {
   FOR_T(r, c.p) out[r] = 0.0;
   FOR_T(t, c.l + c.nsoc) {
-    if (t < c.l) {
-      const int r = c.p + t;
+    if (t >= c.nsoc) {
+      const int r = c.p + (t - c.nsoc);
       out[r] = c.cu[r] * x[r];
     } else {
-      const int b = t - c.l;
+      const int b = t;
       const int off = c.socOff[b], d = c.socDim[b];
       socApplyG(c.sp[b], c.cu + off, d, x + off, out + off);
     }
@@ -271,11 +316,11 @@ static __device__ __noinline__ void coneApplyG(Ctx& c, const double* x, double* 
 static __device__ __noinline__ void coneProduct(Ctx& c, bool inverse, const double* u, const double* v, double* out) {
   FOR_T(r, c.p) out[r] = 0.0;
   FOR_T(t, c.l + c.nsoc) {
-    if (t < c.l) {
-      const int r = c.p + t;
+    if (t >= c.nsoc) {
+      const int r = c.p + (t - c.nsoc);
       out[r] = inverse ? v[r] / u[r] : u[r] * v[r];
     } else {
-      const int b = t - c.l;
+      const int b = t;
       const int off = c.socOff[b], d = c.socDim[b];
       if (inverse) socInverseProduct(u + off, v + off, d, out + off);
       else socProduct(u + off, v + off, d, out + off);
@@ -284,17 +329,25 @@ static __device__ __noinline__ void coneProduct(Ctx& c, bool inverse, const doub
   __syncthreads();
 }
 
-// ConeSet::maxStep (cone_set.cpp:108-115) as a block-wide min of per-unit limits.
-static __device__ __noinline__ double coneMaxStep(Ctx& c, const double* x, const double* dx, double amax) {
+// ConeSet::maxStep (cone_set.cpp:108-115) of (s, ds) and (z, dz) as one block-wide min of per-unit
+// limits.
+static __device__ __noinline__ double coneMaxStep2(Ctx& c, double amax) {
   double al = amax;
-  FOR_T(t, c.l + c.nsoc) {
-    if (t < c.l) {
+  const int nu = c.l + c.nsoc;
+  FOR_T(t2, 2 * nu) {  // the SOC blocks of both, then the NN rows of both
+    const bool soc = t2 < 2 * c.nsoc;
+    const int t1 = soc ? t2 : t2 - 2 * c.nsoc, len = soc ? c.nsoc : c.l;
+    const bool second = t1 >= len;
+    const int t = second ? t1 - len : t1;
+    const double* x = second ? c.s : c.z;
+    const double* dx = second ? c.ds : c.dz;
+    if (!soc) {
       const int r = c.p + t;
-      if (dx[r] < 0) al = fmin(al, -x[r] / dx[r]);
+      if (negBits(dx[r])) al = minBits(al, -x[r] / dx[r]);
     } else {
-      const int b = t - c.l;
+      const int b = t;
       const int off = c.socOff[b], d = c.socDim[b];
-      al = fmin(al, socMaxStep(x + off, dx + off, d, amax));
+      al = minBits(al, socMaxStep(x + off, dx + off, d, amax));
     }
   }
   return blockMin(al, c.red);
@@ -355,17 +408,21 @@ static __device__ __noinline__ void pmul(Ctx& c, const double* x, double* y) {
 }
 
 // res = rhs - K sol for the statically-regularised K (the matrix refinement targets,
-// kkt_system.cpp:296-311): top = (P + epsP I) x + A'z, bottom = A x - (Hs + epsA I) z.
+// kkt_system.cpp:296-311): top = (P + epsP I) x + A'z, bottom = A x - (Hs + epsA I) z. Returns
+// |res| / rhsNorm; rhsNorm is computed when `first` (the first residual for this rhs), and P x is
+// left in c.tn.
 static __device__ __noinline__ double kktResidualImpl(Ctx& c, const DevSettings& st, const double* rhs, const double* sol,
-                                  double* res, double& rhsNorm) {
+                                  double* res, double& rhsNorm, bool first) {
   const int n = c.n, m = c.m;
   const double* xs = sol;
   const double* zs = sol + n;
   double acc2[2] = {0.0, 0.0};
   FOR_T(t, n + m) {
     if (t < n) {
-      double acc = st.static_reg_P * xs[t] + csrDot(c.Pv, c.psCol, c.psRow[t], c.psRow[t + 1], xs);
+      const double px = csrDot(c.Pv, c.psCol, c.psRow[t], c.psRow[t + 1], xs);
+      double acc = __dadd_rn(__dmul_rn(st.static_reg_P, xs[t]), px);
       acc += csrDot(c.Av, c.ai, c.ap[t], c.ap[t + 1], zs);
+      c.tn[t] = px;
       res[t] = rhs[t] - acc;
     } else {
       const int r = t - n;
@@ -379,13 +436,29 @@ static __device__ __noinline__ double kktResidualImpl(Ctx& c, const DevSettings&
   coneApply(c, kHsEps, st.static_reg_A, zs, c.tm2);
   FOR_T(r, m) res[n + r] += c.tm2[r];
   __syncthreads();
-  FOR_T(t, n + m) {
-    acc2[0] += res[t] * res[t];
-    acc2[1] += rhs[t] * rhs[t];
+  FOR_T(t, n + m) acc2[0] += res[t] * res[t];
+  if (first) FOR_T(t, n + m) acc2[1] += rhs[t] * rhs[t];
+  // both norms and the quotient by one warp: a square root and a division hold the FP64 unit for
+  // some 600 cycles each
+  if (blockDim.x & (blockDim.x - 1)) {
+    blockSum<2>(acc2, c.red);
+    if (first) rhsNorm = fmax(sqrt(acc2[1]), 1e-30);
+    return sqrt(acc2[0]) / rhsNorm;
   }
-  blockSum<2>(acc2, c.red);
-  rhsNorm = fmax(sqrt(acc2[1]), 1e-30);
-  return sqrt(acc2[0]) / rhsNorm;
+  const int nw = blockDim.x >> 5;
+  blockPartials<2>(acc2, c.red);
+  if (threadIdx.x < 32) {
+    const double norm = sqrt(warpTotals(c.red, 0, nw));
+    const double rn = first ? fmax(__shfl_sync(0xffffffffu, norm, nw), 1e-30) : rhsNorm;
+    const double rel = norm / rn;
+    if (threadIdx.x == 0) {
+      c.red[120] = rel;
+      c.red[121] = rn;
+    }
+  }
+  __syncthreads();
+  rhsNorm = c.red[121];
+  return c.red[120];
 }
 
 // y = K sol for the same statically regularised K (the operator of the GMRES refinement).
@@ -412,9 +485,9 @@ static __device__ __noinline__ void kktApply(Ctx& c, const DevSettings& st, cons
 }
 
 static __device__ double kktResidual(Ctx& c, const DevSettings& st, const double* rhs, const double* sol, double* res,
-                              double& rhsNorm) {
+                              double& rhsNorm, bool first) {
   const long long t0 = (st.record_timings && threadIdx.x == 0) ? clock64() : 0;
-  const double r = kktResidualImpl(c, st, rhs, sol, res, rhsNorm);
+  const double r = kktResidualImpl(c, st, rhs, sol, res, rhsNorm, first);
   if (st.record_timings && threadIdx.x == 0) timers(c)[TM_RESID] += clock64() - t0;
   return r;
 }
@@ -542,30 +615,29 @@ __device__ __forceinline__ T groupSum(T v, int s) {
 // y <- M^-1 y for the factored tiled root; y has Tn*32 entries (padding entries are zero).
 // Every block product (the diagonal tile's Linv and each off-diagonal tile) is a set of 32-term
 // dot products, split over s lanes per row (dotSplit) and reduced by shuffles, so that the few
-// rows of the late steps still occupy the whole block.
+// rows of the late steps still occupy the whole block. A solved tile goes to a buffer in the
+// reduction area first, so that a step takes two barriers. (Half of the warps on the chain of
+// diagonal tiles and half on the rows beyond, with one barrier, was slower by a third: the chain
+// is bound by the issue of its double-float operations, not by the barriers.)
 template <typename T>
 __device__ void denseSolve(Ctx& c, const T* M, T* y) {
   const int Tn = rootTiles(c.nr);
   const int nth = blockDim.x;
+  const int sd = dotSplit(32), wd = 32 / sd;
+  const int di = (int)threadIdx.x / sd, dp = (int)threadIdx.x % sd;  // row and part in a diagonal product
+  T* x = reinterpret_cast<T*>(c.red);
   // forward: y_J = Linv_JJ y_J, then y_I -= L_IJ y_J for I > J
   for (int J = 0; J < Tn; ++J) {
     const T* Ajj = M + tileBase(Tn, J, J);
     T* yJ = y + J * 32;
-    {
-      const int sd = dotSplit(32), w = 32 / sd;
-      T tot = (T)0;
-      int i = 0, p = 0;
-      if ((int)threadIdx.x < 32 * sd) {
-        i = threadIdx.x / sd;
-        p = threadIdx.x % sd;
-        T acc = (T)0;
-        for (int col = p * w; col < (p + 1) * w && col < i; ++col) acc = accT(acc, Ajj[i * kTileLd + col], yJ[col]);
-        tot = groupSum(accEnd(acc), sd);
-      }
-      __syncthreads();
-      if ((int)threadIdx.x < 32 * sd && p == 0) yJ[i] = yJ[i] + tot;
-      __syncthreads();
+    if ((int)threadIdx.x < 32 * sd) {
+      T acc = (T)0;
+      for (int col = dp * wd; col < (dp + 1) * wd && col < di; ++col) acc = accT(acc, Ajj[di * kTileLd + col], yJ[col]);
+      const T tot = groupSum(accEnd(acc), sd);
+      if (dp == 0) x[di] = yJ[di] + tot;
     }
+    __syncthreads();
+    if (threadIdx.x < 32) yJ[threadIdx.x] = x[threadIdx.x];
     const int rows = (Tn - J - 1) * 32;
     if (rows > 0) {
       const int s = dotSplit(rows), w = 32 / s;
@@ -575,7 +647,7 @@ __device__ void denseSolve(Ctx& c, const T* M, T* y) {
         const T* Lij = M + tileBase(Tn, I, J);
         T acc = (T)0;
 #pragma unroll 4
-        for (int col = p * w; col < (p + 1) * w; ++col) acc = accT(acc, Lij[col * kTileLd + rr], yJ[col]);
+        for (int col = p * w; col < (p + 1) * w; ++col) acc = accT(acc, Lij[col * kTileLd + rr], x[col]);
         acc = groupSum(accEnd(acc), s);
         if (p == 0) y[I * 32 + rr] -= acc;
       }
@@ -591,34 +663,27 @@ __device__ void denseSolve(Ctx& c, const T* M, T* y) {
   for (int J = Tn - 1; J >= 0; --J) {
     const T* Ajj = M + tileBase(Tn, J, J);
     T* yJ = y + J * 32;
-    {
-      const int sd = dotSplit(32), w = 32 / sd;
-      T tot = (T)0;
-      int i = 0, p = 0;
-      if ((int)threadIdx.x < 32 * sd) {
-        i = threadIdx.x / sd;
-        p = threadIdx.x % sd;
-        T acc = (T)0;
-        for (int row = p * w; row < (p + 1) * w; ++row)
-          if (row > i) acc = accT(acc, Ajj[row * kTileLd + i], yJ[row]);
-        tot = groupSum(accEnd(acc), sd);
-      }
-      __syncthreads();
-      if ((int)threadIdx.x < 32 * sd && p == 0) yJ[i] = yJ[i] + tot;
-      __syncthreads();
-    }
-    if (J == 0) break;
-    const int rows = J * 32;
-    const int s = dotSplit(rows), w = 32 / s;
-    for (int t = threadIdx.x; t < rows * s; t += nth) {
-      const int row = t / s, p = t % s;
-      const int K = row / 32, cc = row % 32;
-      const T* Ljk = M + tileBase(Tn, J, K);
+    if ((int)threadIdx.x < 32 * sd) {
       T acc = (T)0;
+      for (int row = max(dp * wd, di + 1); row < (dp + 1) * wd; ++row) acc = accT(acc, Ajj[row * kTileLd + di], yJ[row]);
+      const T tot = groupSum(accEnd(acc), sd);
+      if (dp == 0) x[di] = yJ[di] + tot;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) yJ[threadIdx.x] = x[threadIdx.x];
+    const int rows = J * 32;
+    if (rows > 0) {
+      const int s = dotSplit(rows), w = 32 / s;
+      for (int t = threadIdx.x; t < rows * s; t += nth) {
+        const int row = t / s, p = t % s;
+        const int K = row / 32, cc = row % 32;
+        const T* Ljk = M + tileBase(Tn, J, K);
+        T acc = (T)0;
 #pragma unroll 4
-      for (int r2 = p * w; r2 < (p + 1) * w; ++r2) acc = accT(acc, Ljk[cc * kTileLd + r2], yJ[r2]);
-      acc = groupSum(accEnd(acc), s);
-      if (p == 0) y[K * 32 + cc] -= acc;
+        for (int r2 = p * w; r2 < (p + 1) * w; ++r2) acc = accT(acc, Ljk[cc * kTileLd + r2], x[r2]);
+        acc = groupSum(accEnd(acc), s);
+        if (p == 0) y[K * 32 + cc] -= acc;
+      }
     }
     __syncthreads();
   }
@@ -2173,11 +2238,11 @@ __device__ __noinline__ void reducedSolve(Ctx& c, const DevSettings& st, const T
   }
   __syncthreads();
   FOR_T(t, c.l + c.nsoc) {
-    if (t < c.l) {
-      const int r = p + t;
+    if (t >= c.nsoc) {
+      const int r = p + (t - c.nsoc);
       sol[n + r] = c.tm[r] * c.cu[r];
     } else {
-      const int b = t - c.l;
+      const int b = t;
       const int off = c.socOff[b], d = c.socDim[b];
       socApplyG(c.sp[b], c.cu + off, d, c.tm + off, sol + n + off);
     }
@@ -2274,7 +2339,7 @@ __device__ void solveOnce(Ctx& c, const DevSettings& st, const FactState& fs, co
 static __device__ __noinline__ bool vecFinite(Ctx& c, const double* v, int len) {
   int bad = 0;
   FOR_T(i, len) bad |= !finiteBits(v[i]);
-  return blockOrInt(bad, c.redi) == 0;
+  return !blockAny(bad);
 }
 
 // Refinement of the whole-GPU form: restarted GMRES in FP64 on the statically regularised K
@@ -2293,7 +2358,7 @@ __device__ void solveOnce(Ctx& c, const DevSettings& st, const FactState& fs, co
 
 template <typename FT, bool G>
 __device__ __noinline__ double gmresRefine(Ctx& c, const DevSettings& st, const FactState& fs, const double* rhs,
-                                           double* sol, double rel, double rhsNorm) {
+                                           double* sol, double rel, double rhsNorm, bool& pxOk) {
   const int N = c.n + c.m;
   const int64_t ld = ((int64_t)N + 1) & ~int64_t(1);
   constexpr int hl = kGmresDim + 1;  // leading dimension of H (column-major)
@@ -2372,9 +2437,10 @@ __device__ __noinline__ double gmresRefine(Ctx& c, const DevSettings& st, const 
       c.cor[t] = acc;
     }
     __syncthreads();
-    double rn = 1.0;
-    const double relNew = kktResidual(c, st, rhs, c.cor, c.res, rn);
-    if (!(relNew < rel)) break;  // no progress (or a non-finite candidate): keep sol
+    double rn = rhsNorm;
+    const double relNew = kktResidual(c, st, rhs, c.cor, c.res, rn, false);
+    pxOk = relNew < rel;
+    if (!pxOk) break;  // no progress (or a non-finite candidate): keep sol
     FOR_T(t, N) sol[t] = c.cor[t];
     __syncthreads();
     rel = relNew;
@@ -2385,7 +2451,8 @@ __device__ __noinline__ double gmresRefine(Ctx& c, const DevSettings& st, const 
 }
 
 // KktSystem::solve (kkt_system.cpp:296-311) incl. escalateAndResolve (:266-294), plus the
-// MIXED-precision fallback to the double-float factor. Returns the final relative residual.
+// MIXED-precision fallback to the double-float factor. Returns the final relative residual, and
+// in SC_PXOK whether c.tn holds P sol (the last residual's product, of the solution kept).
 template <typename FT, bool G = false>
 __device__ bool factorizeWithRetry(Ctx& c, const DevSettings& st, FactState& fs);
 
@@ -2418,11 +2485,12 @@ __device__ __noinline__ double kktSolveImpl(Ctx& c, const DevSettings& st, FactS
       }
     }
     double rhsNorm = 1.0;
-    double rel = kktResidual(c, st, rhs, sol, c.res, rhsNorm);
+    bool pxOk = true;
+    double rel = kktResidual(c, st, rhs, sol, c.res, rhsNorm, true);
     const bool fp32Factor = (sizeof(FT) == 4) && !fs.use64;
     const int maxRef = G ? 0 : (fp32Factor ? st.mixed_refine_max_iter : st.refine_max_iter);
     if constexpr (G) {
-      if (rel > st.refine_tol) rel = gmresRefine<FT, G>(c, st, fs, rhs, sol, rel, rhsNorm);
+      if (rel > st.refine_tol) rel = gmresRefine<FT, G>(c, st, fs, rhs, sol, rel, rhsNorm, pxOk);
     }
     int steps = 0;
     for (int it = 0; it < maxRef && rel > st.refine_tol; ++it) {
@@ -2430,7 +2498,7 @@ __device__ __noinline__ double kktSolveImpl(Ctx& c, const DevSettings& st, FactS
       FOR_T(i, N) sol[i] += c.cor[i];
       __syncthreads();
       const double prev = rel;
-      rel = kktResidual(c, st, rhs, sol, c.res, rhsNorm);
+      rel = kktResidual(c, st, rhs, sol, c.res, rhsNorm, false);
       ++steps;
       // an FP32 factor whose refinement contracts by less than 4x per step will not reach the
       // tolerance in the remaining steps: go to the high-precision factor now
@@ -2441,6 +2509,7 @@ __device__ __noinline__ double kktSolveImpl(Ctx& c, const DevSettings& st, FactS
         FOR_T(i, N) sol[i] -= c.cor[i];
         __syncthreads();
         rel = prev;
+        pxOk = false;
         break;
       }
     }
@@ -2454,6 +2523,7 @@ __device__ __noinline__ double kktSolveImpl(Ctx& c, const DevSettings& st, FactS
       continue;
     }
     if (threadIdx.x == 0) {
+      c.sc[SC_PXOK] = pxOk ? 1.0 : 0.0;
       if (!(rel <= c.sc[SC_MAXREL])) c.sc[SC_MAXREL] = rel;
       if (!(rel <= c.sc[SC_ITREL])) c.sc[SC_ITREL] = rel;
     }
@@ -2475,6 +2545,7 @@ template <typename FT, bool G = false>
 __device__ double kktSolve(Ctx& c, const DevSettings& st, FactState& fs, const double* rhs, double* sol) {
   const long long t0 = st.record_timings ? clock64() : 0;
   const long long f0 = st.record_timings ? timers(c)[TM_FACTOR] : 0;
+  if (threadIdx.x == 0) c.sc[SC_PXOK] = 0.0;
   __syncthreads();
   // a fallback refactorisation inside counts as factorisation time only
   const double r = kktSolveImpl<FT, G>(c, st, fs, rhs, sol);
@@ -2551,7 +2622,7 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       int bad = 0;
       FOR_T(j, n) bad |= !finiteBits(c.x[j]);
       FOR_T(r, m) bad |= !finiteBits(c.s[r]) | !finiteBits(c.z[r]);
-      initOk = blockOrInt(bad, c.redi) == 0;
+      initOk = !blockAny(bad);
     }
   }
   if (!initOk) status = 5;
@@ -2581,7 +2652,10 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
     FOR_T(r, m) c.z1[r] = c.sol[n + r];
     __syncthreads();
     if (!vecFinite(c, c.sol, N)) { status = 5; break; }
-    pmul(c, c.x1, c.Px1);
+    // P times a solution: what its last KKT residual formed, unless that solution was not kept
+    if (c.sc[SC_PXOK] != 0.0) FOR_T(j, n) c.Px1[j] = c.tn[j];
+    else pmul(c, c.x1, c.Px1);
+    __syncthreads();
     // 3. residuals
     pmul(c, c.x, c.tn);  // Px
     {
@@ -2653,7 +2727,7 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       __syncthreads();
       kktSolve<FT, G>(c, st, fs, c.rhs, c.sol);
       if (!vecFinite(c, c.sol, N)) { status = 5; break; }
-      pmul(c, c.sol, c.tn);  // P xv
+      if (c.sc[SC_PXOK] == 0.0) pmul(c, c.sol, c.tn);  // P xv
       double tn3[3] = {0, 0, 0};
       FOR_T(j, n) {
         tn3[0] += c.qs[j] * c.sol[j];
@@ -2676,14 +2750,13 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
         int bad = !finiteBits(dtauA) || !finiteBits(dkappaA);
         FOR_T(j, n) bad |= !finiteBits(c.dx[j]);
         FOR_T(r, m) bad |= !finiteBits(c.dz[r]) | !finiteBits(c.ds[r]);
-        if (blockOrInt(bad, c.redi)) { status = 5; break; }
+        if (blockAny(bad)) { status = 5; break; }
       }
       // 6. affine step length (no fraction), mu_aff, sigma
       double aaff = 1.0;
       if (dtauA < 0) aaff = fmin(aaff, -tau / dtauA);
       if (dkappaA < 0) aaff = fmin(aaff, -kappa / dkappaA);
-      aaff = coneMaxStep(c, c.z, c.dz, aaff);
-      aaff = coneMaxStep(c, c.s, c.ds, aaff);
+      aaff = coneMaxStep2(c, aaff);
       double sa[1] = {0.0};
       FOR_T(r, m) sa[0] += (c.s[r] + aaff * c.ds[r]) * (c.z[r] + aaff * c.dz[r]);
       blockSum<1>(sa, c.red);
@@ -2712,7 +2785,7 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       __syncthreads();
       kktSolve<FT, G>(c, st, fs, c.rhs, c.sol);
       if (!vecFinite(c, c.sol, N)) { status = 5; break; }
-      pmul(c, c.sol, c.tn);
+      if (c.sc[SC_PXOK] == 0.0) pmul(c, c.sol, c.tn);
       tn3[0] = tn3[1] = tn3[2] = 0.0;
       FOR_T(j, n) {
         tn3[0] += c.qs[j] * c.sol[j];
@@ -2736,14 +2809,13 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
         int bad = !finiteBits(dtau) || !finiteBits(dkappa);
         FOR_T(j, n) bad |= !finiteBits(c.dx[j]);
         FOR_T(r, m) bad |= !finiteBits(c.dz[r]) | !finiteBits(c.ds[r]);
-        if (blockOrInt(bad, c.redi)) { status = 5; break; }
+        if (blockAny(bad)) { status = 5; break; }
       }
       // 8. step length with the fraction-to-boundary factor
       double alpha = 1.0;
       if (dtau < 0) alpha = fmin(alpha, -tau / dtau);
       if (dkappa < 0) alpha = fmin(alpha, -kappa / dkappa);
-      alpha = coneMaxStep(c, c.z, c.dz, alpha);
-      alpha = coneMaxStep(c, c.s, c.ds, alpha);
+      alpha = coneMaxStep2(c, alpha);
       alpha *= st.max_step_fraction;
       if (trow && threadIdx.x == 0) { trow[7] = alpha; trow[10] = c.sc[SC_ITREL]; }
       if (!isfinite(alpha) || alpha <= 0.0) { status = 5; break; }
@@ -2804,7 +2876,7 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       Bs[bl.cu + r] = c.cu[r];
       Bs[bl.zh + r] = c.z[r] / tau;
     }
-    FOR_T(k, 8 * c.nsoc) Bs[bl.sp + k] = reinterpret_cast<const double*>(c.sp)[k];
+    FOR_T(k, kSocScaleDoubles * c.nsoc) Bs[bl.sp + k] = reinterpret_cast<const double*>(c.sp)[k];
     FOR_T(j, n) Bs[bl.xh + j] = c.x[j] / tau;
     if (threadIdx.x == 0) {
       Bs[bl.sc + 0] = fs.ea;
@@ -2903,7 +2975,7 @@ static __device__ void setupCtx(Ctx& c, const LaunchArgs& a, int inst, unsigned 
   c.dcon = take(mM); c.lam = take(mM); c.tm = take(mM); c.tm2 = take(mM); c.cw = take(mM); c.cu = take(mM);
   c.rhs = take(NM); c.sol = take(NM); c.res = take(NM); c.cor = take(NM);
   c.rr = take(rM);
-  c.sp = reinterpret_cast<SocScale*>(take(8 * L.nsocMax));
+  c.sp = reinterpret_cast<SocScale*>(take(kSocScaleDoubles * L.nsocMax));
   // used once or twice per iteration: always in scratch (vecGlobalDoubles)
   c.ev = scratch + D.sVecG;
   c.z1 = c.ev + ((mM + 1) & ~1);
@@ -2990,7 +3062,7 @@ static __device__ __noinline__ void adjointInstance(Ctx& c, const LaunchArgs& a)
     c.cw[r] = Bs[bl.cw + r];
     c.cu[r] = Bs[bl.cu + r];
   }
-  FOR_T(k, 8 * c.nsoc) reinterpret_cast<double*>(c.sp)[k] = Bs[bl.sp + k];
+  FOR_T(k, kSocScaleDoubles * c.nsoc) reinterpret_cast<double*>(c.sp)[k] = Bs[bl.sp + k];
   if (a.lay.root64InSmem) {
     const int64_t rs = rootSize(c.nr);
     for (int64_t t = threadIdx.x; t < rs; t += blockDim.x) c.root64[t] = Bs[bl.root + t];

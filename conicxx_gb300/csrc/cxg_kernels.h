@@ -28,7 +28,7 @@ constexpr int64_t kGridTcStageBytes = 4 * 16384 + 2 * 16 * (int64_t)kTileElems *
 inline int64_t vecDoubles(int nMax, int mMax, int nrMax, int nsocMax) {
   auto r2 = [](int64_t v) { return (v + 1) & ~int64_t(1); };
   return 6 * r2(nMax) + 11 * r2(mMax) + 4 * r2((int64_t)nMax + mMax) + (int64_t)rootTiles(nrMax) * kTile +
-         r2(8 * (int64_t)nsocMax);
+         r2(kSocScaleDoubles * (int64_t)nsocMax);
 }
 // Vectors used once or twice per iteration (the cone identity e and the constant-solve z1), kept
 // in the CTA's scratch so the shared-memory vector area stays small enough for the largest root.

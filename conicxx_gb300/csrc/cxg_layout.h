@@ -92,6 +92,9 @@ struct InstanceDesc {
   double cost;                        // scheduling weight (~ nr^3)
 };
 
+// Doubles of one SOC block's scaling parameters (SocScale).
+constexpr int kSocScaleDoubles = 9;
+
 // Saved final state of one instance for the adjoint (differentiable batches), in doubles:
 // FP64 root factor, NN/SOC scaling (w, G eigenvalues / u, SOC parameters), normalised iterate
 // x/tau and z/tau, and [bump_a, bump_p, status, tau].
@@ -104,7 +107,7 @@ CXG_HD BwdLayout bwdLayout(int nr, int n, int m, int nsoc) {
   b.root = o; o += rootSize(nr);
   b.cw = o; o += m;
   b.cu = o; o += m;
-  b.sp = o; o += 8 * (int64_t)nsoc;
+  b.sp = o; o += kSocScaleDoubles * (int64_t)nsoc;
   b.xh = o; o += n;
   b.zh = o; o += m;
   b.sc = o; o += 4;
