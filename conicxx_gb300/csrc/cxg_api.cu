@@ -231,10 +231,6 @@ static const int kCtaMaxRoot = 4096;
 static const int kGridAutoRoot = 512;
 static const int kGridMaxRoot = 131072;
 static const int kGridMaxAdjointRoot = 8192;
-// shared memory of the whole-GPU trailing update (8-byte entries; see gridStageBytes)
-// (8-byte entries; see gridStageBytes), or the FP32 tensor-core update's, whichever is larger
-static const int64_t kGridStageBytes = std::max<int64_t>((2ll * kTile * 128 + 16ll * kTileElems) * 8, kGridTcStageBytes);
-
 static int chooseBlock(int nrMax, int requested) {
   if (requested == 32 || requested == 64 || requested == 128 || requested == 256) return requested;
   if (nrMax <= 32) return 32;
@@ -408,7 +404,7 @@ static int buildGroups(cxg_batch* B) {
       InstanceDesc& D = B->pools.desc[(size_t)idx[(size_t)t]];
       int64_t o = 0;
       D.sPv = o; o += r2((int64_t)D.nnzPu + D.nnzPs);
-      D.sAv = o; o += r2(D.nnzA);
+      D.sAv = o; o += r2(3 * (int64_t)D.nnzA);
       D.sAd = o; o += r2(D.nAd);
       D.sT = o; o += r2(D.nAd);
       D.sQ = o; o += r2(D.n);

@@ -30,34 +30,91 @@ namespace cxg {
 
 #define FOR_T(i, n) for (int i = (int)threadIdx.x; i < (n); i += (int)blockDim.x)
 
-// sum_{k=beg}^{end-1} val[k] * x[col[k]]: eight loads in flight per round (the values and
-// column indices live in the CTA's scratch, in L2) and four independent accumulators (one would
-// make every row a dependent FP64 chain, the cost on GB300's narrow FP64 pipe).
-__device__ __forceinline__ double csrDot(const double* __restrict__ val, const int* __restrict__ col, int beg, int end,
-                                         const double* x) {
+// A sparse matrix in the plan's slice order (sliceRows): rows sorted by length, 32 a slice.
+struct Sliced {
+  const double* val;
+  const int *col, *ptr, *perm;  // per entry; slot ptr; slot -> row
+  int rows;
+};
+
+// Products of the 32 rows of slice `sl` with x, one row a lane (a whole warp calls it); row receives
+// this lane's row, or -1. init (by row, negated when kNeg; may be null) + sum of val * x[col]. kFour:
+// four interleaved sums over the whole groups of eight entries, the rest added to the first, then
+// ((0 + 1) + (2 + 3)); else one sum in sequence, without the entries with col < cmin.
+//
+// The order puts a warp's k-th entries next to each other, sorted rows make a slice's lengths alike, and
+// no load hangs on a branch (a lane without an entry reads its slice's first one and multiplies zeros),
+// so the loads of eight entries are in flight together, during the eight before. With one row per
+// thread in plain CSR order a 189-row P of 9 100 entries took 19 000 cycles, now 11 400; the same order
+// with the loads under their conditions 29 000. One FP64 instruction (64 cycles) per entry of a slice's
+// longest row is 7 000. Inlined: a function would save and restore its registers through L1.
+__device__ __forceinline__ double sliceDot(const Sliced& A, bool kFour, int sl, const double* x, int& row,
+                                           const double* init = nullptr, bool negInit = false, int cmin = 0) {
+  const int lane = threadIdx.x & 31, slot = 32 * sl + lane, rows = A.rows;
+  const int *ptr = A.ptr, *col = A.col;
+  const double* val = A.val;
+  const bool real = slot < rows;
+  const int b0 = ptr[min(slot, rows)], b1 = ptr[min(slot + 1, rows)], r0 = A.perm[min(slot, rows - 1)];
+  row = real ? r0 : -1;
+  const int len = b1 - b0;
+  const int start = __shfl_sync(0xffffffffu, b0, 0), longest = __shfl_sync(0xffffffffu, len, 0);
+  const int whole = kFour ? (len & ~7) : 0;
   double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-  int k = beg;
-  for (; k + 7 < end; k += 8) {
-    double v[8];
-    int ci[8];
+  if (init) {
+    const double i0 = init[r0];
+    a0 = negInit ? -i0 : i0;
+  }
+  if (longest == 0) return a0;
+  int base = start + lane;
+  double v[8];
+  int ci[8];
+  auto load = [&](int k) {
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      v[u] = val[k + u];
-      ci[u] = col[k + u];
+      const bool on = k + u < len;
+      const int at = on ? base : start;
+      v[u] = val[at];
+      ci[u] = col[at];
+      base += __popc(__ballot_sync(0xffffffffu, on));
     }
-    a0 = fma(v[0], x[ci[0]], a0);
-    a1 = fma(v[1], x[ci[1]], a1);
-    a2 = fma(v[2], x[ci[2]], a2);
-    a3 = fma(v[3], x[ci[3]], a3);
-    a0 = fma(v[4], x[ci[4]], a0);
-    a1 = fma(v[5], x[ci[5]], a1);
-    a2 = fma(v[6], x[ci[6]], a2);
-    a3 = fma(v[7], x[ci[7]], a3);
+  };
+  load(0);
+  for (int k = 0; k < longest; k += 8) {
+    double w[8], xv[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) xv[u] = x[ci[u]];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const bool on = k + u < len && ci[u] >= cmin;
+      w[u] = on ? v[u] : 0.0;
+      xv[u] = on ? xv[u] : 0.0;
+    }
+    if (k + 8 < longest) load(k + 8);
+    const bool four = k < whole;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (u > 0 && k + u >= longest) break;
+      if ((u & 3) == 0) {
+        a0 = fma(w[u], xv[u], a0);
+      } else {
+        double& a = (u & 3) == 1 ? a1 : (u & 3) == 2 ? a2 : a3;
+        const double t = fma(w[u], xv[u], four ? a : a0);
+        a = four ? t : a;
+        a0 = four ? a0 : t;
+      }
+    }
   }
-  for (; k < end; ++k) a0 = fma(val[k], x[col[k]], a0);
-  return (a0 + a1) + (a2 + a3);
+  if (kFour && longest >= 8) return (a0 + a1) + (a2 + a3);
+  return a0;
 }
 
+// The task of a warp in round `round` of a list that comes longest first: back and forth over the SM's
+// four sub-partitions (warp w runs on sub-partition w % 4), so that they get alike shares.
+__device__ __forceinline__ int snakeTask(int round) {
+  const int nw = blockDim.x >> 5, q = round * nw + (threadIdx.x >> 5);
+  if (nw & 3) return round * nw + ((round & 1) ? nw - 1 - (int)(threadIdx.x >> 5) : (int)(threadIdx.x >> 5));
+  return ((q >> 2) & 1) ? (q ^ 3) : q;
+}
 
 // ------------------------------------------------------------------------------------------
 // block reductions (deterministic: fixed summation order, identical result in every thread)
@@ -168,11 +225,12 @@ struct GridCtl;
 struct Ctx {
   int n, m, p, l, nsoc, nr, nUnits;
   const InstanceDesc* D;
-  const int *psRow, *psCol, *pdiag, *plowSrc, *ap, *ai, *arRow, *arCol, *arSrc;
-  const int *azSrc, *socOff, *socDim, *unitAd, *unitSup, *tgtBeg, *contrib;
+  const int *pdiag, *plowSrc, *ap, *ai, *arSrc;
+  const int *azSrc, *socOff, *socDim, *unitAd, *unitSup, *tgtBeg, *contrib, *scUnit, *scOff;
+  Sliced sP, sAc, sAr;  // P, A by columns, A by rows
   const long long *plowIdx, *azIdx, *tgtIdx;  // 64-bit root element offsets (8-byte aligned in the pool)
   // FP64 scratch (scaled data)
-  double *Pu, *Pv, *Av, *Ad, *T, *qs, *bs, *root64;
+  double *Pu, *Pv, *Av, *Avc, *Avr, *Ad, *T, *qs, *bs, *root64;
   // shared-memory (or scratch) vectors
   double *x, *s, *z, *rx, *rz, *x1, *z1, *Px1, *dx, *dz, *ds, *dcon, *lam, *tn, *tm, *tm2;
   double *rhs, *sol, *res, *cor, *rr, *cw, *cu, *ev;
@@ -226,6 +284,11 @@ static __device__ __noinline__ void loadInstance(Ctx& c, const LaunchArgs& a) {
   __syncthreads();
   FOR_T(b2, c.nsoc) c.ev[c.socOff[b2]] = 1.0;
   FOR_T(k, D.nnzPs) c.Pv[k] = c.Pu[psSrc[k]];
+  const int* acSrc = a.ipool + D.iAcSrc;
+  FOR_T(k, D.nnzA) {
+    c.Avc[k] = c.Av[acSrc[k]];
+    c.Avr[k] = c.Av[c.arSrc[k]];
+  }
   const int* adSrc = a.ipool + D.iAdSrc;
   FOR_T(k, D.nAd) {
     const int src = adSrc[k];
@@ -401,9 +464,36 @@ static __device__ void ensureStrictlyInteriorWarm(Ctx& c, double* v) {
 // ------------------------------------------------------------------------------------------
 // SpMVs with the scaled data (FP64)
 // ------------------------------------------------------------------------------------------
-// y = P_sym x (full symmetric CSR, one thread per row)
+// Slices of 32 rows.
+__device__ __forceinline__ int slices(int rows) { return (rows + 31) >> 5; }
+
+// y = P_sym x (full symmetric P, one thread per row)
 static __device__ __noinline__ void pmul(Ctx& c, const double* x, double* y) {
-  FOR_T(i, c.n) y[i] = csrDot(c.Pv, c.psCol, c.psRow[i], c.psRow[i + 1], x);
+  for (int q, i = 0; i * (int)(blockDim.x >> 5) < slices(c.n); ++i) {
+    q = snakeTask(i);
+    if (q >= slices(c.n)) break;
+    int row;
+    const double v = sliceDot(c.sP, true, q, x, row);
+    if (row >= 0) y[row] = v;
+  }
+  __syncthreads();
+}
+
+// px = P x, atz = A'z (interleaved sums) and ax = A x: the slices of all three as one list of tasks,
+// the long rows of P first.
+static __device__ __noinline__ void kktProducts(Ctx& c, const double* x, const double* z, double* px, double* atz,
+                                                double* ax) {
+  const int sn = slices(c.n), sm = slices(c.m);
+  for (int q, i = 0; i * (int)(blockDim.x >> 5) < 2 * sn + sm; ++i) {
+    q = snakeTask(i);
+    if (q >= 2 * sn + sm) continue;
+    const int kind = (q >= sn) + (q >= 2 * sn);
+    const Sliced& A = kind == 0 ? c.sP : kind == 1 ? c.sAc : c.sAr;
+    double* out = kind == 0 ? px : kind == 1 ? atz : ax;
+    int row;
+    const double v = sliceDot(A, kind < 2, q - (kind == 0 ? 0 : kind == 1 ? sn : 2 * sn), kind == 1 ? z : x, row);
+    if (row >= 0) out[row] = v;
+  }
   __syncthreads();
 }
 
@@ -417,20 +507,13 @@ static __device__ __noinline__ double kktResidualImpl(Ctx& c, const DevSettings&
   const double* xs = sol;
   const double* zs = sol + n;
   double acc2[2] = {0.0, 0.0};
-  FOR_T(t, n + m) {
-    if (t < n) {
-      const double px = csrDot(c.Pv, c.psCol, c.psRow[t], c.psRow[t + 1], xs);
-      double acc = __dadd_rn(__dmul_rn(st.static_reg_P, xs[t]), px);
-      acc += csrDot(c.Av, c.ai, c.ap[t], c.ap[t + 1], zs);
-      c.tn[t] = px;
-      res[t] = rhs[t] - acc;
-    } else {
-      const int r = t - n;
-      double acc = 0.0;
-      for (int k = c.arRow[r]; k < c.arRow[r + 1]; ++k) acc += c.Av[c.arSrc[k]] * xs[c.arCol[k]];
-      res[t] = rhs[t] - acc;
-    }
+  kktProducts(c, xs, zs, c.tn, c.dx, res + n);  // dx: free during a solve
+  FOR_T(t, n) {
+    // the product with the small regularisation rounded first (not fused into the sum)
+    const double acc = __dadd_rn(__dmul_rn(st.static_reg_P, xs[t]), c.tn[t]) + c.dx[t];
+    res[t] = rhs[t] - acc;
   }
+  FOR_T(r, m) res[n + r] = rhs[n + r] - res[n + r];
   __syncthreads();
   // + (Hs + epsA I) z on the cone rows
   coneApply(c, kHsEps, st.static_reg_A, zs, c.tm2);
@@ -466,18 +549,8 @@ static __device__ __noinline__ void kktApply(Ctx& c, const DevSettings& st, cons
   const int n = c.n, m = c.m;
   const double* xs = sol;
   const double* zs = sol + n;
-  FOR_T(t, n + m) {
-    if (t < n) {
-      double acc = st.static_reg_P * xs[t] + csrDot(c.Pv, c.psCol, c.psRow[t], c.psRow[t + 1], xs);
-      acc += csrDot(c.Av, c.ai, c.ap[t], c.ap[t + 1], zs);
-      y[t] = acc;
-    } else {
-      const int r = t - n;
-      double acc = 0.0;
-      for (int k = c.arRow[r]; k < c.arRow[r + 1]; ++k) acc += c.Av[c.arSrc[k]] * xs[c.arCol[k]];
-      y[t] = acc;
-    }
-  }
+  kktProducts(c, xs, zs, c.tn, c.dx, y + n);
+  FOR_T(t, n) y[t] = __dadd_rn(__dmul_rn(st.static_reg_P, xs[t]), c.tn[t]) + c.dx[t];
   __syncthreads();
   coneApply(c, kHsEps, st.static_reg_A, zs, c.tm2);
   FOR_T(r, m) y[n + r] -= c.tm2[r];
@@ -632,7 +705,11 @@ __device__ void denseSolve(Ctx& c, const T* M, T* y) {
     T* yJ = y + J * 32;
     if ((int)threadIdx.x < 32 * sd) {
       T acc = (T)0;
-      for (int col = dp * wd; col < (dp + 1) * wd && col < di; ++col) acc = accT(acc, Ajj[di * kTileLd + col], yJ[col]);
+#pragma unroll 4
+      for (int col = dp * wd; col < (dp + 1) * wd; ++col) {
+        const T l = Ajj[di * kTileLd + col];
+        acc = accT(acc, col < di ? l : (T)0, yJ[col]);
+      }
       const T tot = groupSum(accEnd(acc), sd);
       if (dp == 0) x[di] = yJ[di] + tot;
     }
@@ -665,7 +742,11 @@ __device__ void denseSolve(Ctx& c, const T* M, T* y) {
     T* yJ = y + J * 32;
     if ((int)threadIdx.x < 32 * sd) {
       T acc = (T)0;
-      for (int row = max(dp * wd, di + 1); row < (dp + 1) * wd; ++row) acc = accT(acc, Ajj[row * kTileLd + di], yJ[row]);
+#pragma unroll 4
+      for (int row = dp * wd; row < (dp + 1) * wd; ++row) {
+        const T l = Ajj[row * kTileLd + di];
+        acc = accT(acc, row > di ? l : (T)0, yJ[row]);
+      }
       const T tot = groupSum(accEnd(acc), sd);
       if (dp == 0) x[di] = yJ[di] + tot;
     }
@@ -697,8 +778,10 @@ __device__ void denseSolve(Ctx& c, const T* M, T* y) {
 // two root-sized steps, assembly + LDL' and the triangular solves, it posts a job that every
 // CTA runs with it. Jobs are the same tile operations in the same order per tile as the
 // single-CTA root, spread over the warps of the grid, with a grid barrier between dependent
-// steps (two per tile column of the factor, one per tile of each triangular pass).
+// steps of the factor (two per tile column); the triangular passes hand solved tiles over by flags.
 enum { kGridOpFactor = 1, kGridOpSolve = 2, kGridOpExit = 3 };
+
+constexpr int kGridMaxTiles = 131072 / kTile;  // of the largest whole-GPU root
 
 struct GridCtl {
   unsigned arrive;   // barrier: arrivals in the current round
@@ -706,13 +789,14 @@ struct GridCtl {
   int error;         // a barrier wait ran out; every later barrier fails at once
   int op;            // job posted by CTA 0
   int arith;         // root arithmetic of the job: 0 FP64, 1 FP32, 2 double-float
-  int pad;
+  int epoch;         // number of the job (tile flags of the triangular solves)
   void* M;           // root of the job
   void* y;           // solve vector (root arithmetic), rootTiles(nr) * 32 entries
   double ep, ea;     // regularisation bumps of the assembly
   int64_t stageOff;  // byte offset of the tile staging area in dynamic shared memory
   unsigned long long waitNs;  // longest barrier wait; 0 = kGridWaitNs
   Ctx ctx;           // CTA 0's instance context (pointers into global memory only)
+  int flags[2 * kGridMaxTiles];  // job whose forward / backward pass has solved the tile
 };
 
 // Shared memory of the whole-GPU trailing update for one 128x128 super-block (4x4 tiles): the
@@ -780,6 +864,64 @@ static __device__ __noinline__ bool gridSync(GridCtl* g) {
   return sOk != 0;
 }
 
+// The cone-unit contributions added to the root, slices of 32 targets (one a lane), warp w0 of nw: a
+// target's contributions in their order, A_u' (G_u A_u) as d multiply-adds each. Four contributions'
+// loads are in flight together, none under a condition (see sliceDot); one at a time cost two
+// dependent loads from L2 each.
+template <typename T>
+__device__ __forceinline__ void addContributions(const Ctx& c, T* M, int64_t w0, int64_t nw) {
+  const InstanceDesc& D = *c.D;
+  const int lane = threadIdx.x & 31, nT = D.nTgt;
+  const int *ci = c.contrib, *cj = ci + D.nContrib, *cd = cj + D.nContrib;
+  for (int64_t sl = w0; sl < (nT + 31) / 32; sl += nw) {
+    const int t = (int)(32 * sl) + lane;
+    const int b0 = c.tgtBeg[min(t, nT)], len = c.tgtBeg[min(t + 1, nT)] - b0;
+    const int64_t at = c.tgtIdx[min(t, nT - 1)];
+    const int start = __shfl_sync(0xffffffffu, b0, 0), longest = __shfl_sync(0xffffffffu, len, 0);
+    int base = start + lane;
+    double acc = 0.0;
+    for (int k = 0; k < longest; k += 4) {
+      int oi[4], oj[4], d[4];
+      double va[4], vt[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool on = k + u < len;
+        const int q = on ? base : start;
+        base += __popc(__ballot_sync(0xffffffffu, on));
+        oi[u] = ci[q];
+        oj[u] = cj[q];
+        const int dq = cd[q];
+        d[u] = on ? dq : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        va[u] = c.Ad[oi[u]];
+        vt[u] = c.T[oj[u]];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (k + u >= longest) break;
+        acc = fma(d[u] > 0 ? va[u] : 0.0, d[u] > 0 ? vt[u] : 0.0, acc);
+        for (int r0 = 1; __any_sync(0xffffffffu, r0 < d[u]); r0 += 3) {
+          double a[3], b[3];
+#pragma unroll
+          for (int e = 0; e < 3; ++e) {
+            const int r = min(r0 + e, max(d[u] - 1, 0));
+            a[e] = c.Ad[oi[u] + r];
+            b[e] = c.T[oj[u] + r];
+          }
+#pragma unroll
+          for (int e = 0; e < 3; ++e) {
+            const bool on = r0 + e < d[u];
+            if (__any_sync(0xffffffffu, on)) acc = fma(on ? a[e] : 0.0, on ? b[e] : 0.0, acc);
+          }
+        }
+      }
+    }
+    if (t < nT) M[at] += (T)acc;
+  }
+}
+
 // Root assembly spread over the grid, the same writes as the single-CTA assembly in
 // assembleFactor: zero, then the distinct entries (padding identity, P diagonal + bump,
 // strictly-upper P, Zero-row A, Zero-row diagonal), then the cone-unit contributions (one target
@@ -801,14 +943,7 @@ __device__ __noinline__ bool gridAssemble(GridCtl* g, const Ctx& c, const DevSet
   for (int64_t k = gt; k < D.nAZ; k += gs) M[c.azIdx[k]] = (T)c.Av[c.azSrc[k]];
   for (int64_t r = gt; r < c.p; r += gs) M[rootIdx(nr, n + (int)r, n + (int)r)] = (T)(-(st.static_reg_A + ea));
   if (!gridSync(g)) return false;
-  for (int64_t t = gt; t < D.nTgt; t += gs) {
-    double acc = 0.0;
-    for (int q = c.tgtBeg[t]; q < c.tgtBeg[t + 1]; ++q) {
-      const int oi = c.contrib[3 * q], oj = c.contrib[3 * q + 1], d = c.contrib[3 * q + 2];
-      for (int r = 0; r < d; ++r) acc += c.Ad[oi + r] * c.T[oj + r];
-    }
-    M[c.tgtIdx[t]] += (T)acc;
-  }
+  addContributions<T>(c, M, (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x, (int64_t)gridDim.x * (blockDim.x >> 5));
   return gridSync(g);
 }
 
@@ -1857,197 +1992,238 @@ __device__ __noinline__ bool gridLdltSteps(GridCtl* g, int nr, int nx, const Dev
   return true;
 }
 
-// y_J <- Linv_JJ y_J (unit-lower inverse kept transposed in the diagonal tile), by one CTA:
-// 32 rows, each a dot product split over 4 lanes.
+// ---- triangular solves over the grid --------------------------------------------------------------
+// y <- M^-1 y as a dataflow over row tiles, without grid barriers inside. Each warp owns up to
+// kSolveRows row tiles (a CTA a run of consecutive ones) and keeps their part of y in registers. It
+// applies the solved tiles x_j to its rows in order (forward: j ascending, backward: descending), as
+// they are published, solves its own tile when its turn comes and publishes it: within the CTA
+// through shared memory, to the others in y with a flag per tile. Its tiles of the root arrive by
+// asynchronous copies, two ahead of the one in use. So a tile step costs one product and one diagonal
+// solve (about 0.5 us), and only every eighth one a hand-over between SMs; in blocks of four tiles
+// with a grid barrier each it was 17 us a block, mostly tiles read from L2 on the critical path.
+// Every y tile takes its updates one source tile at a time in the same order as before.
+constexpr int kSolveRows = 4;   // row tiles a warp owns at a time, at most
+constexpr int kSolveBufs = 3;   // tile buffers of a warp
+// FP64: four owners a CTA, one per sub-partition (a product holds the FP64 unit for 2000 cycles).
 template <typename T>
-__device__ void ctaDiagForward(const T* Ajj, T* yJ) {
-  constexpr int sd = 4, w = 32 / sd;
-  T tot = (T)0;
-  int i = 0, p = 0;
-  if ((int)threadIdx.x < 32 * sd) {
-    i = threadIdx.x / sd;
-    p = threadIdx.x % sd;
-    T acc = (T)0;
-    for (int col = p * w; col < (p + 1) * w && col < i; ++col) acc = accT(acc, Ajj[i * kTileLd + col], yJ[col]);
-    tot = groupSum(accEnd(acc), sd);
-  }
-  __syncthreads();
-  if ((int)threadIdx.x < 32 * sd && p == 0) yJ[i] = yJ[i] + tot;
-  __syncthreads();
-}
+__device__ __forceinline__ constexpr int solveWarps() { return ArithOf<T>::v == 0 ? 4 : 8; }
 
-// x_J <- Linv_JJ^T y_J, by one CTA.
-template <typename T>
-__device__ void ctaDiagBackward(const T* Ajj, T* yJ) {
-  constexpr int sd = 4, w = 32 / sd;
-  T tot = (T)0;
-  int i = 0, p = 0;
-  if ((int)threadIdx.x < 32 * sd) {
-    i = threadIdx.x / sd;
-    p = threadIdx.x % sd;
-    T acc = (T)0;
-    for (int row = p * w; row < (p + 1) * w; ++row)
-      if (row > i) acc = accT(acc, Ajj[row * kTileLd + i], yJ[row]);
-    tot = groupSum(accEnd(acc), sd);
-  }
-  __syncthreads();
-  if ((int)threadIdx.x < 32 * sd && p == 0) yJ[i] = yJ[i] + tot;
-  __syncthreads();
-}
-
-// y_I -= L_IJ y_J for one off-diagonal tile, one warp (lane = row of the tile).
-template <typename T>
-__device__ __forceinline__ void warpRowsForward(const T* Lij, const T* yJ, T* yI) {
-  const int lane = threadIdx.x & 31;
-  const T yv = yJ[lane];
-  T acc = (T)0;
-#pragma unroll 8
-  for (int col = 0; col < 32; ++col) acc = accT(acc, Lij[col * kTileLd + lane], shflT(yv, col));
-  yI[lane] = yI[lane] - accEnd(acc);
-}
-
-// y_K -= L_JK^T x_J for one off-diagonal tile, one warp (lane = column of the tile).
-template <typename T>
-__device__ __forceinline__ void warpRowsBackward(const T* Ljk, const T* xJ, T* yK) {
-  const int lane = threadIdx.x & 31;
-  const T xv = xJ[lane];
-  T acc = (T)0;
-#pragma unroll 8
-  for (int r2 = 0; r2 < 32; ++r2) acc = accT(acc, Ljk[lane * kTileLd + r2], shflT(xv, r2));
-  yK[lane] = yK[lane] - accEnd(acc);
-}
-
-// y <- M^-1 y over the grid, in blocks of kSolveBlk tiles (one barrier per block step).
-// Forward step B: warps 0..3 of CTA 0 update the tiles of block B+1 from block B, warp 4 scales
-// block B-1 (finished) by D, then CTA 0 solves block B+1 within itself (ctaBlockForward, CTA
-// barriers only); meanwhile the warps of the other CTAs update
-// every tile of blocks B+2.. from block B, one tile each. The backward pass mirrors it. Each
-// y tile receives its updates one source tile at a time, in increasing (forward) / decreasing
-// (backward) source order. Needs at least two CTAs.
-constexpr int kSolveBlk = 4;
-
-// Solve of one block of tiles b0 .. b1-1 within itself by the calling CTA: per tile j, the
-// diagonal block (ctaDiag*) then the updates of the block's other tiles from tile j, one warp
-// each, with CTA barriers only.
-template <typename T>
-__device__ void ctaBlockForward(const T* M, int Tn, int b0, int b1, T* y) {
-  const int warp = threadIdx.x >> 5;
-  for (int j = b0; j < b1; ++j) {
-    ctaDiagForward<T>(M + tileBase(Tn, j, j), y + j * 32);
-    const int i = j + 1 + warp;
-    if (i < b1) warpRowsForward<T>(M + tileBase(Tn, i, j), y + j * 32, y + i * 32);
-    __syncthreads();
-  }
-}
-
-template <typename T>
-__device__ void ctaBlockBackward(const T* M, int Tn, int b0, int b1, T* y) {
-  const int warp = threadIdx.x >> 5;
-  for (int j = b1 - 1; j >= b0; --j) {
-    ctaDiagBackward<T>(M + tileBase(Tn, j, j), y + j * 32);
-    const int k = j - 1 - warp;
-    if (k >= b0) warpRowsBackward<T>(M + tileBase(Tn, j, k), y + j * 32, y + k * 32);
-    __syncthreads();
-  }
-}
-
-// L2 prefetch of tile rows [I0, I1) of tile column j (contiguous in the packed layout), spread
-// over nt threads: one prefetch per 128-byte line.
-template <typename T>
-__device__ __forceinline__ void prefetchTileRun(const T* M, int Tn, int I0, int I1, int j, int t, int nt) {
-  if (I0 >= I1) return;
-  const char* p = reinterpret_cast<const char*>(M + tileBase(Tn, I0, j));
-  const int64_t bytes = (int64_t)(I1 - I0) * kTileElems * (int64_t)sizeof(T);
-  for (int64_t o = (int64_t)t * 128; o < bytes; o += (int64_t)nt * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + o));
-}
-
-template <typename T>
-__device__ __noinline__ bool gridSolve(GridCtl* g, int nr, const T* M, T* y) {
-  const int Tn = rootTiles(nr);
-  const int NB = (Tn + kSolveBlk - 1) / kSolveBlk;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
-  const bool drv = blockIdx.x == 0;
-  const int ww = ((int)blockIdx.x - 1) * W + warp, WW = ((int)gridDim.x - 1) * W;
-  auto blo = [&](int B) { return B * kSolveBlk; };
-  auto bhi = [&](int B) { return min(Tn, (B + 1) * kSolveBlk); };
-  auto scaleBlock = [&](int B) {  // one warp
-    for (int j = blo(B); j < bhi(B); ++j) y[j * 32 + lane] /= M[tileBase(Tn, j, j) + lane * kTileLd + lane];
-  };
-  // CTA 0's step reads its tiles one dependent round after another; the last CTA, whose warps
-  // have no far tiles to update at this size, prefetches them into L2 one step ahead.
-  const bool pf = (int)blockIdx.x == (int)gridDim.x - 1 && !drv;
-  auto prefetchFwd = [&](int B) {  // the tiles of forward step B: block B+1 from block B, block B+1 itself
-    if (B + 1 >= NB) return;
-    for (int j = blo(B); j < bhi(B); ++j) prefetchTileRun<T>(M, Tn, blo(B + 1), bhi(B + 1), j, threadIdx.x, blockDim.x);
-    for (int j = blo(B + 1); j < bhi(B + 1); ++j) prefetchTileRun<T>(M, Tn, j, bhi(B + 1), j, threadIdx.x, blockDim.x);
-  };
-  auto prefetchBwd = [&](int B) {  // the tiles of backward step B: block B-1 from block B, block B-1 itself
-    if (B < 1) return;
-    for (int k = blo(B - 1); k < bhi(B - 1); ++k) {
-      prefetchTileRun<T>(M, Tn, blo(B), bhi(B), k, threadIdx.x, blockDim.x);
-      prefetchTileRun<T>(M, Tn, k, bhi(B - 1), k, threadIdx.x, blockDim.x);
+// Number of tiles solved in a row from tile j on (direction `step`, at most 32 and up to `last`
+// exclusive), at least one: waits for tile j. The lanes read one flag each. 0 when the wait ran out or
+// the launch has failed; bounded as gridSync is.
+static __device__ __forceinline__ int waitTiles(GridCtl* g, const int* flags, int j, int last, int step, int epoch) {
+  const int mine = j + step * (int)(threadIdx.x & 31);
+  const bool in = step > 0 ? mine < last : mine > last;
+  unsigned long long t0 = 0;
+  for (int spin = 0;; ++spin) {
+    int v = epoch - 1;
+    if (in) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(flags + mine) : "memory");
+    const unsigned open = ~__ballot_sync(0xffffffffu, v == epoch);
+    const int ready = open ? __ffs(open) - 1 : 32;
+    if (ready > 0) return ready;
+    if ((spin & 63) == 63) {
+      volatile GridCtl* vg = g;
+      const unsigned long long now = globalNs();
+      unsigned long long limit = vg->waitNs;
+      if (limit == 0) limit = kGridWaitNs;
+      if (t0 == 0) t0 = now;
+      const bool late = now - t0 > limit;
+      if (late && (threadIdx.x & 31) == 0) atomicExch(&g->error, 1);
+      if (__any_sync(0xffffffffu, late || vg->error)) return 0;
     }
+    __nanosleep(20);
+  }
+}
+
+// Publishes a solved tile: this lane's entry into y, then the tile's flag.
+template <typename T>
+__device__ __forceinline__ void publishTile(T* yJ, int* f, int epoch, T x) {
+  const int lane = threadIdx.x & 31;
+  yJ[lane] = x;
+  __syncwarp();
+  if (lane == 0) {
+    __threadfence();
+    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(f), "r"(epoch) : "memory");
+  }
+}
+
+__device__ __forceinline__ float loadL2(const float* p) { return __ldcg(p); }
+__device__ __forceinline__ double loadL2(const double* p) { return __ldcg(p); }
+__device__ __forceinline__ df64 loadL2(const df64* p) {
+  const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
+  return df64(v.x, v.y);
+}
+
+// One row's part of Linv_JJ y_J (forward) or Linv_JJ^T y_J (backward): terms k < i or k > i in four
+// sums of eight, added pairwise. A: the diagonal tile, yb: y_J (shared), lane = row i.
+template <bool kForward, typename T>
+__device__ __forceinline__ T diagPart(const T* A, const T* yb) {
+  const int i = threadIdx.x & 31;
+  T v[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) v[p] = (T)0;
+#pragma unroll 2
+  for (int t = 0; t < 8; ++t) {
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const int k = 8 * p + t;
+      const T a = kForward ? A[i * kTileLd + k] : A[k * kTileLd + i];
+      if (kForward ? k < i : k > i) v[p] = accT(v[p], a, yb[k]);
+    }
+  }
+  return (accEnd(v[0]) + accEnd(v[1])) + (accEnd(v[2]) + accEnd(v[3]));
+}
+
+// One pass (forward or backward) for the calling CTA's row tiles first .. end-1; yv: this lane's
+// entries of the warp's rows. All warps of the CTA call it. xs (shared): two solved tiles of the CTA,
+// the tile being solved, then one source tile per warp.
+template <bool kForward, typename T>
+__device__ __forceinline__ bool solvePass(GridCtl* g, int Tn, const T* M, T* y, int first, int end, int epoch, T* bufs,
+                                          T* xs, T (&yv)[kSolveRows]) {
+  constexpr int W = solveWarps<T>();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool owner = warp < W;
+  int* flags = g->flags + (kForward ? 0 : kGridMaxTiles);
+  T* buf = bufs + (int64_t)warp * kSolveBufs * kTileElems;
+  auto rowOf = [&](int r) { return first + r * W + warp; };
+  // this warp's tiles in the order it uses them: source j outermost (forward 0 .., backward Tn-1 ..),
+  // then its rows from the one nearest to j on (j itself first: the diagonal tile)
+  const int jEnd = kForward ? end : first - 1, jStep = kForward ? 1 : -1;
+  auto uses = [&](int j, int r) {
+    const int I = rowOf(r);
+    return owner && I < end && (kForward ? I >= j : I <= j);
   };
-  // forward
-  if (drv) ctaBlockForward<T>(M, Tn, blo(0), bhi(0), y);
-  if (pf) prefetchFwd(0);
-  if (!gridSync(g)) return false;
-  for (int B = 0; B + 1 < NB; ++B) {
-    if (drv) {
-      const int I = blo(B + 1) + warp;
-      if (warp < kSolveBlk && I < bhi(B + 1)) {
-        for (int j = blo(B); j < bhi(B); ++j) {
-          warpRowsForward<T>(M + tileBase(Tn, I, j), y + j * 32, y + I * 32);
-          __syncwarp();
+  int nj = kForward ? 0 : Tn - 1, nrr = 0, issued = 0;  // the next tile to copy: source nj, row index nrr in order
+  auto issueNext = [&]() {
+    while (nj != jEnd) {
+      const int r = kForward ? nrr : kSolveRows - 1 - nrr;
+      const int j = nj;
+      if (++nrr == kSolveRows) { nrr = 0; nj += jStep; }
+      if (!uses(j, r)) continue;
+      const int I = rowOf(r);
+      const char* src = reinterpret_cast<const char*>(kForward ? M + tileBase(Tn, I, j) : M + tileBase(Tn, j, I));
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(buf + (issued % kSolveBufs) * kTileElems);
+      constexpr int nv = kTileElems * (int)sizeof(T) / 16;
+#pragma unroll 4
+      for (int v = lane; v < nv; v += 32)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * v), "l"(src + 16 * v) : "memory");
+      break;
+    }
+    ++issued;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // the oldest tile copied; once read, its buffer is filled again (refill, off the critical path)
+  int used = 0;
+  auto oldest = [&]() -> const T* {
+    asm volatile("cp.async.wait_group 2;" ::: "memory");
+    __syncwarp();
+    return buf + (used++ % kSolveBufs) * kTileElems;
+  };
+  auto refill = [&]() {
+    __syncwarp();
+    issueNext();
+  };
+  for (int i = 0; i < kSolveBufs; ++i) issueNext();
+  T* xw = xs + 96 + 32 * warp;  // this warp's copy of a source tile from another CTA
+  bool ok = true;
+  int ready = 0;  // source tiles known to be solved from j on
+  T xNext = (T)0;
+  for (int j = kForward ? 0 : Tn - 1; j != jEnd; j += jStep) {
+    const T* x;
+    if (kForward ? j < first : j >= end) {
+      if (!owner) continue;
+      if (ready == 0) {
+        ready = waitTiles(g, flags, j, kForward ? first : end - 1, jStep, epoch);
+        if (ready == 0) {
+          ok = false;
+          ready = 1;
         }
-      } else if (warp == kSolveBlk && B >= 1) {
-        scaleBlock(B - 1);
+        xNext = loadL2(y + (int64_t)j * 32 + lane);
+      }
+      __syncwarp();
+      xw[lane] = xNext;
+      __syncwarp();
+      if (--ready > 0) xNext = loadL2(y + (int64_t)(j + jStep) * 32 + lane);
+      x = xw;
+    } else {
+      const int t = j - first;
+      T* xt = xs + (t & 1) * 32;
+      T yI = (T)0, dI = (T)0;
+      const bool mine = warp == t % W;
+      const int r0 = t / W;
+      if (mine) {
+        T* yb = xs + 64;
+        yI = yv[0];
+#pragma unroll
+        for (int r = 1; r < kSolveRows; ++r)
+          if (r == r0) yI = yv[r];
+        yb[lane] = yI;
+        const T* A = oldest();
+        if (kForward) dI = A[lane * kTileLd + lane];
+        yI = yI + diagPart<kForward>(A, yb);
+        xt[lane] = yI;
       }
       __syncthreads();
-      ctaBlockForward<T>(M, Tn, blo(B + 1), bhi(B + 1), y);
-    } else {
-      if (pf) prefetchFwd(B + 1);
-      for (int I = blo(B + 2) + ww; I < Tn; I += WW) {
-        for (int j = blo(B); j < bhi(B); ++j) {
-          warpRowsForward<T>(M + tileBase(Tn, I, j), y + j * 32, y + I * 32);
-          __syncwarp();
+      if (mine) {  // the rest is not waited for by this CTA's other warps
+        publishTile(y + (int64_t)j * 32, flags + j, epoch, yI);
+        if (kForward) yI = yI / dI;  // the backward pass starts from y / D
+#pragma unroll
+        for (int r = 0; r < kSolveRows; ++r)
+          if (r == r0) yv[r] = yI;
+        refill();
+      }
+      x = xt;
+    }
+#pragma unroll
+    for (int rr = 0; rr < kSolveRows; ++rr) {
+      const int r = kForward ? rr : kSolveRows - 1 - rr;
+      if (!uses(j, r) || rowOf(r) == j) continue;
+      const T* A = oldest();
+      T acc = (T)0;
+#pragma unroll 8
+      for (int k = 0; k < 32; ++k) acc = accT(acc, kForward ? A[k * kTileLd + lane] : A[lane * kTileLd + k], x[k]);
+      yv[r] = yv[r] - accEnd(acc);
+      refill();
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  return ok;
+}
+
+template <typename T>
+__device__ __noinline__ bool gridSolve(GridCtl* g, int nr, const T* M, T* y, T* stage) {
+  constexpr int W = solveWarps<T>();
+  const int Tn = rootTiles(nr), warp = threadIdx.x >> 5, lane = threadIdx.x & 31, G = (int)gridDim.x;
+  const int rows = min(kSolveRows, (Tn + W * G - 1) / (W * G));  // per warp
+  const int run = W * rows;                                      // consecutive row tiles of a CTA
+  // a root with more tiles than the grid's warps own at once: every G-th run, in order
+  const int runs = (Tn + run * G - 1) / (run * G);
+  const int epoch = reinterpret_cast<volatile GridCtl*>(g)->epoch;
+  T* xs = stage;
+  T* bufs = stage + 96 + 32 * 8;
+  T yv[kSolveRows];
+  bool ok = true;
+  for (int k = 0; k < 2 * runs; ++k) {
+    const bool forward = k < runs;
+    const int first = ((forward ? k : 2 * runs - 1 - k) * G + (int)blockIdx.x) * run, end = min(Tn, first + run);
+    if (first >= Tn) continue;
+    if (forward || runs > 1) {
+#pragma unroll
+      for (int r = 0; r < kSolveRows; ++r) {
+        const int I = first + r * W + warp;
+        yv[r] = (T)0;
+        if (warp < W && I < end) {
+          yv[r] = loadL2(y + (int64_t)I * 32 + lane);
+          if (!forward) yv[r] = yv[r] / M[tileBase(Tn, I, I) + lane * kTileLd + lane];
         }
       }
     }
-    if (!gridSync(g)) return false;
+    if (forward) ok = solvePass<true>(g, Tn, M, y, first, end, epoch, bufs, xs, yv) && ok;
+    else ok = solvePass<false>(g, Tn, M, y, first, end, epoch, bufs, xs, yv) && ok;
   }
-  // backward
-  if (drv) {
-    // blocks NB-2 and NB-1 are not scaled yet (the forward steps scale blocks up to NB-3)
-    if (warp < 2 && NB - 1 - warp >= 0) scaleBlock(NB - 1 - warp);
-    __syncthreads();
-    ctaBlockBackward<T>(M, Tn, blo(NB - 1), bhi(NB - 1), y);
-  }
-  if (pf) prefetchBwd(NB - 1);
-  if (!gridSync(g)) return false;
-  for (int B = NB - 1; B >= 1; --B) {
-    if (drv) {
-      const int K = blo(B - 1) + warp;
-      if (warp < kSolveBlk && K < bhi(B - 1)) {
-        for (int j = bhi(B) - 1; j >= blo(B); --j) {
-          warpRowsBackward<T>(M + tileBase(Tn, j, K), y + j * 32, y + K * 32);
-          __syncwarp();
-        }
-      }
-      __syncthreads();
-      ctaBlockBackward<T>(M, Tn, blo(B - 1), bhi(B - 1), y);
-    } else {
-      if (pf) prefetchBwd(B - 1);
-      for (int K = blo(B - 1) - 1 - ww; K >= 0; K -= WW) {
-        for (int j = bhi(B) - 1; j >= blo(B); --j) {
-          warpRowsBackward<T>(M + tileBase(Tn, j, K), y + j * 32, y + K * 32);
-          __syncwarp();
-        }
-      }
-    }
-    if (!gridSync(g)) return false;
-  }
-  return true;
+  tc::fenceProxyAsyncShared();  // these accesses before a factor's bulk copies into the area
+  return gridSync(g) && ok;
 }
 
 // One posted job, run by every CTA (CTA 0 passes its pivot statistics).
@@ -2060,7 +2236,7 @@ __device__ bool gridJobT(GridCtl* g, const DevSettings& st, int op, PivotStats* 
   T* stage = reinterpret_cast<T*>(dynSmem + vg->stageOff);
   if (op == kGridOpFactor)
     return gridAssemble<T>(g, c, st, M, vg->ep, vg->ea) && gridLdlt<T>(g, c.nr, c.n, st, M, ps, stage, c.slices);
-  if (op == kGridOpSolve) return gridSolve<T>(g, c.nr, M, reinterpret_cast<T*>(vg->y));
+  if (op == kGridOpSolve) return gridSolve<T>(g, c.nr, M, reinterpret_cast<T*>(vg->y), stage);
   return false;
 }
 
@@ -2092,6 +2268,7 @@ __device__ bool gridPost(Ctx& c, const DevSettings& st, int op, T* M, T* y, doub
     g->y = y;
     g->ep = ep;
     g->ea = ea;
+    g->epoch += 1;
   }
   if (!gridSync(g)) return false;
   return gridJobT<T>(g, st, op, ps);
@@ -2111,19 +2288,21 @@ __device__ __noinline__ void assembleFactor(Ctx& c, const DevSettings& st, T* M,
   const long long t0 = (st.record_timings && threadIdx.x == 0) ? clock64() : 0;
   // G_u = (Hs_u + epsA I)^-1 as eigenvalues (NN: cu[row]; SOC: sp.r0..r2), then
   // T_u = G_u Ad_u column by column
-  FOR_T(u, c.nUnits) {
-    const int a0 = c.unitAd[u], a1 = c.unitAd[u + 1];
-    if (u < c.l) {
-      const double w = c.cw[c.p + u];
-      const double g = 1.0 / (w * w + epsA);
-      c.cu[c.p + u] = g;
-      for (int k = a0; k < a1; ++k) c.T[k] = g * c.Ad[k];
+  FOR_T(u, c.nUnits) {  // the SOC blocks first (three divisions against one)
+    if (u >= c.nsoc) {
+      const int i = u - c.nsoc;
+      const double w = c.cw[c.p + i];
+      const double g = 1.0 / sqEps(w, epsA, true);
+      c.cu[c.p + i] = g;
+      for (int k = c.unitAd[i]; k < c.unitAd[i + 1]; ++k) c.T[k] = g * c.Ad[k];
     } else {
-      const int b = u - c.l;
-      const int off = c.socOff[b], d = c.socDim[b];
-      socPrepareG(c.sp[b], epsA);
-      for (int k = a0; k < a1; k += d) socApplyG(c.sp[b], c.cu + off, d, c.Ad + k, c.T + k);
+      socPrepareG(c.sp[u], epsA);
     }
+  }
+  __syncthreads();
+  FOR_T(k, D.nSocCols) {
+    const int b = c.scUnit[k], o = c.scOff[k];
+    socApplyG(c.sp[b], c.cu + c.socOff[b], c.socDim[b], c.Ad + o, c.T + o);
   }
   if constexpr (G) {
     // whole-GPU launch: the assembly and the LDL' run on every CTA
@@ -2174,14 +2353,7 @@ __device__ __noinline__ void assembleFactor(Ctx& c, const DevSettings& st, T* M,
   FOR_T(k, D.nAZ) M[c.azIdx[k]] = (T)c.Av[c.azSrc[k]];
   FOR_T(r, c.p) M[rootIdx(nr, n + r, n + r)] = (T)(-(st.static_reg_A + ea));
   __syncthreads();
-  FOR_T(t, D.nTgt) {
-    double acc = 0.0;
-    for (int q = c.tgtBeg[t]; q < c.tgtBeg[t + 1]; ++q) {
-      const int oi = c.contrib[3 * q], oj = c.contrib[3 * q + 1], d = c.contrib[3 * q + 2];
-      for (int r = 0; r < d; ++r) acc += c.Ad[oi + r] * c.T[oj + r];
-    }
-    M[c.tgtIdx[t]] += (T)acc;
-  }
+  addContributions<T>(c, M, threadIdx.x >> 5, blockDim.x >> 5);
   __syncthreads();
   const long long t1 = (st.record_timings && threadIdx.x == 0) ? clock64() : 0;
   denseLdlt<T>(c, M, st, fail, wrongSign, minAbsD);
@@ -2203,13 +2375,11 @@ __device__ __noinline__ void reducedSolve(Ctx& c, const DevSettings& st, const T
   coneApplyG(c, r2, c.tm);
   // t = [r1 + A_C' u ; r2_Z] in T precision
   T* y = reinterpret_cast<T*>(c.rr);
-  FOR_T(j, n) {
-    double acc = r1[j];
-    for (int k = c.ap[j]; k < c.ap[j + 1]; ++k) {
-      const int r = c.ai[k];
-      if (r >= p) acc += c.Av[k] * c.tm[r];
-    }
-    y[j] = (T)acc;
+  for (int q, i = 0; i * (int)(blockDim.x >> 5) < slices(n); ++i) {
+    if ((q = snakeTask(i)) >= slices(n)) break;
+    int j;
+    const double acc = sliceDot(c.sAc, false, q, c.tm, j, r1, false, p);
+    if (j >= 0) y[j] = (T)acc;
   }
   FOR_T(r, p) y[n + r] = (T)r2[r];
   for (int i = nr + (int)threadIdx.x; i < rootTiles(nr) * kTile; i += blockDim.x) y[i] = (T)0;
@@ -2229,12 +2399,11 @@ __device__ __noinline__ void reducedSolve(Ctx& c, const DevSettings& st, const T
   FOR_T(r, p) sol[n + r] = (double)y[n + r];
   __syncthreads();
   // z_C = G_C (A_C x - r2_C)
-  FOR_T(r, m) {
-    if (r >= p) {
-      double acc = -r2[r];
-      for (int k = c.arRow[r]; k < c.arRow[r + 1]; ++k) acc += c.Av[c.arSrc[k]] * sol[c.arCol[k]];
-      c.tm[r] = acc;
-    }
+  for (int q, i = 0; i * (int)(blockDim.x >> 5) < slices(m); ++i) {
+    if ((q = snakeTask(i)) >= slices(m)) break;
+    int r;
+    const double acc = sliceDot(c.sAr, false, q, sol, r, r2, true);
+    if (r >= p) c.tm[r] = acc;
   }
   __syncthreads();
   FOR_T(t, c.l + c.nsoc) {
@@ -2659,21 +2828,26 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
     // 3. residuals
     pmul(c, c.x, c.tn);  // Px
     {
+      // A'z and A x (into dx and tm, free here)
+      for (int q, i = 0; i * (int)(blockDim.x >> 5) < slices(n) + slices(m); ++i) {
+        if ((q = snakeTask(i)) >= slices(n) + slices(m)) continue;
+        const bool cols = q < slices(n);
+        int row;
+        const double v = sliceDot(cols ? c.sAc : c.sAr, false, cols ? q : q - slices(n), cols ? c.z : c.x, row);
+        if (row >= 0) (cols ? c.dx : c.tm)[row] = v;
+      }
+      __syncthreads();
       double v[6] = {0, 0, 0, 0, 0, 0};
       FOR_T(t, n + m) {
         if (t < n) {
-          double atz = 0.0;
-          for (int k = c.ap[t]; k < c.ap[t + 1]; ++k) atz += c.Av[k] * c.z[c.ai[k]];
-          const double r = -atz - c.tn[t] - tau * c.qs[t];
+          const double r = fma(-tau, c.qs[t], -c.dx[t] - c.tn[t]);
           c.rx[t] = r;
           v[0] += r * r;
           v[2] += c.qs[t] * c.x[t];
           v[5] += c.x[t] * c.tn[t];
         } else {
           const int r = t - n;
-          double ax = 0.0;
-          for (int k = c.arRow[r]; k < c.arRow[r + 1]; ++k) ax += c.Av[c.arSrc[k]] * c.x[c.arCol[k]];
-          const double rr = ax + c.s[r] - tau * c.bs[r];
+          const double rr = c.tm[r] + c.s[r] - tau * c.bs[r];
           c.rz[r] = rr;
           v[1] += rr * rr;
           v[3] += c.bs[r] * c.z[r];
@@ -2686,7 +2860,9 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       dsz = v[4];
       dxPx = v[5];
       rtau = dqx + dbz + kappa + dxPx / tau;
-      const double mu = (dsz + tau * kappa) / (double)(degree + 1);
+      // the scalars' products are fused into their sums as written out here and below (the root's
+      // arithmetic decides one of them), whatever the compiler finds around them
+      const double mu = fma(tau, kappa, dsz) / (double)(degree + 1);
       const double nrx = sqrt(v[0]) / tau, nrz = sqrt(v[1]) / tau;
       const double pobj = (0.5 * dxPx / tau + dqx) / tau;
       const double dobj = (-0.5 * dxPx / tau - dbz) / tau;
@@ -2745,7 +2921,8 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       coneApply(c, kHs, 0.0, c.dz, c.tm);
       FOR_T(r, m) c.ds[r] = -(c.tm[r] + c.s[r]);
       __syncthreads();
-      const double dkappaA = -(dkrA + kappa * dtauA) / tau;
+      const double dkappaA =
+          -(sizeof(FT) == 8 ? fma(tau, kappa, __dmul_rn(kappa, dtauA)) : fma(kappa, dtauA, dkrA)) / tau;
       {
         int bad = !finiteBits(dtauA) || !finiteBits(dkappaA);
         FOR_T(j, n) bad |= !finiteBits(c.dx[j]);
@@ -2760,8 +2937,9 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       double sa[1] = {0.0};
       FOR_T(r, m) sa[0] += (c.s[r] + aaff * c.ds[r]) * (c.z[r] + aaff * c.dz[r]);
       blockSum<1>(sa, c.red);
-      const double tauAff = tau + aaff * dtauA, kappaAff = kappa + aaff * dkappaA;
-      const double muAff = (sa[0] + tauAff * kappaAff) / (double)(degree + 1);
+      const double tauAff = fma(aaff, dtauA, tau);
+      const double kappaAff = fma(aaff, dkappaA, kappa);
+      const double muAff = fma(tauAff, kappaAff, sa[0]) / (double)(degree + 1);
       double sigma;
       if (mu > 0) {
         const double rt = fmax(muAff / mu, 0.0);
@@ -2794,7 +2972,7 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       FOR_T(r, m) tn3[1] += c.bs[r] * c.sol[n + r];
       blockSum<3>(tn3, c.red);
       const double dtrC = (1.0 - sigma) * rtau;
-      const double dkrC = tau * kappa + dtauA * dkappaA - sigma * mu;
+      const double dkrC = fma(-sigma, mu, fma(tau, kappa, __dmul_rn(dtauA, dkappaA)));
       const double tauNumC = dtrC - dkrC / tau + tn3[0] + tn3[1] + 2.0 * tn3[2];
       if (tauDen == 0.0 || !isfinite(tauNumC)) { status = 5; break; }
       const double dtau = tauNumC / tauDen;
@@ -2804,7 +2982,7 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       coneApply(c, kHs, 0.0, c.dz, c.tm);
       FOR_T(r, m) c.ds[r] = -(c.tm[r] + c.dcon[r]);
       __syncthreads();
-      const double dkappa = -(dkrC + kappa * dtau) / tau;
+      const double dkappa = -fma(kappa, dtau, dkrC) / tau;
       {
         int bad = !finiteBits(dtau) || !finiteBits(dkappa);
         FOR_T(j, n) bad |= !finiteBits(c.dx[j]);
@@ -2825,8 +3003,8 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
         c.s[r] += alpha * c.ds[r];
         c.z[r] += alpha * c.dz[r];
       }
-      tau += alpha * dtau;
-      kappa += alpha * dkappa;
+      tau = fma(alpha, dtau, tau);
+      kappa = fma(alpha, dkappa, kappa);
       __syncthreads();
       const double scl = fmax(tau, kappa);
       if (scl > 1e8 || scl < 1e-8) {
@@ -2948,10 +3126,11 @@ static __device__ void setupCtx(Ctx& c, const LaunchArgs& a, int inst, unsigned 
   c.D = &D;
   c.n = D.n; c.m = D.m; c.p = D.p; c.l = D.l; c.nsoc = D.nsoc; c.nr = D.nr; c.nUnits = D.nUnits;
   const int* I = a.ipool;
-  c.psRow = I + D.iPsRow; c.psCol = I + D.iPsCol; c.pdiag = I + D.iPdiag;
+  c.pdiag = I + D.iPdiag;
   c.plowIdx = reinterpret_cast<const long long*>(I + D.iPlowIdx); c.plowSrc = I + D.iPlowSrc;
   c.ap = I + D.iAp; c.ai = I + D.iAi;
-  c.arRow = I + D.iArRow; c.arCol = I + D.iArCol; c.arSrc = I + D.iArSrc;
+  c.arSrc = I + D.iArSrc;
+  c.scUnit = I + D.iScUnit; c.scOff = I + D.iScOff;
   c.azIdx = reinterpret_cast<const long long*>(I + D.iAZIdx); c.azSrc = I + D.iAZSrc;
   c.socOff = I + D.iSocOff; c.socDim = I + D.iSocDim;
   c.unitAd = I + D.iUnitAd; c.unitSup = I + D.iUnitSup;
@@ -2960,6 +3139,11 @@ static __device__ void setupCtx(Ctx& c, const LaunchArgs& a, int inst, unsigned 
   c.Pu = scratch + D.sPv;
   c.Pv = c.Pu + D.nnzPu;
   c.Av = scratch + D.sAv;
+  c.Avc = c.Av + D.nnzA;
+  c.Avr = c.Avc + D.nnzA;
+  c.sP = {c.Pv, I + D.iPsCol, I + D.iPsRow, I + D.iPsPerm, D.n};
+  c.sAc = {c.Avc, I + D.iAcCol, I + D.iAcRow, I + D.iAcPerm, D.n};
+  c.sAr = {c.Avr, I + D.iArCol, I + D.iArRow, I + D.iArPerm, D.m};
   c.Ad = scratch + D.sAd;
   c.T = scratch + D.sT;
   c.qs = scratch + D.sQ;

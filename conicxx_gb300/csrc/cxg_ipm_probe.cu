@@ -108,7 +108,9 @@ __global__ void __launch_bounds__(256, 1) denseProbeGridKernel(int nr, int nx, c
   }
   for (int64_t i = gt; i < nr; i += gs) Dout[i] = (double)M[rootIdx(nr, (int)i, (int)i)];
   const unsigned long long t2 = globalNs();
-  ok = ok && gridSolve<T>(g, nr, M, y);
+  if (blockIdx.x == 0 && threadIdx.x == 0) g->epoch = 1;
+  ok = ok && gridSync(g);
+  ok = ok && gridSolve<T>(g, nr, M, y, stage);
   const unsigned long long t3 = globalNs();
   for (int64_t i = gt; i < nr; i += gs) xout[i] = (double)y[i];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -128,7 +130,7 @@ static cudaError_t probeGridLaunch(int nr, int nx, const double* K, const double
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&numSM, cudaDevAttrMultiProcessorCount, dev);
   // FP32: the tensor-core trailing update stages TF32 hi/lo panels (kTcStageBytes)
-  const size_t smem = (size_t)std::max<int64_t>(gridStageBytes((int)sizeof(T)), sizeof(T) == 4 ? kTcStageBytes : 0);
+  const size_t smem = (size_t)kGridStageBytes;
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(denseProbeGridKernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, denseProbeGridKernel<T>, 256, smem);

@@ -24,6 +24,16 @@ struct SmemLayout {
 // 128 bytes of alignment slack.
 constexpr int64_t kGridTcStageBytes = 4 * 16384 + 2 * 16 * (int64_t)kTileElems * 4 + 128;
 
+// Staging area of a CTA in the whole-GPU form, for every arithmetic: the trailing update on the
+// CUDA cores (two 32x128 panels and 16 tiles of 8-byte entries), the one on the tensor cores, or the
+// triangular solves (three tiles and one 32-entry vector a warp, three vectors more), whichever is
+// largest.
+constexpr int64_t kGridStageBytes = []() constexpr {
+  const int64_t syrk = (2ll * kTile * 128 + 16ll * kTileElems) * 8, solve = (8 * 3 * (int64_t)kTileElems + 96 + 256) * 8;
+  const int64_t a = syrk > kGridTcStageBytes ? syrk : kGridTcStageBytes;
+  return a > solve ? a : solve;
+}();
+
 // Doubles of FP64 vectors per CTA for given maxima (must match the carve-up in ipmKernel).
 inline int64_t vecDoubles(int nMax, int mMax, int nrMax, int nsocMax) {
   auto r2 = [](int64_t v) { return (v + 1) & ~int64_t(1); };

@@ -58,22 +58,27 @@ struct InstanceDesc {
   int nTgt;                    // root entries receiving cone-unit contributions
   int nContrib;                // contributions
   int pStoredNnz;              // P.nonZeros() of the user's P (the initial-point branch test)
-  int pad0;
+  int nSocCols;                // columns of the SOC blocks' densified A blocks
   // int pool offsets
   int64_t iPp, iPi;                   // the user's P pattern (upper CSC as given)
-  int64_t iPsRow, iPsCol, iPsSrc;     // full symmetric P: CSR row ptr (n+1), cols, source index into Px
+  int64_t iPsRow, iPsCol, iPsSrc;     // full symmetric P in slice order (sliceRows): slot ptr (n+1), then per
+  int64_t iPsPerm;                    // entry its column and its source index into Px; slot -> row (n)
   int64_t iPdiag;                     // n: source index of P(i,i) in Px or -1
   int64_t iPlowIdx, iPlowSrc;         // nPlow: root index, Px source
   int64_t iAp, iAi;                   // A CSC: col ptr (n+1), row idx (nnzA)
-  int64_t iArRow, iArCol, iArSrc;     // A CSR: row ptr (m+1), col idx, source index into Ax
+  int64_t iArRow, iArCol, iArSrc;     // A by rows in slice order: slot ptr (m+1), col idx, source index into Ax
+  int64_t iArPerm;                    // m: slot -> row
+  int64_t iAcRow, iAcCol, iAcSrc;     // A by columns in slice order: slot ptr (n+1), row idx, source into Ax
+  int64_t iAcPerm;                    // n: slot -> column
   int64_t iAZIdx, iAZSrc;             // nAZ: root index, Ax source
   int64_t iSocOff, iSocDim;           // nsoc: row offset (within m) and dimension of each SOC block
   int64_t iUnitAd;                    // nUnits+1: offset of each unit's Ad block (d_u x s_u, col-major)
   int64_t iUnitSup;                   // nUnits+1: offset of each unit's support list
   int64_t iSup;                       // support lists (x column indices)
   int64_t iAdSrc;                     // nAd: Ax source index or -1 (structural zero)
-  int64_t iTgtIdx, iTgtBeg;           // nTgt root indices; nTgt+1 contribution ranges
-  int64_t iContrib;                   // 3*nContrib: (Ad column offset i, Ad column offset j, d)
+  int64_t iTgtIdx, iTgtBeg;           // nTgt root indices, most contributions first; nTgt+1 slot ptr
+  int64_t iContrib;                   // nContrib Ad column offsets i, then offsets j, then d (slice order)
+  int64_t iScUnit, iScOff;            // nSocCols: SOC block and Ad offset of each column of its block
   // double pool offsets (equilibration, src/conicxx/kkt/equilibration.h:45-54)
   int64_t dD, dE;                     // n, m
   double cscale;
@@ -81,7 +86,8 @@ struct InstanceDesc {
   int64_t vPx, vQ, vAx, vB;           // user values (P upper CSC order, q, A CSC order, b)
   int64_t vX, vS, vZ;                 // outputs: x at vQ-like offset (n), s/z at vB-like offset (m)
   // per-instance FP64 scratch offsets (relative to the CTA's scratch base)
-  int64_t sPv, sAv, sAd, sT, sQ, sB;  // scaled P (user order, then CSR order), scaled A, Ad, T, q, b
+  int64_t sPv, sAv, sAd, sT, sQ, sB;  // scaled P (user order, then slice order), scaled A (CSC order, then
+                                      // by columns and by rows in slice order), Ad, T, q, b
   int64_t sRoot64;                    // FP64 root (fallback / FP64 precision when not in SMEM)
   int64_t sVec;                       // FP64 vectors that do not fit in shared memory
   int64_t sVecG;                      // FP64 vectors always kept in scratch (vecGlobalDoubles)

@@ -5,6 +5,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <numeric>
 #include <stdexcept>
 #include <utility>
 
@@ -171,6 +172,34 @@ static int64_t pushOffsets(std::vector<int>& pool, const std::vector<int64_t>& v
   return off;
 }
 
+// A sparse matrix's rows (CSR: rowPtr, and per entry col and src) as a warp reads them, 32 rows at a
+// time: the rows are sorted by length, longest first (perm: slot -> row; rowPtr becomes the slots'),
+// and in each slice of 32 slots the entries are laid out first entries first, without padding. At
+// level k the slots with more than k entries are the first ones, so a slice's entries of one level are
+// consecutive, in slot order, and a slice starts at its first slot's rowPtr.
+static void sliceRows(std::vector<int>& rowPtr, std::vector<int>& col, std::vector<int>& src, std::vector<int>& perm) {
+  const int rows = (int)rowPtr.size() - 1;
+  auto len = [&](int r) { return rowPtr[(size_t)r + 1] - rowPtr[(size_t)r]; };
+  perm.resize((size_t)rows);
+  std::iota(perm.begin(), perm.end(), 0);
+  std::stable_sort(perm.begin(), perm.end(), [&](int a, int b) { return len(a) > len(b); });
+  std::vector<int> p2(1, 0), c2, s2;
+  c2.reserve(col.size());
+  s2.reserve(src.size());
+  for (int t = 0; t < rows; ++t) p2.push_back(p2.back() + len(perm[(size_t)t]));
+  for (int t0 = 0; t0 < rows; t0 += 32) {
+    const int t1 = std::min(rows, t0 + 32), longest = len(perm[(size_t)t0]);
+    for (int k = 0; k < longest; ++k)
+      for (int t = t0; t < t1 && len(perm[(size_t)t]) > k; ++t) {
+        c2.push_back(col[(size_t)(rowPtr[(size_t)perm[(size_t)t]] + k)]);
+        s2.push_back(src[(size_t)(rowPtr[(size_t)perm[(size_t)t]] + k)]);
+      }
+  }
+  rowPtr.swap(p2);
+  col.swap(c2);
+  src.swap(s2);
+}
+
 void planInstance(const cxg_problem& pr, const cxg_settings& st, Pools& pools) {
   InstanceDesc D{};
   const int n = pr.n, m = pr.m, p = pr.zero_dim, l = pr.nonneg_dim, nsoc = pr.n_soc;
@@ -209,6 +238,9 @@ void planInstance(const cxg_problem& pr, const cxg_settings& st, Pools& pools) {
   }
   D.nnzPs = (int)psCol.size();
   D.nPlow = (int)plowIdx.size();
+  std::vector<int> psPerm;
+  sliceRows(psRow, psCol, psSrc, psPerm);
+  D.iPsPerm = pushInts(I, psPerm);
   D.iPp = pushInts(I, std::vector<int>(pr.Pp, pr.Pp + n + 1));
   D.iPi = pushInts(I, std::vector<int>(pr.Pi, pr.Pi + D.nnzPu));
   D.iPsRow = pushInts(I, psRow);
@@ -243,9 +275,21 @@ void planInstance(const cxg_problem& pr, const cxg_settings& st, Pools& pools) {
   D.nAZ = (int)azIdx.size();
   D.iAp = pushInts(I, ap);
   D.iAi = pushInts(I, ai);
-  D.iArRow = pushInts(I, arRow);
-  D.iArCol = pushInts(I, arCol);
-  D.iArSrc = pushInts(I, arSrc);
+  {
+    // both orders of A as the products read them (sliceRows); the plain ones serve the planning below
+    std::vector<int> rp(arRow), rc(arCol), rs(arSrc), rperm, cp(ap), cc(ai), cs((size_t)D.nnzA), cperm;
+    std::iota(cs.begin(), cs.end(), 0);
+    sliceRows(rp, rc, rs, rperm);
+    sliceRows(cp, cc, cs, cperm);
+    D.iArRow = pushInts(I, rp);
+    D.iArCol = pushInts(I, rc);
+    D.iArSrc = pushInts(I, rs);
+    D.iArPerm = pushInts(I, rperm);
+    D.iAcRow = pushInts(I, cp);
+    D.iAcCol = pushInts(I, cc);
+    D.iAcSrc = pushInts(I, cs);
+    D.iAcPerm = pushInts(I, cperm);
+  }
   D.iAZIdx = pushOffsets(I, azIdx);
   D.iAZSrc = pushInts(I, azSrc);
 
@@ -294,19 +338,34 @@ void planInstance(const cxg_problem& pr, const cxg_settings& st, Pools& pools) {
   }
   std::stable_sort(tgtContrib.begin(), tgtContrib.end(),
                    [](const std::pair<int64_t, int>& a, const std::pair<int64_t, int>& b) { return a.first < b.first; });
-  std::vector<int64_t> tgtIdx;
-  std::vector<int> tgtBeg, contribSorted;
+  // The targets as rows of contributions, for sliceRows: those with most contributions first, so that
+  // the 32 targets a warp takes together are alike; each target's contributions keep their order.
+  std::vector<int64_t> tgtIdx, tgtAll;
+  std::vector<int> tgtBeg(1, 0), cid, unused, tperm;
   for (size_t t = 0; t < tgtContrib.size(); ++t) {
     if (t == 0 || tgtContrib[t].first != tgtContrib[t - 1].first) {
-      tgtIdx.push_back(tgtContrib[t].first);
-      tgtBeg.push_back((int)(contribSorted.size() / 3));
+      tgtAll.push_back(tgtContrib[t].first);
+      tgtBeg.push_back(tgtBeg.back());
     }
-    const int cid = tgtContrib[t].second;
-    contribSorted.push_back(contrib[(size_t)cid * 3 + 0]);
-    contribSorted.push_back(contrib[(size_t)cid * 3 + 1]);
-    contribSorted.push_back(contrib[(size_t)cid * 3 + 2]);
+    cid.push_back(tgtContrib[t].second);
+    tgtBeg.back()++;
   }
-  tgtBeg.push_back((int)(contribSorted.size() / 3));
+  unused = cid;
+  sliceRows(tgtBeg, cid, unused, tperm);
+  for (int t : tperm) tgtIdx.push_back(tgtAll[(size_t)t]);
+  std::vector<int> contribSorted;
+  for (int f = 0; f < 3; ++f)
+    for (int id : cid) contribSorted.push_back(contrib[(size_t)id * 3 + (size_t)f]);
+  // the columns of the SOC blocks' densified A: block and offset of each
+  std::vector<int> scUnit, scOff;
+  for (int b = 0; b < nsoc; ++b)
+    for (int o = unitAd[(size_t)(l + b)]; o < unitAd[(size_t)(l + b) + 1]; o += socDim[(size_t)b]) {
+      scUnit.push_back(b);
+      scOff.push_back(o);
+    }
+  D.nSocCols = (int)scOff.size();
+  D.iScUnit = pushInts(I, scUnit);
+  D.iScOff = pushInts(I, scOff);
   D.nAd = (int)adSrc.size();
   D.nTgt = (int)tgtIdx.size();
   D.nContrib = (int)(contribSorted.size() / 3);
@@ -348,7 +407,8 @@ void appendPools(Pools& dst, const Pools& src) {
   for (InstanceDesc D : src.desc) {
     for (int64_t* f : {&D.iPp, &D.iPi, &D.iPsRow, &D.iPsCol, &D.iPsSrc, &D.iPdiag, &D.iPlowIdx, &D.iPlowSrc, &D.iAp,
                        &D.iAi, &D.iArRow, &D.iArCol, &D.iArSrc, &D.iAZIdx, &D.iAZSrc, &D.iSocOff, &D.iSocDim,
-                       &D.iUnitAd, &D.iUnitSup, &D.iSup, &D.iAdSrc, &D.iTgtIdx, &D.iTgtBeg, &D.iContrib})
+                       &D.iUnitAd, &D.iUnitSup, &D.iSup, &D.iAdSrc, &D.iTgtIdx, &D.iTgtBeg, &D.iContrib, &D.iPsPerm,
+                       &D.iArPerm, &D.iAcRow, &D.iAcCol, &D.iAcSrc, &D.iAcPerm, &D.iScUnit, &D.iScOff})
       *f += ib;
     D.dD += db;
     D.dE += db;

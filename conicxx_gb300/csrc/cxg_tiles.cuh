@@ -200,7 +200,8 @@ __device__ __forceinline__ int tileLeafPanel(T* A, int b, int J, int nr, int nx,
 #pragma unroll
   for (int t = 0; t < 8; ++t) {
     const int ct = c0 + t;
-    a[t] = leaf ? ((t <= li) ? A[ct * kTileLd + r] : A[r * kTileLd + ct]) : (T)0;
+    const T v = A[(t <= li) ? ct * kTileLd + r : r * kTileLd + ct];
+    a[t] = leaf ? v : (T)0;
   }
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
@@ -238,7 +239,7 @@ __device__ __forceinline__ int tileLeafPanel(T* A, int b, int J, int nr, int nx,
     const bool below = r >= c0 + 8;
     T u[8];
 #pragma unroll
-    for (int t = 0; t < 8; ++t) u[t] = below ? A[(c0 + t) * kTileLd + r] : (T)0;
+    for (int t = 0; t < 8; ++t) u[t] = A[(c0 + t) * kTileLd + r];  // rows above: not stored
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
 #pragma unroll
@@ -299,7 +300,12 @@ __device__ __forceinline__ void tileInverseFinish(T* A, int I, int Jb) {
   for (int h = 0; h < 2; ++h) {
     const int i = i0 + 4 * h;
     T acc = A[(o + i) * kTileLd + C];
-    for (int k = 0; k < i; ++k) acc = accT(acc, A[(o + i) * kTileLd + o + k], A[(o + k) * kTileLd + C]);
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+      if (k >= 3 + 4 * h) break;
+      const T l = A[(o + i) * kTileLd + o + k];
+      acc = accT(acc, k < i ? l : (T)0, A[(o + k) * kTileLd + C]);
+    }
     v[h] = -accEnd(acc);
   }
   __syncwarp();
@@ -316,8 +322,8 @@ __device__ __forceinline__ void tileInverseSum(T* A, int I, int Jb) {
   T a0 = (T)0, a1 = (T)0, b0 = (T)0, b1 = (T)0;
 #pragma unroll 4
   for (int k = 8 * Jb; k < 8 * I; k += 2) {
-    const T lv0 = (k > C) ? A[k * kTileLd + C] : ((k == C) ? (T)1 : (T)0);
-    const T lv1 = (k + 1 > C) ? A[(k + 1) * kTileLd + C] : ((k + 1 == C) ? (T)1 : (T)0);
+    const T l0 = A[k * kTileLd + C], l1 = A[(k + 1) * kTileLd + C];
+    const T lv0 = (k > C) ? l0 : ((k == C) ? (T)1 : (T)0), lv1 = (k + 1 > C) ? l1 : ((k + 1 == C) ? (T)1 : (T)0);
     a0 = accT(a0, A[k * kTileLd + R], lv0);
     a1 = accT(a1, A[(k + 1) * kTileLd + R], lv1);
     b0 = accT(b0, A[k * kTileLd + R + 4], lv0);
