@@ -110,6 +110,7 @@ extern "C" void cxg_default_settings(cxg_settings* s) {
 struct Group {
   int begin = 0, count = 0;  // range in `order`
   int block = 128, grid = 1;
+  int sumThreads = 128;      // threads whose sums the block has (block, or fewer in a wide block)
   bool fp32 = false;
   SmemLayout lay{};
   size_t smem = 0;
@@ -159,6 +160,7 @@ struct cxg_batch {
   int lastLaunches = 0;
   double setupTime = 0.0;
   int device = 0;
+  bool wide = false;                        // an SM for every instance: 256-thread blocks (buildGroups)
   bool gridMode = false;                    // one instance, root spread over every SM (launchIpmGrid)
   bool bwdDropped = false;                  // differentiable asked for, not kept (whole-GPU root > 8192 rows)
   bool bwdStale = false;                    // instances replaced since the last solve: no saved states
@@ -395,7 +397,13 @@ static int buildGroups(cxg_batch* B) {
     }
     L.total = used;
     g.smem = (size_t)used;
-    g.block = gridMode ? 256 : chooseBlock(L.nrMax, B->st.threads_per_instance);
+    g.sumThreads = gridMode ? 256 : chooseBlock(L.nrMax, B->st.threads_per_instance);
+    // A batch with an SM for every instance runs 256-thread blocks whatever the size: the sums keep
+    // the order of the narrower block (same bits), while the factor's tiles, the cones' lists and the
+    // sparse products spread over all four sub-partitions. Not when the caller fixed the threads, and
+    // not with more instances than SMs, where the narrow blocks share an SM's FP64 units better.
+    B->wide = N <= numSM && B->st.threads_per_instance == 0;
+    g.block = B->wide ? 256 : g.sumThreads;
     // per-instance scratch layout (relative to the CTA base); the FP64 root is needed when the
     // root is not in shared memory (FP64 precision) or for the mixed-precision fallback.
     const bool needRoot64 = !L.root64InSmem;
@@ -966,6 +974,7 @@ static LaunchArgs solveArgs(const cxg_batch* B, const Group& g, const DevSetting
   a.traceRows = B->traceRows;
   a.scratch = scratch;
   a.scratchStride = g.stride;
+  a.sumThreads = g.sumThreads;
   a.st = ds;
   a.lay = g.lay;
   return a;
@@ -1380,7 +1389,7 @@ extern "C" int cxg_batch_autotune(cxg_batch* B, int trials, char* report, int re
   };
   for (size_t gi = 0; gi < B->groups.size() && rc == CXG_OK; ++gi) {
     Group& g = B->groups[gi];
-    const int start = g.block;
+    const int start = g.sumThreads;
     int bestBlock = start;
     float bestMs = 0.0f;
     char line[256];
@@ -1389,8 +1398,9 @@ extern "C" int cxg_batch_autotune(cxg_batch* B, int trials, char* report, int re
     for (int b : kCand) {
       if (b < 64 && g.lay.nrMax > 64) continue;  // one warp only for small roots
       int occ = 0;
-      if (ipmOccupancy(&occ, b, g.smem, g.fp32) != cudaSuccess || occ < 1) occ = 1;
-      g.block = b;
+      g.sumThreads = b;
+      g.block = B->wide ? 256 : b;
+      if (ipmOccupancy(&occ, g.block, g.smem, g.fp32) != cudaSuccess || occ < 1) occ = 1;
       g.occupancy = occ;
       float med = 0.0f;
       if ((rc = timeSolve(med))) break;
@@ -1402,10 +1412,11 @@ extern "C" int cxg_batch_autotune(cxg_batch* B, int trials, char* report, int re
       }
     }
     if (rc) break;
-    g.block = bestBlock;
+    g.sumThreads = bestBlock;
+    g.block = B->wide ? 256 : bestBlock;
     {
       int occ = 0;
-      if (ipmOccupancy(&occ, bestBlock, g.smem, g.fp32) != cudaSuccess || occ < 1) occ = 1;
+      if (ipmOccupancy(&occ, g.block, g.smem, g.fp32) != cudaSuccess || occ < 1) occ = 1;
       g.occupancy = occ;
     }
     std::snprintf(line, sizeof(line), " -> %d\n", bestBlock);
@@ -1588,6 +1599,7 @@ static int enqueueAdjoint(cxg_batch* B, cudaStream_t s, const double* gx, double
     a.gA = gA;
     a.scratch = B->dScratch + g.scratchOff;
     a.scratchStride = g.stride;
+    a.sumThreads = g.sumThreads;
     a.st = ds;
     a.lay = g.lay;
     // whole-GPU form: the single instance and its scratch belong to CTA 0 (one CTA)
@@ -1721,6 +1733,7 @@ extern "C" int cxg_batch_solve_device_noalloc(cxg_batch* B, double* x, double* s
     a.bwd = B->dBwd;
     a.scratch = scratch;
     a.scratchStride = g.stride;
+    a.sumThreads = g.sumThreads;
     a.st = ds;
     a.lay = g.lay;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(g.gridAlone, capDoubles / g.stride));

@@ -29,6 +29,10 @@
 namespace cxg {
 
 #define FOR_T(i, n) for (int i = (int)threadIdx.x; i < (n); i += (int)blockDim.x)
+// The elements a thread sums: over the first `vb` threads of the block (Ctx::vb). A sum's order, and so its
+// rounding, is that of a block of vb threads whatever the block's real size; a batch that leaves SMs
+// free runs blocks wider than that (threads beyond vb add zeros to nothing).
+#define FOR_V(i, n, vb) for (int i = (int)threadIdx.x < (vb) ? (int)threadIdx.x : (n); i < (n); i += (vb))
 
 // A sparse matrix in the plan's slice order (sliceRows): rows sorted by length, 32 a slice.
 struct Sliced {
@@ -164,19 +168,19 @@ __device__ __forceinline__ double warpTotals(const double* red, int k0, int nw) 
 }
 
 template <int K>
-__device__ __forceinline__ void blockPartials(const double (&v)[K], double* red) {
+__device__ __forceinline__ void blockPartials(const double (&v)[K], double* red, int nw) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const double p = warpSums<K>(v);
   const int k = ((lane >> 4) & 1) | ((lane >> 2) & 2) | (lane & 4);
   __syncthreads();  // the last reduction's readers are done with red
-  if (lane == sumLane(k) && k < K) red[k * 16 + w] = p;
+  if (w < nw && lane == sumLane(k) && k < K) red[k * 16 + w] = p;
   __syncthreads();
 }
 
 template <int K>
-__device__ __forceinline__ void blockSum(double (&v)[K], double* red) {
-  const int nw = blockDim.x >> 5;
-  blockPartials<K>(v, red);
+__device__ __forceinline__ void blockSum(double (&v)[K], double* red, int vb) {
+  const int nw = vb >> 5;
+  blockPartials<K>(v, red, nw);
   if (nw & (nw - 1)) {  // a number of warps that is no power of two: in sequence
 #pragma unroll
     for (int k = 0; k < K; ++k) {
@@ -224,6 +228,7 @@ struct GridCtl;
 
 struct Ctx {
   int n, m, p, l, nsoc, nr, nUnits;
+  int vb;  // threads of the block whose sums the instance has (FOR_V)
   const InstanceDesc* D;
   const int *pdiag, *plowSrc, *ap, *ai, *arSrc;
   const int *azSrc, *socOff, *socDim, *unitAd, *unitSup, *tgtBeg, *contrib, *scUnit, *scOff;
@@ -421,7 +426,7 @@ static __device__ __noinline__ void coneMargins(Ctx& c, const double* x, double&
   double nnmin = INFINITY;
   FOR_T(t, c.l) nnmin = fmin(nnmin, x[c.p + t]);
   double smin = INFINITY, spos = 0.0;
-  FOR_T(b, c.nsoc) {
+  FOR_V(b, c.nsoc, c.vb) {
     const double mg = socMargin(x + c.socOff[b], c.socDim[b]);
     smin = fmin(smin, mg);
     spos += fmax(mg, 0.0);
@@ -429,7 +434,7 @@ static __device__ __noinline__ void coneMargins(Ctx& c, const double* x, double&
   nnmin = blockMin(nnmin, c.red);
   smin = blockMin(smin, c.red);
   double v[1] = {spos};
-  blockSum<1>(v, c.red);
+  blockSum<1>(v, c.red, c.vb);
   mn = fmin(nnmin, smin);
   pos = v[0] + ((c.l > 0) ? fmax(nnmin, 0.0) : 0.0);
   if (!isfinite(mn)) mn = 0.0;
@@ -519,17 +524,17 @@ static __device__ __noinline__ double kktResidualImpl(Ctx& c, const DevSettings&
   coneApply(c, kHsEps, st.static_reg_A, zs, c.tm2);
   FOR_T(r, m) res[n + r] += c.tm2[r];
   __syncthreads();
-  FOR_T(t, n + m) acc2[0] += res[t] * res[t];
-  if (first) FOR_T(t, n + m) acc2[1] += rhs[t] * rhs[t];
+  FOR_V(t, n + m, c.vb) acc2[0] += res[t] * res[t];
+  if (first) FOR_V(t, n + m, c.vb) acc2[1] += rhs[t] * rhs[t];
   // both norms and the quotient by one warp: a square root and a division hold the FP64 unit for
   // some 600 cycles each
-  if (blockDim.x & (blockDim.x - 1)) {
-    blockSum<2>(acc2, c.red);
+  if (c.vb & (c.vb - 1)) {
+    blockSum<2>(acc2, c.red, c.vb);
     if (first) rhsNorm = fmax(sqrt(acc2[1]), 1e-30);
     return sqrt(acc2[0]) / rhsNorm;
   }
-  const int nw = blockDim.x >> 5;
-  blockPartials<2>(acc2, c.red);
+  const int nw = c.vb >> 5;
+  blockPartials<2>(acc2, c.red, nw);
   if (threadIdx.x < 32) {
     const double norm = sqrt(warpTotals(c.red, 0, nw));
     const double rn = first ? fmax(__shfl_sync(0xffffffffu, norm, nw), 1e-30) : rhsNorm;
@@ -671,10 +676,10 @@ __device__ __forceinline__ df64 shflXorT(df64 v, int m) {
 }
 
 // Largest split s in {1, 2, 4, 8} of a 32-term dot product such that rows * s threads fit in
-// one pass of the block (rows is a multiple of 32, so each warp holds whole groups of s lanes).
-__device__ __forceinline__ int dotSplit(int rows) {
+// one pass of a block of vb threads (rows is a multiple of 32, so each warp holds whole groups of s lanes).
+__device__ __forceinline__ int dotSplit(int rows, int vb) {
   int s = 1;
-  while (s < 8 && rows * s * 2 <= (int)blockDim.x) s *= 2;
+  while (s < 8 && rows * s * 2 <= vb) s *= 2;
   return s;
 }
 
@@ -696,7 +701,7 @@ template <typename T>
 __device__ void denseSolve(Ctx& c, const T* M, T* y) {
   const int Tn = rootTiles(c.nr);
   const int nth = blockDim.x;
-  const int sd = dotSplit(32), wd = 32 / sd;
+  const int sd = dotSplit(32, c.vb), wd = 32 / sd;
   const int di = (int)threadIdx.x / sd, dp = (int)threadIdx.x % sd;  // row and part in a diagonal product
   T* x = reinterpret_cast<T*>(c.red);
   // forward: y_J = Linv_JJ y_J, then y_I -= L_IJ y_J for I > J
@@ -717,7 +722,7 @@ __device__ void denseSolve(Ctx& c, const T* M, T* y) {
     if (threadIdx.x < 32) yJ[threadIdx.x] = x[threadIdx.x];
     const int rows = (Tn - J - 1) * 32;
     if (rows > 0) {
-      const int s = dotSplit(rows), w = 32 / s;
+      const int s = dotSplit(rows, c.vb), w = 32 / s;
       for (int t = threadIdx.x; t < rows * s; t += nth) {
         const int row = t / s, p = t % s;
         const int I = J + 1 + row / 32, rr = row % 32;
@@ -754,7 +759,7 @@ __device__ void denseSolve(Ctx& c, const T* M, T* y) {
     if (threadIdx.x < 32) yJ[threadIdx.x] = x[threadIdx.x];
     const int rows = J * 32;
     if (rows > 0) {
-      const int s = dotSplit(rows), w = 32 / s;
+      const int s = dotSplit(rows, c.vb), w = 32 / s;
       for (int t = threadIdx.x; t < rows * s; t += nth) {
         const int row = t / s, p = t % s;
         const int K = row / 32, cc = row % 32;
@@ -2554,15 +2559,15 @@ __device__ __noinline__ double gmresRefine(Ctx& c, const DevSettings& st, const 
       for (int i = 0; i <= j; ++i) {
         const double* vi = V + (int64_t)i * ld;
         double d[1] = {0.0};
-        FOR_T(t, N) d[0] += w[t] * vi[t];
-        blockSum<1>(d, c.red);
+        FOR_V(t, N, c.vb) d[0] += w[t] * vi[t];
+        blockSum<1>(d, c.red, c.vb);
         FOR_T(t, N) w[t] -= d[0] * vi[t];
         if (threadIdx.x == 0) H[j * hl + i] = d[0];
         __syncthreads();
       }
       double nn[1] = {0.0};
-      FOR_T(t, N) nn[0] += w[t] * w[t];
-      blockSum<1>(nn, c.red);
+      FOR_V(t, N, c.vb) nn[0] += w[t] * w[t];
+      blockSum<1>(nn, c.red, c.vb);
       const double hn = sqrt(nn[0]);
       if (threadIdx.x == 0) {
         double* h = H + j * hl;
@@ -2838,7 +2843,7 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       }
       __syncthreads();
       double v[6] = {0, 0, 0, 0, 0, 0};
-      FOR_T(t, n + m) {
+      FOR_V(t, n + m, c.vb) {
         if (t < n) {
           const double r = fma(-tau, c.qs[t], -c.dx[t] - c.tn[t]);
           c.rx[t] = r;
@@ -2854,7 +2859,7 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
           v[4] += c.s[r] * c.z[r];
         }
       }
-      blockSum<6>(v, c.red);
+      blockSum<6>(v, c.red, c.vb);
       dqx = v[2];
       dbz = v[3];
       dsz = v[4];
@@ -2876,9 +2881,9 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       const double ratio = tau / fmax(kappa, 1e-30);
       if (ratio <= st.tol_infeas) {
         double w[2] = {0.0, 0.0};
-        FOR_T(r, m) w[0] += c.z[r] * c.z[r];
-        FOR_T(j, n) w[1] += c.x[j] * c.x[j];
-        blockSum<2>(w, c.red);
+        FOR_V(r, m, c.vb) w[0] += c.z[r] * c.z[r];
+        FOR_V(j, n, c.vb) w[1] += c.x[j] * c.x[j];
+        blockSum<2>(w, c.red, c.vb);
         if (dbz < -st.tol_infeas * fmax(1.0, sqrt(w[0]))) { status = 2; break; }
         if (dqx < -st.tol_infeas * fmax(1.0, sqrt(w[1]))) { status = 3; break; }
       }
@@ -2888,13 +2893,13 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       __syncthreads();
       pmul(c, c.tn, c.dx);
       double td[4] = {0, 0, 0, 0};
-      FOR_T(j, n) {
+      FOR_V(j, n, c.vb) {
         td[0] += c.qs[j] * c.x1[j];
         td[2] += c.tn[j] * c.dx[j];
         td[3] += c.x1[j] * c.Px1[j];
       }
-      FOR_T(r, m) td[1] += c.bs[r] * c.z1[r];
-      blockSum<4>(td, c.red);
+      FOR_V(r, m, c.vb) td[1] += c.bs[r] * c.z1[r];
+      blockSum<4>(td, c.red, c.vb);
       const double tauDen = kappa / tau - td[0] - td[1] + td[2] - td[3];
 
       // 5. affine step: rhs (rx, s - rz)
@@ -2905,12 +2910,12 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       if (!vecFinite(c, c.sol, N)) { status = 5; break; }
       if (c.sc[SC_PXOK] == 0.0) pmul(c, c.sol, c.tn);  // P xv
       double tn3[3] = {0, 0, 0};
-      FOR_T(j, n) {
+      FOR_V(j, n, c.vb) {
         tn3[0] += c.qs[j] * c.sol[j];
         tn3[2] += (c.x[j] / tau) * c.tn[j];
       }
-      FOR_T(r, m) tn3[1] += c.bs[r] * c.sol[n + r];
-      blockSum<3>(tn3, c.red);
+      FOR_V(r, m, c.vb) tn3[1] += c.bs[r] * c.sol[n + r];
+      blockSum<3>(tn3, c.red, c.vb);
       const double dkrA = tau * kappa;
       const double tauNumA = rtau - dkrA / tau + tn3[0] + tn3[1] + 2.0 * tn3[2];
       if (tauDen == 0.0 || !isfinite(tauNumA) || !isfinite(tauDen)) { status = 5; break; }
@@ -2935,8 +2940,8 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       if (dkappaA < 0) aaff = fmin(aaff, -kappa / dkappaA);
       aaff = coneMaxStep2(c, aaff);
       double sa[1] = {0.0};
-      FOR_T(r, m) sa[0] += (c.s[r] + aaff * c.ds[r]) * (c.z[r] + aaff * c.dz[r]);
-      blockSum<1>(sa, c.red);
+      FOR_V(r, m, c.vb) sa[0] += (c.s[r] + aaff * c.ds[r]) * (c.z[r] + aaff * c.dz[r]);
+      blockSum<1>(sa, c.red, c.vb);
       const double tauAff = fma(aaff, dtauA, tau);
       const double kappaAff = fma(aaff, dkappaA, kappa);
       const double muAff = fma(tauAff, kappaAff, sa[0]) / (double)(degree + 1);
@@ -2965,12 +2970,12 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       if (!vecFinite(c, c.sol, N)) { status = 5; break; }
       if (c.sc[SC_PXOK] == 0.0) pmul(c, c.sol, c.tn);
       tn3[0] = tn3[1] = tn3[2] = 0.0;
-      FOR_T(j, n) {
+      FOR_V(j, n, c.vb) {
         tn3[0] += c.qs[j] * c.sol[j];
         tn3[2] += (c.x[j] / tau) * c.tn[j];
       }
-      FOR_T(r, m) tn3[1] += c.bs[r] * c.sol[n + r];
-      blockSum<3>(tn3, c.red);
+      FOR_V(r, m, c.vb) tn3[1] += c.bs[r] * c.sol[n + r];
+      blockSum<3>(tn3, c.red, c.vb);
       const double dtrC = (1.0 - sigma) * rtau;
       const double dkrC = fma(-sigma, mu, fma(tau, kappa, __dmul_rn(dtauA, dkappaA)));
       const double tauNumC = dtrC - dkrC / tau + tn3[0] + tn3[1] + 2.0 * tn3[2];
@@ -3064,9 +3069,9 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
     }
   }
   double nr2[2] = {0.0, 0.0};
-  FOR_T(j, n) nr2[0] += c.rx[j] * c.rx[j];
-  FOR_T(r, m) nr2[1] += c.rz[r] * c.rz[r];
-  blockSum<2>(nr2, c.red);
+  FOR_V(j, n, c.vb) nr2[0] += c.rx[j] * c.rx[j];
+  FOR_V(r, m, c.vb) nr2[1] += c.rz[r] * c.rz[r];
+  blockSum<2>(nr2, c.red, c.vb);
   if (status == 1 && st.warm_start && a.warmX) {
     FOR_T(j, n) a.warmX[D.vQ + j] = c.x[j];
     FOR_T(r, m) {
@@ -3124,6 +3129,7 @@ static __device__ void setupCtx(Ctx& c, const LaunchArgs& a, int inst, unsigned 
   const SmemLayout& L = a.lay;
   const InstanceDesc& D = a.desc[inst];
   c.D = &D;
+  c.vb = a.sumThreads;
   c.n = D.n; c.m = D.m; c.p = D.p; c.l = D.l; c.nsoc = D.nsoc; c.nr = D.nr; c.nUnits = D.nUnits;
   const int* I = a.ipool;
   c.pdiag = I + D.iPdiag;

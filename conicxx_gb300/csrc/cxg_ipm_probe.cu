@@ -25,6 +25,7 @@ __global__ void __launch_bounds__(256) denseProbeKernel(int nr, int nx, const do
   if (threadIdx.x == 0) {
     c.nr = nr;
     c.n = nx;
+    c.vb = blockDim.x;
     c.red = scArea;
     c.sc = scArea + 128;
   }

@@ -97,6 +97,7 @@ struct LaunchArgs {
   int traceRows;
   double* scratch;        // gridDim.x * scratchStride doubles
   int64_t scratchStride;
+  int sumThreads;         // threads whose sums the block has (<= block size; FOR_V)
   DevSettings st;
   SmemLayout lay;
   struct GridCtl* grid;   // whole-GPU form of one instance (cooperative launch), else null

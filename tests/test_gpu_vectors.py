@@ -72,3 +72,19 @@ def test_blocks_that_skip_the_pivot_test_pass_it(d):
         assert np.min(np.abs(A[:, k, k])) > deps
         l = A[:, k + 1:, k] / A[:, k, k][:, None]
         A[:, k + 1:, k + 1:] -= l[:, :, None] * A[:, k, k + 1:][:, None, :]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("contacts,threads", [(1, 32), (10, 32), (11, 64), (21, 64), (22, 128), (42, 128)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_wide_blocks_give_the_narrow_blocks_bits(contacts, threads, precision):
+    """A batch with an SM for every instance runs 256-thread blocks with the sums of the narrow block:
+    the same bits as the narrow block itself, in the solve and in the adjoint."""
+    qps = [generators.contact_qp(s, contacts=contacts) for s in range(3)]
+    got = []
+    for t in (0, threads):
+        B = BatchSolver(qps, precision=precision, warm_start=0, threads_per_instance=t, differentiable=1)
+        x, s, z, infos = B.solve()
+        got.append((x, s, z, infos["iterations"], infos["refine_steps"]) + B.backward(np.ones(B.n_total)))
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
