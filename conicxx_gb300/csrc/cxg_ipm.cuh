@@ -804,13 +804,6 @@ struct GridCtl {
   int flags[2 * kGridMaxTiles];  // job whose forward / backward pass has solved the tile
 };
 
-// Shared memory of the whole-GPU trailing update for one 128x128 super-block (4x4 tiles): the
-// panel rows A[32][128] and the D-scaled panel columns B[32][128] (k-major), and the 16 result
-// tiles in tile layout.
-constexpr int kSbDim = 128;
-constexpr int kStageElems = 2 * kTile * kSbDim + 16 * kTileElems;
-constexpr int64_t gridStageBytes(int elemBytes) { return (int64_t)kStageElems * elemBytes; }
-
 template <typename T> struct ArithOf;
 template <> struct ArithOf<double> { static constexpr int v = 0; };
 template <> struct ArithOf<float> { static constexpr int v = 1; };
@@ -952,125 +945,89 @@ __device__ __noinline__ bool gridAssemble(GridCtl* g, const Ctx& c, const DevSet
   return gridSync(g);
 }
 
-// Four consecutive entries of a shared-memory row (16-byte aligned for 4-byte T, two 16-byte
-// halves for 8-byte T).
+// Asynchronous copy of one tile into shared memory (16-byte cp.async), thread t of nt; not committed.
 template <typename T>
-__device__ __forceinline__ void lds4(const T* p, T (&v)[4]) {
-  if constexpr (sizeof(T) == 4) {
-    const float4 f = *reinterpret_cast<const float4*>(p);
-    v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-  } else {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = p[i];
-  }
+__device__ __forceinline__ void copyTileAsync(T* dst, const T* src, int t, int nt) {
+  constexpr int nv = kTileElems * (int)sizeof(T) / 16;
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+#pragma unroll 4
+  for (int v = t; v < nv; v += nt)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16u * v),
+                 "l"(reinterpret_cast<const char*>(src) + 16 * v)
+                 : "memory");
 }
 
-// C -= A D B^T for one super-block of up to 4x4 tiles, by one CTA of 256 threads:
-// rows I0 .. I0+ni-1 and columns K0 .. K0+nk-1 (tile indices); only tiles with column <= row when
-// the super-block is on the diagonal, and not its first tile when skip00 (updated elsewhere).
-// A = the panel tiles L_IJ, B = L_KJ, D = diag of tile (J, J).
-// The C tiles are copied into shared memory asynchronously (cp.async) while the panel is staged
-// k-major (B pre-scaled by D exactly as tileSyrk scales it) and each thread accumulates an 8x8
-// block of the 128x128 product over k = 0..31 in the order tileSyrk uses; then C -= product in
-// shared memory (so every entry gets the same bits as tileSyrk) and the tiles are stored back
-// with 16-byte vectors.
+// Trailing update of tile column J on the CUDA cores (FP64 and double-float): C_IK -= L_IJ D_J L_KJ^T
+// for the tiles J < K <= I but (J+1, J+1), one tile at a time and CTA (CTAs 1 .., 256 threads). The
+// three tiles of the next product arrive by cp.async meanwhile; L_KJ is scaled by D_J once in shared
+// memory; warp w takes columns 4 w .. 4 w + 3, a lane one row, with the tile routine's operations in its
+// order. Single tiles rather than 128x128 super-blocks: a super-block holds one SM's FP64 units for
+// 127 us (24 us of FP32 issue in double-float) while a root of some thousand rows has fewer
+// super-blocks than the GPU has SMs; a tile takes 9 us (2 us).
 template <typename T>
-__device__ __noinline__ void superSyrk(T* M, int Tn, int J, int I0, int K0, int ni, int nk, bool diagSb, bool skip00,
-                                      T* sm) {
-  T* As = sm;
-  T* Bs = sm + kTile * kSbDim;
-  T* Cs = sm + 2 * kTile * kSbDim;
+__device__ __noinline__ void gridTileUpdate(T* M, int Tn, int J, T* sm) {
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, c0 = 4 * (tid >> 5);
+  const int rem = Tn - J - 1, stride = (int)gridDim.x - 1;
+  const long long tiles = (long long)rem * (rem + 1) / 2;
   const T* Ajj = M + tileBase(Tn, J, J);
-  const int tid = threadIdx.x;
-  constexpr int per16 = 16 / (int)sizeof(T);
-  constexpr int vpt = kTileElems / per16;  // 16-byte vectors per tile
-  // (1) the C tiles of this super-block, global -> Cs, as asynchronous 16-byte copies that
-  //     proceed while the panel is staged and the product computed
-  for (int v = tid; v < 16 * vpt; v += blockDim.x) {
-    const int t = v / vpt, a = t >> 2, b = t & 3;
-    if (a < ni && b < nk && !(diagSb && b > a) && !(skip00 && t == 0)) {
-      const T* src = M + tileBase(Tn, I0 + a, K0 + b) + (v - t * vpt) * per16;
-      const unsigned dst = (unsigned)__cvta_generic_to_shared(Cs + v * per16);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+  T* dg = sm;              // the diagonal of D_J
+  T* bufs = sm + 32;       // two sets of L_IJ, L_KJ, C_IK
+  // tile t (row order: t = i (i + 1) / 2 + k, tile (J+1+i, J+1+k)); t = 0 belongs to CTA 0
+  auto where = [&](long long t, int& I, int& K) {
+    int i = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+    while ((long long)i * (i + 1) / 2 > t) --i;
+    while ((long long)(i + 1) * (i + 2) / 2 <= t) ++i;
+    I = J + 1 + i;
+    K = J + 1 + (int)(t - (long long)i * (i + 1) / 2);
+  };
+  auto fetch = [&](long long t, int set) {
+    if (t < tiles) {
+      int I, K;
+      where(t, I, K);
+      T* b = bufs + set * 3 * kTileElems;
+      copyTileAsync(b, M + tileBase(Tn, I, J), tid, nt);
+      copyTileAsync(b + kTileElems, M + tileBase(Tn, K, J), tid, nt);
+      copyTileAsync(b + 2 * kTileElems, M + tileBase(Tn, I, K), tid, nt);
     }
-  }
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-  {
-    // (2) the panel: thread tid stages column i = tid & 127 for k = tid >> 7, +2, ... (all loads
-    //     of a half issued before any store, so their latencies overlap)
-    const int i = tid & (kSbDim - 1), a = i >> 5, rr = i & 31, k0 = tid >> 7;
-    const T* pa = (a < ni) ? M + tileBase(Tn, I0 + a, J) + rr : nullptr;
-    const T* pb = (a < nk) ? M + tileBase(Tn, K0 + a, J) + rr : nullptr;
-    constexpr int kPer = 8;  // 256 threads: two k rows per step, 8 steps per half
-#pragma unroll 1
-    for (int h = 0; h < 2; ++h) {
-      T va[kPer], vb[kPer], dk[kPer];
-#pragma unroll
-      for (int t = 0; t < kPer; ++t) {
-        const int k = k0 + 2 * (h * kPer + t);
-        va[t] = pa ? pa[k * kTileLd] : (T)0;
-        vb[t] = pb ? pb[k * kTileLd] : (T)0;
-        dk[t] = Ajj[k * kTileLd + k];
-      }
-#pragma unroll
-      for (int t = 0; t < kPer; ++t) {
-        const int k = k0 + 2 * (h * kPer + t);
-        As[k * kSbDim + i] = va[t];
-        Bs[k * kSbDim + i] = pb ? vb[t] * dk[t] : (T)0;
-      }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  long long t = (long long)blockIdx.x;
+  if (t >= tiles) return;
+  fetch(t, 0);
+  if (tid < 32) dg[tid] = Ajj[tid * kTileLd + tid];
+  for (int set = 0; t < tiles; t += stride, set ^= 1) {
+    fetch(t + stride, set ^ 1);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    T* A = bufs + set * 3 * kTileElems;
+    T *B = A + kTileElems, *C = B + kTileElems;
+    for (int e = tid; e < kTile * kTile; e += nt) {
+      const int k = e >> 5, i = e & 31;
+      B[k * kTileLd + i] = B[k * kTileLd + i] * dg[k];
     }
-  }
-  __syncthreads();
-  // (3) the product, 8x8 per thread, k = 0..31 in the tile routine's order
-  const int tx = tid & 15, ty = tid >> 4;  // rows tx*4 + {0..3, 64..67}, columns ty*4 + {0..3, 64..67}
-  T acc[8][8];
+    __syncthreads();
+    T acc[4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+    for (int j = 0; j < 4; ++j) acc[j] = (T)0;
+#pragma unroll 4
+    for (int k = 0; k < kTile; ++k) {
+      const T av = A[k * kTileLd + lane];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = (T)0;
-#pragma unroll 2
-  for (int k = 0; k < kTile; ++k) {
-    T a0[4], a1[4], b0[4], b1[4];
-    lds4(As + k * kSbDim + tx * 4, a0);
-    lds4(As + k * kSbDim + 64 + tx * 4, a1);
-    lds4(Bs + k * kSbDim + ty * 4, b0);
-    lds4(Bs + k * kSbDim + 64 + ty * 4, b1);
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        acc[i][j] = accT(acc[i][j], a0[i], b0[j]);
-        acc[i][4 + j] = accT(acc[i][4 + j], a0[i], b1[j]);
-        acc[4 + i][j] = accT(acc[4 + i][j], a1[i], b0[j]);
-        acc[4 + i][4 + j] = accT(acc[4 + i][4 + j], a1[i], b1[j]);
-      }
-  }
-  // (4) C -= product in shared memory (each thread its own 64 entries of the copied C tiles;
-  //     entries of tiles that are not updated are never stored back)
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int R = (i < 4) ? tx * 4 + i : 64 + tx * 4 + (i - 4);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int Cc = (j < 4) ? ty * 4 + j : 64 + ty * 4 + (j - 4);
-      T& cref = Cs[((R >> 5) * 4 + (Cc >> 5)) * kTileElems + (Cc & 31) * kTileLd + (R & 31)];
-      cref = cref - accEnd(acc[i][j]);
+      for (int j = 0; j < 4; ++j) acc[j] = accT(acc[j], av, B[k * kTileLd + c0 + j]);
     }
+    int I, K;
+    where(t, I, K);
+    T* out = M + tileBase(Tn, I, K);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      out[(c0 + j) * kTileLd + lane] = C[(c0 + j) * kTileLd + lane] - accEnd(acc[j]);
+    __syncthreads();  // this set of tiles is free for the copies after the next
   }
-  __syncthreads();
-  // (5) back to global memory, 16-byte vectors
-  for (int v = tid; v < 16 * vpt; v += blockDim.x) {
-    const int t = v / vpt, a = t >> 2, b = t & 3;
-    if (a < ni && b < nk && !(diagSb && b > a) && !(skip00 && t == 0))
-      *reinterpret_cast<uint4*>(M + tileBase(Tn, I0 + a, K0 + b) + (v - t * vpt) * per16) =
-          *reinterpret_cast<const uint4*>(Cs + v * per16);
-  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // FP32 trailing update of tile column J on the tensor cores (tcgen05, kind::tf32): the same
-// C_IK -= L_IJ D_J L_KJ^T as superSyrk, over every super-block this CTA owns in the step
+// C_IK -= L_IJ D_J L_KJ^T as gridTileUpdate, over every super-block this CTA owns in the step
 // (sb = blockIdx.x - 1, + gridDim.x - 1, ...). Each FP32 operand is split as hi + lo (hi = its
 // TF32 rounding, lo = the TF32 rounding of the remainder) and the product taken as
 // A_lo B_hi + A_hi B_lo + A_hi B_hi (3xTF32; the A_lo B_lo term is below FP32 rounding): twelve
@@ -1890,14 +1847,14 @@ __device__ __noinline__ bool gridLdltPairs(GridCtl* g, int nr, int nx, const Dev
 
 // Tiled right-looking LDL' of the root over the whole grid. Per tile column J:
 //  (A) the off-diagonal tiles of column J, up to four warps each; barrier;
-//  (B) the trailing update C_IK -= L_IJ D_J L_KJ^T, J < K <= I, in super-blocks of 4x4 tiles, one
-//      CTA each (CTAs 1..: FP32 on the tensor cores, tcTrailingStep; FP64 and double-float on the
-//      CUDA cores, superSyrk), while CTA 0 updates the tile (J+1, J+1) with the tile routine and
+//  (B) the trailing update C_IK -= L_IJ D_J L_KJ^T, J < K <= I, on CTAs 1.. (FP32: super-blocks of 4x4
+//      tiles on the tensor cores, tcTrailingStep; FP64 and double-float: tile by tile on the CUDA
+//      cores, gridTileUpdate), while CTA 0 updates the tile (J+1, J+1) with the tile routine and
 //      factors it (one-column lookahead); barrier.
 // In FP64 every root entry receives its updates in increasing J with the same operations and
 // rounding as the single-CTA factor, so both give the same bits. Only CTA 0 factors diagonal
 // tiles, so the pivot statistics stay in its shared memory (ps). `stage` holds
-// gridStageBytes. Large FP32 and double-float roots run over column pairs instead (gridLdltPairs).
+// kGridStageBytes. Large FP32 and double-float roots run over column pairs instead (gridLdltPairs).
 template <typename T>
 __device__ __noinline__ bool gridLdltSteps(GridCtl* g, int nr, int nx, const DevSettings& st, T* M, PivotStats* ps,
                                            T* stage, unsigned char* slices, int Tn, int warp, int gw, int GW, bool cta0,
@@ -1972,8 +1929,7 @@ __device__ __noinline__ bool gridLdltSteps(GridCtl* g, int nr, int nx, const Dev
     const int nb = (rem + 3) >> 2;
     const long long nsb = (long long)nb * (nb + 1) / 2;
     // CTA 0 updates and factors the next diagonal tile (J+1, J+1), the critical path of the next
-    // column; the super-blocks (row order: sb = r (r + 1) / 2 + k, tile rows J+1+4r.., tile
-    // columns J+1+4k..) go to CTAs 1.. cyclically, super-block 0 without that tile
+    // column; the rest of the update goes to CTAs 1.. cyclically
     if (cta0) {
       gridNextDiag<T>(M, Tn, J + 1, M + tileBase(Tn, J + 1, J), Ajj, nullptr, nullptr, nr, nx, st, ps, cs);
       if (!gridSync(g)) return false;
@@ -1986,11 +1942,7 @@ __device__ __noinline__ bool gridLdltSteps(GridCtl* g, int nr, int nx, const Dev
         return false;
       }
     } else {
-      for (long long sb = (long long)blockIdx.x - 1; sb < nsb; sb += (long long)gridDim.x - 1) {
-        const SbGeo gg = sbGeo(sb, J, Tn);
-        __syncthreads();  // the previous super-block is done with the staging area
-        superSyrk<T>(M, Tn, J, gg.I0, gg.K0, gg.ni, gg.nk, gg.diag, gg.skip00, stage);
-      }
+      gridTileUpdate<T>(M, Tn, J, stage);
     }
     if (!gridSync(g)) return false;
   }

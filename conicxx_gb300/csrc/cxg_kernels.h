@@ -24,13 +24,12 @@ struct SmemLayout {
 // 128 bytes of alignment slack.
 constexpr int64_t kGridTcStageBytes = 4 * 16384 + 2 * 16 * (int64_t)kTileElems * 4 + 128;
 
-// Staging area of a CTA in the whole-GPU form, for every arithmetic: the trailing update on the
-// CUDA cores (two 32x128 panels and 16 tiles of 8-byte entries), the one on the tensor cores, or the
-// triangular solves (three tiles and one 32-entry vector a warp, three vectors more), whichever is
-// largest.
+// Staging area of a CTA in the whole-GPU form, for every arithmetic: the trailing update on the tensor
+// cores, the column phases of the factor (19 tiles of 8-byte entries and two vectors) or the triangular
+// solves (three tiles and one 32-entry vector a warp, three vectors more), whichever is largest.
 constexpr int64_t kGridStageBytes = []() constexpr {
-  const int64_t syrk = (2ll * kTile * 128 + 16ll * kTileElems) * 8, solve = (8 * 3 * (int64_t)kTileElems + 96 + 256) * 8;
-  const int64_t a = syrk > kGridTcStageBytes ? syrk : kGridTcStageBytes;
+  const int64_t col = (64 + 19 * (int64_t)kTileElems) * 8, solve = (8 * 3 * (int64_t)kTileElems + 96 + 256) * 8;
+  const int64_t a = col > kGridTcStageBytes ? col : kGridTcStageBytes;
   return a > solve ? a : solve;
 }();
 

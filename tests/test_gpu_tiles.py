@@ -29,3 +29,20 @@ def test_factor_is_the_same_for_every_split(nr, arith):
             assert np.max(np.abs(D - D0)) <= tol * np.max(np.abs(D0))
             assert np.max(np.abs(L - L0)) <= tol * max(1.0, np.max(np.abs(L0)))
         assert np.array_equal(L, ref[0]) and np.array_equal(D, ref[1]), threads
+
+
+@pytest.mark.parametrize("arith", ["fp64", "df64"])
+@pytest.mark.parametrize("nr", [64, 65, 97, 545, 577, 801])
+def test_whole_gpu_update_tile_by_tile(nr, arith):
+    """The whole-GPU trailing update at its edges: no tile beside the lookahead's (2 tile columns),
+    two (3), then fewer tiles than CTAs, about one each (18 tile columns: 152 tiles in the first
+    step), and more than one each (both copy buffers in turn)."""
+    nx = nr - nr // 8
+    K = quasi_definite(nr, nx, seed=nr)
+    b = np.random.default_rng(nr).standard_normal(nr)
+    L, D, x, _, flags = probe(K, nx, b, arith, -1)
+    assert flags[0] == 0 and flags[1] == 0
+    L0, D0 = ldlt_ref(K)
+    tol = TOL[arith]
+    assert np.max(np.abs(D - D0)) <= tol * np.max(np.abs(D0))
+    assert np.max(np.abs(L - L0)) <= tol * max(1.0, np.max(np.abs(L0)))
