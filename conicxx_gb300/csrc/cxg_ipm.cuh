@@ -28,11 +28,11 @@
 
 namespace cxg {
 
-#define FOR_T(i, n) for (int i = (int)threadIdx.x; i < (n); i += (int)blockDim.x)
+#define FOR_T(i, n) _Pragma("unroll 1") for (int i = (int)threadIdx.x; i < (n); i += (int)blockDim.x)
 // The elements a thread sums: over the first `vb` threads of the block (Ctx::vb). A sum's order, and so its
 // rounding, is that of a block of vb threads whatever the block's real size; a batch that leaves SMs
 // free runs blocks wider than that (threads beyond vb add zeros to nothing).
-#define FOR_V(i, n, vb) for (int i = (int)threadIdx.x < (vb) ? (int)threadIdx.x : (n); i < (n); i += (vb))
+#define FOR_V(i, n, vb) _Pragma("unroll 1") for (int i = (int)threadIdx.x < (vb) ? (int)threadIdx.x : (n); i < (n); i += (vb))
 
 // A sparse matrix in the plan's slice order (sliceRows): rows sorted by length, 32 a slice.
 struct Sliced {

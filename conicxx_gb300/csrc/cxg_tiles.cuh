@@ -119,7 +119,7 @@ __device__ __forceinline__ void tilePivotStats(const T* A, int J, int nr, int nx
 // factor, which is stored transposed in the upper half: Linv(r, c) at r*ld + c. Only the
 // per-pivot regularisation test runs inside the loop, in the tile's own arithmetic.
 template <typename T>
-__device__ void tileFactorDiagRegs(T* A, int J, int nr, int nx, const DevSettings& st, PivotStats* ps, T* invD) {
+__device__ __noinline__ void tileFactorDiagRegs(T* A, int J, int nr, int nx, const DevSettings& st, PivotStats* ps, T* invD) {
   const int r = threadIdx.x & 31;
   const bool regularized = st.linear_solver == 2;
   const T epsT = (T)st.dynamic_reg_eps, deltaT = (T)st.dynamic_reg_delta;
