@@ -28,11 +28,19 @@
 
 namespace cxg {
 
-#define FOR_T(i, n) _Pragma("unroll 1") for (int i = (int)threadIdx.x; i < (n); i += (int)blockDim.x)
+// Rolled loops in the batched kernels: most run once or twice, and the unrolled copies were a third of
+// 1.6 MB of code, far more than an SM's instruction caches hold. SMs that run different code then slow
+// each other down: in a batch of 4096 problems an iteration of a 165-row root took 860 us where it takes
+// 630 us alone; with 0.5 MB less of code on its path 650 to 700 us. The whole-GPU kernels, one instance
+// with vectors in global memory, unroll by four to have more loads in flight.
+#ifndef CXG_VEC_UNROLL
+#define CXG_VEC_UNROLL "unroll 1"
+#endif
+#define FOR_T(i, n) _Pragma(CXG_VEC_UNROLL) for (int i = (int)threadIdx.x; i < (n); i += (int)blockDim.x)
 // The elements a thread sums: over the first `vb` threads of the block (Ctx::vb). A sum's order, and so its
 // rounding, is that of a block of vb threads whatever the block's real size; a batch that leaves SMs
 // free runs blocks wider than that (threads beyond vb add zeros to nothing).
-#define FOR_V(i, n, vb) _Pragma("unroll 1") for (int i = (int)threadIdx.x < (vb) ? (int)threadIdx.x : (n); i < (n); i += (vb))
+#define FOR_V(i, n, vb) _Pragma(CXG_VEC_UNROLL) for (int i = (int)threadIdx.x < (vb) ? (int)threadIdx.x : (n); i < (n); i += (vb))
 
 // A sparse matrix in the plan's slice order (sliceRows): rows sorted by length, 32 a slice.
 struct Sliced {
@@ -161,8 +169,9 @@ __device__ __forceinline__ double warpSums(const double (&v)[K]) {
 // 32 / nw) values from k0 on: value k0 + i's in the lanes i * nw .. of the calling warp. Block
 // sizes of 1, 2, 4 or 8 warps.
 __device__ __forceinline__ double warpTotals(const double* red, int k0, int nw) {
-  const int lane = threadIdx.x & 31;
-  double t = red[min(k0 + lane / nw, 7) * 16 + lane % nw];
+  const int lane = threadIdx.x & 31, sh = 31 - __clz(nw);
+  double t = red[min(k0 + (lane >> sh), 7) * 16 + (lane & (nw - 1))];
+#pragma unroll 1
   for (int o = 1; o < nw; o <<= 1) t = t + __shfl_xor_sync(0xffffffffu, t, o);
   return t;
 }
@@ -177,17 +186,17 @@ __device__ __forceinline__ void blockPartials(const double (&v)[K], double* red,
   __syncthreads();
 }
 
+// A function of its own, called with K = 2, 4 and 6: inlined it was 25 KB of code at six sums.
 template <int K>
-__device__ __forceinline__ void blockSum(double (&v)[K], double* red, int vb) {
-  const int nw = vb >> 5;
+__device__ __noinline__ void blockSum(double (&v)[K], double* red, int vb) {
+  const int nw = vb >> 5, lane = threadIdx.x & 31;
   blockPartials<K>(v, red, nw);
-  if (nw & (nw - 1)) {  // a number of warps that is no power of two: in sequence
+  if (nw & (nw - 1)) {  // a number of warps that is no power of two: in sequence, value k in lane k
+    double t = 0.0;
+#pragma unroll 1
+    for (int j = 0; j < nw; ++j) t += red[min(lane, 7) * 16 + j];
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      double t = 0.0;
-      for (int j = 0; j < nw; ++j) t += red[k * 16 + j];
-      v[k] = t;
-    }
+    for (int k = 0; k < K; ++k) v[k] = __shfl_sync(0xffffffffu, t, k);
     return;
   }
 #pragma unroll
@@ -364,9 +373,10 @@ static __device__ __noinline__ void coneApply(Ctx& c, int f, double eps, const d
   __syncthreads();
 }
 
-// out = G x on the cone rows with the G eigenvalues prepared at factorisation (Zero rows: 0).
-static __device__ __noinline__ void coneApplyG(Ctx& c, const double* x, double* out) {
-  FOR_T(r, c.p) out[r] = 0.0;
+// out = G x on the cone rows with the G eigenvalues prepared at factorisation (Zero rows: 0, or left as
+// they are).
+static __device__ __noinline__ void coneApplyG(Ctx& c, const double* x, double* out, bool zeroRows) {
+  if (zeroRows) FOR_T(r, c.p) out[r] = 0.0;
   FOR_T(t, c.l + c.nsoc) {
     if (t >= c.nsoc) {
       const int r = c.p + (t - c.nsoc);
@@ -472,34 +482,52 @@ static __device__ void ensureStrictlyInteriorWarm(Ctx& c, double* v) {
 // Slices of 32 rows.
 __device__ __forceinline__ int slices(int rows) { return (rows + 31) >> 5; }
 
-// y = P_sym x (full symmetric P, one thread per row)
-static __device__ __noinline__ void pmul(Ctx& c, const double* x, double* y) {
-  for (int q, i = 0; i * (int)(blockDim.x >> 5) < slices(c.n); ++i) {
+// What sliceProducts forms, and how.
+enum {
+  kProdP = 1,         // px = P x
+  kProdCols = 2,      // atz = A' z
+  kProdRows = 4,      // ax = A x
+  kProdColsFour = 8,  // A' z in four interleaved sums
+  kProdInit = 16,     // A_C' z + init (without the Zero rows) and A_C x - init (on the cone rows)
+  kProdColsF32 = 32, kProdColsDf = 64  // atz is an array of float / df64
+};
+
+// The products asked for, the slices of all of them as one list of tasks, the long rows of P first. One
+// function for every product of the iteration: each inlined copy of sliceDot was 5 to 11 KB of code.
+static __device__ __noinline__ void sliceProducts(Ctx& c, int what, const double* x, const double* z, double* px,
+                                                  void* atz, double* ax, const double* init) {
+  const int sn = slices(c.n);
+  const int eP = (what & kProdP) ? sn : 0, eC = eP + ((what & kProdCols) ? sn : 0);
+  const int end = eC + ((what & kProdRows) ? slices(c.m) : 0);
+  const bool add = what & kProdInit;
+#pragma unroll 1
+  for (int q, i = 0; i * (int)(blockDim.x >> 5) < end; ++i) {
     q = snakeTask(i);
-    if (q >= slices(c.n)) break;
+    if (q >= end) continue;
+    const int kind = (q >= eP) + (q >= eC);
+    const Sliced& A = kind == 0 ? c.sP : kind == 1 ? c.sAc : c.sAr;
     int row;
-    const double v = sliceDot(c.sP, true, q, x, row);
-    if (row >= 0) y[row] = v;
+    const double v = sliceDot(A, kind == 0 || (kind == 1 && (what & kProdColsFour)), q - (kind == 0 ? 0 : kind == 1 ? eP : eC),
+                              kind == 1 ? z : x, row, add ? init : nullptr, kind == 2, add && kind == 1 ? c.p : 0);
+    if (row < 0) continue;
+    if (kind == 0) px[row] = v;
+    else if (kind == 2) { if (!add || row >= c.p) ax[row] = v; }
+    else if (what & kProdColsF32) reinterpret_cast<float*>(atz)[row] = (float)v;
+    else if (what & kProdColsDf) reinterpret_cast<df64*>(atz)[row] = (df64)v;
+    else reinterpret_cast<double*>(atz)[row] = v;
   }
   __syncthreads();
 }
 
-// px = P x, atz = A'z (interleaved sums) and ax = A x: the slices of all three as one list of tasks,
-// the long rows of P first.
-static __device__ __noinline__ void kktProducts(Ctx& c, const double* x, const double* z, double* px, double* atz,
-                                                double* ax) {
-  const int sn = slices(c.n), sm = slices(c.m);
-  for (int q, i = 0; i * (int)(blockDim.x >> 5) < 2 * sn + sm; ++i) {
-    q = snakeTask(i);
-    if (q >= 2 * sn + sm) continue;
-    const int kind = (q >= sn) + (q >= 2 * sn);
-    const Sliced& A = kind == 0 ? c.sP : kind == 1 ? c.sAc : c.sAr;
-    double* out = kind == 0 ? px : kind == 1 ? atz : ax;
-    int row;
-    const double v = sliceDot(A, kind < 2, q - (kind == 0 ? 0 : kind == 1 ? sn : 2 * sn), kind == 1 ? z : x, row);
-    if (row >= 0) out[row] = v;
-  }
-  __syncthreads();
+// y = P_sym x (full symmetric P)
+static __device__ __forceinline__ void pmul(Ctx& c, const double* x, double* y) {
+  sliceProducts(c, kProdP, x, nullptr, y, nullptr, nullptr, nullptr);
+}
+
+// px = P x, atz = A'z (interleaved sums) and ax = A x
+static __device__ __forceinline__ void kktProducts(Ctx& c, const double* x, const double* z, double* px, double* atz,
+                                                   double* ax) {
+  sliceProducts(c, kProdP | kProdCols | kProdRows | kProdColsFour, x, z, px, atz, ax, nullptr);
 }
 
 // res = rhs - K sol for the statically-regularised K (the matrix refinement targets,
@@ -583,7 +611,7 @@ static __device__ double kktResidual(Ctx& c, const DevSettings& st, const double
 __device__ __forceinline__ int diagWarps(int nw) { return nw >= 8 ? 4 : min(nw, 2); }
 
 // The root's LDL' by one CTA, right-looking by tile column J with a one-column lookahead:
-//  (1) the off-diagonal tiles of column J, each split over one, two or four warps by columns;
+//  (1) the off-diagonal tiles of column J by groups of eight columns;
 //  (2) the next diagonal tile's product on up to six warps, then its factorisation by
 //      diagWarps() warps while the others take the other products of column J from a queue
 //      (half a tile each), joined by the factoring warps when they are done.
@@ -608,30 +636,17 @@ __device__ __noinline__ void denseLdlt(Ctx& c, T* M, const DevSettings& st, int&
     T* Ajj = M + tileBase(Tn, J, J);
     const int rem = Tn - J - 1;
     if (threadIdx.x == 0) ps->next = 0;
-    if (2 * rem > nw) {
-      for (int I = J + 1 + warp; I < Tn; I += nw) tileOffDiag<T>(M + tileBase(Tn, I, J), Ajj, invD);
-    } else if (4 * rem > nw) {
-      // two warps a tile: columns 0-7 and 24-31, or 8-23 (five units of 8x8 products each)
-      T* Aij = M + tileBase(Tn, J + 1 + (warp >> 1), J);
-      const bool on = (warp >> 1) < rem;
-      const int g0 = (warp & 1) ? 1 : 0, g1 = (warp & 1) ? 2 : 3;
-      T o0[8], o1[8];
-      if (on) {
-        tileOffDiagGroup(Aij, Ajj, invD, g0, o0);
-        tileOffDiagGroup(Aij, Ajj, invD, g1, o1);
-      }
+    // column groups (tileOffDiagGroup) of the column's tiles, one a warp and round, the last (longest)
+    // groups first. A group reads its own and earlier columns of its tile: what a round stores, after
+    // the barrier, is not read by that tile's groups still to come.
+#pragma unroll 1
+    for (int t = warp; t - warp < 4 * rem; t += nw) {
+      T o[8];
+      const int g = 3 - t / rem;
+      T* Aij = M + tileBase(Tn, J + 1 + t % rem, J);
+      if (t < 4 * rem) tileOffDiagGroup(Aij, Ajj, invD, g, o);
       __syncthreads();
-      if (on) {
-        tileOffDiagStore(Aij, g0, o0);
-        tileOffDiagStore(Aij, g1, o1);
-      }
-    } else {
-      T* Aij = M + tileBase(Tn, J + 1 + (warp >> 2), J);
-      const bool on = (warp >> 2) < rem;
-      T o0[8];
-      if (on) tileOffDiagGroup(Aij, Ajj, invD, warp & 3, o0);
-      __syncthreads();
-      if (on) tileOffDiagStore(Aij, warp & 3, o0);
+      if (t < 4 * rem) tileOffDiagStore(Aij, g, o);
     }
     __syncthreads();
     const int ntask = rem * (rem + 1) - 2;  // halves of the pairs (I, K), J < K <= I, but the first
@@ -710,11 +725,13 @@ __device__ void denseSolve(Ctx& c, const T* M, T* y) {
     T* yJ = y + J * 32;
     if ((int)threadIdx.x < 32 * sd) {
       T acc = (T)0;
-#pragma unroll 4
-      for (int col = dp * wd; col < (dp + 1) * wd; ++col) {
-        const T l = Ajj[di * kTileLd + col];
-        acc = accT(acc, col < di ? l : (T)0, yJ[col]);
-      }
+#pragma unroll 1
+      for (int c0 = dp * wd; c0 < (dp + 1) * wd; c0 += 4)
+#pragma unroll
+        for (int col = c0; col < c0 + 4; ++col) {
+          const T l = Ajj[di * kTileLd + col];
+          acc = accT(acc, col < di ? l : (T)0, yJ[col]);
+        }
       const T tot = groupSum(accEnd(acc), sd);
       if (dp == 0) x[di] = yJ[di] + tot;
     }
@@ -723,19 +740,23 @@ __device__ void denseSolve(Ctx& c, const T* M, T* y) {
     const int rows = (Tn - J - 1) * 32;
     if (rows > 0) {
       const int s = dotSplit(rows, c.vb), w = 32 / s;
+#pragma unroll 1
       for (int t = threadIdx.x; t < rows * s; t += nth) {
         const int row = t / s, p = t % s;
         const int I = J + 1 + row / 32, rr = row % 32;
         const T* Lij = M + tileBase(Tn, I, J);
         T acc = (T)0;
-#pragma unroll 4
-        for (int col = p * w; col < (p + 1) * w; ++col) acc = accT(acc, Lij[col * kTileLd + rr], x[col]);
+#pragma unroll 1
+        for (int c0 = p * w; c0 < (p + 1) * w; c0 += 4)
+#pragma unroll
+          for (int col = c0; col < c0 + 4; ++col) acc = accT(acc, Lij[col * kTileLd + rr], x[col]);
         acc = groupSum(accEnd(acc), s);
         if (p == 0) y[I * 32 + rr] -= acc;
       }
     }
     __syncthreads();
   }
+#pragma unroll 1
   for (int t = threadIdx.x; t < Tn * 32; t += nth) {
     const int J = t / 32, rr = t % 32;
     y[t] /= M[tileBase(Tn, J, J) + rr * kTileLd + rr];
@@ -747,11 +768,13 @@ __device__ void denseSolve(Ctx& c, const T* M, T* y) {
     T* yJ = y + J * 32;
     if ((int)threadIdx.x < 32 * sd) {
       T acc = (T)0;
-#pragma unroll 4
-      for (int row = dp * wd; row < (dp + 1) * wd; ++row) {
-        const T l = Ajj[row * kTileLd + di];
-        acc = accT(acc, row > di ? l : (T)0, yJ[row]);
-      }
+#pragma unroll 1
+      for (int r0 = dp * wd; r0 < (dp + 1) * wd; r0 += 4)
+#pragma unroll
+        for (int row = r0; row < r0 + 4; ++row) {
+          const T l = Ajj[row * kTileLd + di];
+          acc = accT(acc, row > di ? l : (T)0, yJ[row]);
+        }
       const T tot = groupSum(accEnd(acc), sd);
       if (dp == 0) x[di] = yJ[di] + tot;
     }
@@ -760,13 +783,16 @@ __device__ void denseSolve(Ctx& c, const T* M, T* y) {
     const int rows = J * 32;
     if (rows > 0) {
       const int s = dotSplit(rows, c.vb), w = 32 / s;
+#pragma unroll 1
       for (int t = threadIdx.x; t < rows * s; t += nth) {
         const int row = t / s, p = t % s;
         const int K = row / 32, cc = row % 32;
         const T* Ljk = M + tileBase(Tn, J, K);
         T acc = (T)0;
-#pragma unroll 4
-        for (int r2 = p * w; r2 < (p + 1) * w; ++r2) acc = accT(acc, Ljk[cc * kTileLd + r2], x[r2]);
+#pragma unroll 1
+        for (int r0 = p * w; r0 < (p + 1) * w; r0 += 4)
+#pragma unroll
+          for (int r2 = r0; r2 < r0 + 4; ++r2) acc = accT(acc, Ljk[cc * kTileLd + r2], x[r2]);
         acc = groupSum(accEnd(acc), s);
         if (p == 0) y[K * 32 + cc] -= acc;
       }
@@ -2299,8 +2325,10 @@ __device__ __noinline__ void assembleFactor(Ctx& c, const DevSettings& st, T* M,
     return;
   }
   const int64_t rs = rootSize(nr);
+#pragma unroll 1
   for (int64_t t = threadIdx.x; t < rs; t += blockDim.x) M[t] = (T)0;
   __syncthreads();
+#pragma unroll 1
   for (int i = nr + (int)threadIdx.x; i < rootTiles(nr) * kTile; i += blockDim.x) M[rootIdx(nr, i, i)] = (T)1;
   FOR_T(i, n) {
     const int src = c.pdiag[i];
@@ -2324,23 +2352,18 @@ __device__ __noinline__ void assembleFactor(Ctx& c, const DevSettings& st, T* M,
 template <typename T, bool G = false>
 __device__ __noinline__ void reducedSolve(Ctx& c, const DevSettings& st, const T* M, double ea,
                              const double* rhs, double* sol) {
-  const int n = c.n, m = c.m, p = c.p, nr = c.nr;
-  const double epsA = st.static_reg_A + ea;
+  const int n = c.n, p = c.p, nr = c.nr;
   const double* r1 = rhs;
   const double* r2 = rhs + n;
   // u = G_C r2_C (eigenvalues of G prepared at factorisation time)
-  coneApplyG(c, r2, c.tm);
+  coneApplyG(c, r2, c.tm, true);
   // t = [r1 + A_C' u ; r2_Z] in T precision
   T* y = reinterpret_cast<T*>(c.rr);
-  for (int q, i = 0; i * (int)(blockDim.x >> 5) < slices(n); ++i) {
-    if ((q = snakeTask(i)) >= slices(n)) break;
-    int j;
-    const double acc = sliceDot(c.sAc, false, q, c.tm, j, r1, false, p);
-    if (j >= 0) y[j] = (T)acc;
-  }
   FOR_T(r, p) y[n + r] = (T)r2[r];
+#pragma unroll 1
   for (int i = nr + (int)threadIdx.x; i < rootTiles(nr) * kTile; i += blockDim.x) y[i] = (T)0;
-  __syncthreads();
+  constexpr int kOut = ArithOf<T>::v == 1 ? kProdColsF32 : ArithOf<T>::v == 2 ? kProdColsDf : 0;
+  sliceProducts(c, kProdCols | kProdInit | kOut, nullptr, c.tm, nullptr, y, nullptr, r1);
   const long long t0 = (st.record_timings && threadIdx.x == 0) ? clock64() : 0;
   if constexpr (G) {
     // whole-GPU launch; a failed barrier leaves a non-finite solution, which the caller's
@@ -2356,26 +2379,9 @@ __device__ __noinline__ void reducedSolve(Ctx& c, const DevSettings& st, const T
   FOR_T(r, p) sol[n + r] = (double)y[n + r];
   __syncthreads();
   // z_C = G_C (A_C x - r2_C)
-  for (int q, i = 0; i * (int)(blockDim.x >> 5) < slices(m); ++i) {
-    if ((q = snakeTask(i)) >= slices(m)) break;
-    int r;
-    const double acc = sliceDot(c.sAr, false, q, sol, r, r2, true);
-    if (r >= p) c.tm[r] = acc;
-  }
-  __syncthreads();
-  FOR_T(t, c.l + c.nsoc) {
-    if (t >= c.nsoc) {
-      const int r = p + (t - c.nsoc);
-      sol[n + r] = c.tm[r] * c.cu[r];
-    } else {
-      const int b = t;
-      const int off = c.socOff[b], d = c.socDim[b];
-      socApplyG(c.sp[b], c.cu + off, d, c.tm + off, sol + n + off);
-    }
-  }
-  __syncthreads();
-  (void)nr;
-  (void)epsA;
+  sliceProducts(c, kProdRows | kProdInit, sol, nullptr, nullptr, nullptr, c.tm, r2);
+  coneApplyG(c, c.tm, sol + n, false);
+  (void)ea;
 }
 
 // Factorisation state of the current iteration.
@@ -2786,14 +2792,7 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
     pmul(c, c.x, c.tn);  // Px
     {
       // A'z and A x (into dx and tm, free here)
-      for (int q, i = 0; i * (int)(blockDim.x >> 5) < slices(n) + slices(m); ++i) {
-        if ((q = snakeTask(i)) >= slices(n) + slices(m)) continue;
-        const bool cols = q < slices(n);
-        int row;
-        const double v = sliceDot(cols ? c.sAc : c.sAr, false, cols ? q : q - slices(n), cols ? c.z : c.x, row);
-        if (row >= 0) (cols ? c.dx : c.tm)[row] = v;
-      }
-      __syncthreads();
+      sliceProducts(c, kProdCols | kProdRows, c.x, c.z, nullptr, c.dx, c.tm, nullptr);
       double v[6] = {0, 0, 0, 0, 0, 0};
       FOR_V(t, n + m, c.vb) {
         if (t < n) {
@@ -2861,13 +2860,13 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       kktSolve<FT, G>(c, st, fs, c.rhs, c.sol);
       if (!vecFinite(c, c.sol, N)) { status = 5; break; }
       if (c.sc[SC_PXOK] == 0.0) pmul(c, c.sol, c.tn);  // P xv
-      double tn3[3] = {0, 0, 0};
+      double tn3[4] = {0, 0, 0, 0};
       FOR_V(j, n, c.vb) {
         tn3[0] += c.qs[j] * c.sol[j];
         tn3[2] += (c.x[j] / tau) * c.tn[j];
       }
       FOR_V(r, m, c.vb) tn3[1] += c.bs[r] * c.sol[n + r];
-      blockSum<3>(tn3, c.red, c.vb);
+      blockSum<4>(tn3, c.red, c.vb);
       const double dkrA = tau * kappa;
       const double tauNumA = rtau - dkrA / tau + tn3[0] + tn3[1] + 2.0 * tn3[2];
       if (tauDen == 0.0 || !isfinite(tauNumA) || !isfinite(tauDen)) { status = 5; break; }
@@ -2891,9 +2890,9 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       if (dtauA < 0) aaff = fmin(aaff, -tau / dtauA);
       if (dkappaA < 0) aaff = fmin(aaff, -kappa / dkappaA);
       aaff = coneMaxStep2(c, aaff);
-      double sa[1] = {0.0};
+      double sa[2] = {0.0, 0.0};
       FOR_V(r, m, c.vb) sa[0] += (c.s[r] + aaff * c.ds[r]) * (c.z[r] + aaff * c.dz[r]);
-      blockSum<1>(sa, c.red, c.vb);
+      blockSum<2>(sa, c.red, c.vb);
       const double tauAff = fma(aaff, dtauA, tau);
       const double kappaAff = fma(aaff, dkappaA, kappa);
       const double muAff = fma(tauAff, kappaAff, sa[0]) / (double)(degree + 1);
@@ -2927,7 +2926,7 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
         tn3[2] += (c.x[j] / tau) * c.tn[j];
       }
       FOR_V(r, m, c.vb) tn3[1] += c.bs[r] * c.sol[n + r];
-      blockSum<3>(tn3, c.red, c.vb);
+      blockSum<4>(tn3, c.red, c.vb);
       const double dtrC = (1.0 - sigma) * rtau;
       const double dkrC = fma(-sigma, mu, fma(tau, kappa, __dmul_rn(dtauA, dkappaA)));
       const double tauNumC = dtrC - dkrC / tau + tn3[0] + tn3[1] + 2.0 * tn3[2];
@@ -2998,12 +2997,15 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
     const int64_t rs = rootSize(c.nr);
     if (sizeof(FT) == 8) {
       const double* R = fs.use64 ? c.root64 : reinterpret_cast<const double*>(c.root);
+#pragma unroll 1
       for (int64_t t = threadIdx.x; t < rs; t += blockDim.x) Bs[bl.root + t] = R[t];
     } else if (fs.use64) {
       const auto* R = rootHigh<FT>(c);
+#pragma unroll 1
       for (int64_t t = threadIdx.x; t < rs; t += blockDim.x) Bs[bl.root + t] = (double)R[t];
     } else {
       const FT* R = rootT<FT>(c);
+#pragma unroll 1
       for (int64_t t = threadIdx.x; t < rs; t += blockDim.x) Bs[bl.root + t] = (double)R[t];
     }
     FOR_T(r, m) {
@@ -3207,6 +3209,7 @@ static __device__ __noinline__ void adjointInstance(Ctx& c, const LaunchArgs& a)
   FOR_T(k, kSocScaleDoubles * c.nsoc) reinterpret_cast<double*>(c.sp)[k] = Bs[bl.sp + k];
   if (a.lay.root64InSmem) {
     const int64_t rs = rootSize(c.nr);
+#pragma unroll 1
     for (int64_t t = threadIdx.x; t < rs; t += blockDim.x) c.root64[t] = Bs[bl.root + t];
   } else if (threadIdx.x == 0) {
     c.root64 = const_cast<double*>(Bs + bl.root);

@@ -68,9 +68,16 @@ __device__ __forceinline__ double recipT(double d) {
   e = fma(-d, r, 1.0);
   return fma(r, e, r);
 }
+static __device__ __noinline__ float2 dfRecipFar(float hi, float lo) {
+  const df64 q = df64(1.0f, 0.0f) / df64(hi, lo);
+  return make_float2(q.hi, q.lo);
+}
 __device__ __forceinline__ df64 recipT(df64 d) {
   const float af = fabsf(d.hi);
-  if (!(af >= 1e-37f && af <= 1e37f)) return df64(1.0f, 0.0f) / d;
+  if (!(af >= 1e-37f && af <= 1e37f)) {
+    const float2 q = dfRecipFar(d.hi, d.lo);
+    return df64(q.x, q.y);
+  }
   // one step from the 23-bit seed gives ~46 bits, the double-float rounding level
   const df64 r(__frcp_rn(d.hi), 0.0f);
   const df64 one(1.0f, 0.0f);
@@ -188,6 +195,19 @@ __device__ __noinline__ void tileFactorDiagRegs(T* A, int J, int nr, int nx, con
 // is left after the last leaf. One warp alone did all of it in sequence before: 50k cycles per
 // tile in double-float, 43% of them pivots (the chain that is left now).
 
+// The pivot rule (regularized: a pivot below eps with the expected sign is corrected). A function of its
+// own, as dfRecipFar is: eight copies of the two were half of the leaf's code.
+template <typename T>
+__device__ __noinline__ void pivotRule(T& dj, int g, int nr, int nx, T epsT, T deltaT, int& nreg) {
+  if (g >= nr) return;
+  const T sg = (g < nx) ? (T)1 : (T)-1;
+  if (dj * sg < epsT) {
+    dj = dj + sg * deltaT;
+    if (dj * sg < epsT) dj = sg * deltaT;
+    ++nreg;
+  }
+}
+
 // Leaf block b and its panel; one warp. Returns the number of regularised pivots.
 template <typename T>
 __device__ __forceinline__ int tileLeafPanel(T* A, int b, int J, int nr, int nx, bool regularized, T epsT, T deltaT,
@@ -206,17 +226,7 @@ __device__ __forceinline__ int tileLeafPanel(T* A, int b, int J, int nr, int nx,
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     T dj = shflT(a[j], c0 + j);
-    if (regularized) {
-      const int g = J * 32 + c0 + j;
-      if (g < nr) {
-        const T sg = (g < nx) ? (T)1 : (T)-1;
-        if (dj * sg < epsT) {
-          dj = dj + sg * deltaT;
-          if (dj * sg < epsT) dj = sg * deltaT;
-          ++nreg;
-        }
-      }
-    }
+    if (regularized) pivotRule(dj, J * 32 + c0 + j, nr, nx, epsT, deltaT, nreg);
     const T inv = recipT(dj);
     if (li == j) invMine = inv;
     const T lj = a[j] * inv;
@@ -260,6 +270,7 @@ __device__ __forceinline__ int tileLeafPanel(T* A, int b, int J, int nr, int nx,
 template <typename T>
 __device__ __forceinline__ void tileTrailing(T* A, int b, int end, int t, int nt) {
   const int c0 = 8 * b, o = c0 + 8, m = end - o;
+#pragma unroll 1
   for (int e = t; e < m * (m + 1) / 2; e += nt) {
     // e = i (i + 1) / 2 + k
     int i = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
@@ -346,6 +357,7 @@ __device__ __noinline__ void tileFactorDiagBlocked(T* A, int J, int nr, int nx, 
   const int helpers = max(gw - 1, 1), hw = (gw > 1) ? warp - 1 : 0;  // this warp among the helpers
   int nreg = 0;
   if (warp == 0 && (int)(threadIdx.x & 31) >= 8 * nb) invD[threadIdx.x & 31] = (T)1;
+#pragma unroll 1
   for (int b = 0; b < nb; ++b) {
     if (warp == 0) nreg += tileLeafPanel(A, b, J, nr, nx, regularized, epsT, deltaT, invD);
     if (gw == 1) __syncwarp();
@@ -354,6 +366,7 @@ __device__ __noinline__ void tileFactorDiagBlocked(T* A, int J, int nr, int nx, 
       if (hw == 0) tileLeafInverse(A, b - 1);
       if (helpers > 1) asm volatile("bar.sync 2, %0;" ::"r"(32 * helpers) : "memory");
       else __syncwarp();
+#pragma unroll 1
       for (int Jb = hw; Jb < b; Jb += helpers) {
         if (Jb < b - 1) tileInverseFinish(A, b - 1, Jb);
         tileInverseSum(A, b, Jb);
@@ -373,6 +386,7 @@ __device__ __noinline__ void tileFactorDiagBlocked(T* A, int J, int nr, int nx, 
     if (hw == 0) tileLeafInverse(A, nb - 1);
     if (helpers > 1) asm volatile("bar.sync 2, %0;" ::"r"(32 * helpers) : "memory");
     else __syncwarp();
+#pragma unroll 1
     for (int Jb = hw; Jb < nb - 1; Jb += helpers) tileInverseFinish(A, nb - 1, Jb);
   }
   groupSync(gt);
@@ -422,19 +436,6 @@ __device__ __forceinline__ void tileOffDiagStore(T* Aij, int g, const T (&out)[8
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int j = 0; j < 8; ++j) Aij[(8 * g + j) * kTileLd + lane] = out[j];
-}
-
-// The whole tile in place by one warp, last columns first.
-template <typename T>
-__device__ __noinline__ void tileOffDiag(T* Aij, const T* Ajj, const T* invD) {
-#pragma unroll 1
-  for (int g = 3; g >= 0; --g) {
-    T out[8];
-    tileOffDiagGroup(Aij, Ajj, invD, g, out);
-    __syncwarp();
-    tileOffDiagStore(Aij, g, out);
-    __syncwarp();
-  }
 }
 
 // ---- trailing products: C -= A diag(d) B^T, d = diagonal of the factored tile Ajj -----------------

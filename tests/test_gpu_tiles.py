@@ -6,6 +6,7 @@ for every block size; and they agree with numpy's LDL' within test_gpu_dense's t
 import numpy as np
 import pytest
 
+from conicxx_gb300 import _abi
 from test_gpu_dense import TOL, ldlt_ref, probe, quasi_definite
 
 pytestmark = pytest.mark.gpu
@@ -46,3 +47,17 @@ def test_whole_gpu_update_tile_by_tile(nr, arith):
     tol = TOL[arith]
     assert np.max(np.abs(D - D0)) <= tol * np.max(np.abs(D0))
     assert np.max(np.abs(L - L0)) <= tol * max(1.0, np.max(np.abs(L0)))
+
+
+@pytest.mark.parametrize("arith", ["fp64", "fp32", "df64"])
+@pytest.mark.parametrize("pos", [0, 3, 4, 7, 9, 31, 33, 36, 39])
+def test_regularized_pivot_at_every_place_of_a_leaf(pos, arith):
+    """A zero pivot at the edges of the leaf's two halves, in the last block and among the Zero-cone rows:
+    the rule puts delta = 1e-7 with the row's sign there; every other pivot stays exactly what it is."""
+    d = np.arange(1.0, 41.0)
+    d[36:] *= -1.0
+    d[pos] = 0.0
+    _, D, _, _, flags = probe(np.diag(d), 36, np.ones(40), arith, linear_solver=_abi.LINSOLVER_REGULARIZED)
+    assert flags[0] == 0
+    assert D[pos] == pytest.approx(1e-7 if pos < 36 else -1e-7, rel=1e-6)
+    assert np.array_equal(np.delete(D, pos), np.delete(d, pos))
