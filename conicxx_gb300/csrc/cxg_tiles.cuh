@@ -266,6 +266,72 @@ __device__ __forceinline__ int tileLeafPanel(T* A, int b, int J, int nr, int nx,
   return nreg;
 }
 
+#ifndef CXG_UNROLLED_LEAF
+// The double-float form of the batched kernels: rolled loops over the pivots, the row shifted down by
+// one entry a step (entry 0 is the pivot column's), seven updates a step for the first four and three
+// for the others. Alone it takes 13% longer than the unrolled form (4870 cycles a leaf, 4300), which the
+// whole-GPU kernels have; but that is 50 KB of code, and a batch whose SMs run different code then
+// spends 20% more on the factor. Entries shifted in from beyond the block are never used.
+template <int kUpd>
+__device__ __forceinline__ void dfLeafSteps(df64 (&a)[8], df64* A, int c0, int j0, int g0, int nr, int nx,
+                                            bool regularized, df64 epsT, df64 deltaT, int& nreg, df64& invMine) {
+  const int r = threadIdx.x & 31, li = r - c0;
+#pragma unroll 1
+  for (int j = j0; j < j0 + 4; ++j) {
+    const df64 aj = a[0];
+    df64 dj = shflT(aj, c0 + j);
+    if (regularized) pivotRule(dj, g0 + j, nr, nx, epsT, deltaT, nreg);
+    const df64 inv = recipT(dj);
+    if (li == j) invMine = inv;
+    const df64 lj = aj * inv;
+#pragma unroll
+    for (int k = 1; k <= kUpd; ++k) a[k - 1] = msubT(a[k], lj, shflT(aj, (c0 + j + k) & 31));
+    if (li >= j && li < 8) A[(c0 + j) * kTileLd + r] = (li > j) ? lj : dj;
+  }
+}
+template <int kUpd>
+__device__ __forceinline__ void dfPanelSteps(df64 (&u)[8], df64* A, int c0, int t0, const df64* invD) {
+  const int r = threadIdx.x & 31;
+#pragma unroll 1
+  for (int t = t0; t < t0 + 4; ++t) {
+    const df64* Ac = A + (c0 + t) * kTileLd + c0;
+    const df64 ut = u[0];
+#pragma unroll
+    for (int k = 1; k <= kUpd; ++k) u[k - 1] = msubT(u[k], ut, Ac[min(t + k, 7)]);
+    if (r >= c0 + 8) {
+      A[(c0 + t) * kTileLd + r] = ut * invD[c0 + t];
+      A[r * kTileLd + c0 + t] = ut;
+    }
+  }
+}
+__device__ __forceinline__ int tileLeafPanel(df64* A, int b, int J, int nr, int nx, bool regularized, df64 epsT,
+                                             df64 deltaT, df64* invD) {
+  const int r = threadIdx.x & 31, c0 = 8 * b, li = r - c0;
+  const bool leaf = li >= 0 && li < 8;
+  int nreg = 0;
+  df64 invMine(0.0f, 0.0f), a[8];
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {
+    const int ct = c0 + t;
+    const df64 v = A[(t <= li) ? ct * kTileLd + r : r * kTileLd + ct];
+    a[t] = leaf ? v : df64(0.0f, 0.0f);
+  }
+  __syncwarp();
+  dfLeafSteps<7>(a, A, c0, 0, J * 32 + c0, nr, nx, regularized, epsT, deltaT, nreg, invMine);
+  dfLeafSteps<3>(a, A, c0, 4, J * 32 + c0, nr, nx, regularized, epsT, deltaT, nreg, invMine);
+  if (leaf) invD[r] = invMine;
+  __syncwarp();
+  if (c0 + 8 < 32) {
+    df64 u[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) u[t] = A[(c0 + t) * kTileLd + r];  // rows above: not stored
+    dfPanelSteps<7>(u, A, c0, 0, invD);
+    dfPanelSteps<3>(u, A, c0, 4, invD);
+  }
+  return nreg;
+}
+#endif
+
 // Trailing entries (r, k), c0 + 8 <= k <= r < end, of block b: thread t of nt.
 template <typename T>
 __device__ __forceinline__ void tileTrailing(T* A, int b, int end, int t, int nt) {
