@@ -246,12 +246,14 @@ static int chooseBlock(int nrMax, int requested) {
 // earlier ones drain their queues, and their slowest instances then end the batch. Instead the
 // SMs are apportioned among the buckets in proportion to their estimated work, so that every
 // bucket's CTAs are resident from the start and the buckets finish together. Measured on the
-// contact batch, the SM time of an instance's iteration grows about linearly with its root size
-// nr: about 5 us x nr where a CTA has its SM to itself, about 3 us x nr where several CTAs share
-// one (their latency-bound chains overlap). A bucket's work is therefore the sum of its
-// instances' nr, times 0.6 for launch shapes with several CTAs per SM (iteration counts are
-// alike across buckets). A bucket never gets more SMs than its instances can fill; the rest go
-// to the others (largest-remainder apportionment).
+// contact batch (4096 instances, 12 to 192 rows), an iteration of an instance with its SM to itself
+// takes about 217 us + 2.26 us x nr (nr its root's rows), and with 2, 5 or 11 CTAs on the SM 0.76, 0.44
+// or 0.22 times that per instance (their latency-bound chains overlap): about occupancy^-0.5. A
+// bucket's work is therefore the sum of its instances' 96 + nr, times that (iteration counts are alike
+// across buckets). With 5 us x nr, and 3 us where an SM is shared, which fitted the slower kernels, the
+// buckets ended between 102 and 183 ms.
+// A bucket never gets more SMs than its instances can fill; the rest go to the others
+// (largest-remainder apportionment).
 static void partitionGrids(cxg_batch* B, int numSM) {
   const size_t G = B->groups.size();
   if (B->gridMode) {  // one cooperative launch over every SM
@@ -267,7 +269,7 @@ static void partitionGrids(cxg_batch* B, int numSM) {
   std::vector<bool> capped(G, false);
   auto weight = [&](size_t b) {
     const Group& g = B->groups[b];
-    return std::max(g.work, 1.0) * (g.occupancy > 1 ? 0.6 : 1.0);
+    return std::max(g.work, 1.0) * std::pow((double)g.occupancy, -0.5);
   };
   for (size_t b = 0; b < G; ++b) {
     const Group& g = B->groups[b];
@@ -315,6 +317,25 @@ static void partitionGrids(cxg_batch* B, int numSM) {
   for (size_t b = 0; b < G; ++b) {
     Group& g = B->groups[b];
     g.grid = std::max(1, std::min(g.count, sms[b] * g.occupancy));
+  }
+}
+
+// Block size and resident CTAs per SM of a bucket whose sums take g.sumThreads threads. A CTA that has
+// an SM to itself, because the batch has no more instances than SMs or because its shared memory leaves
+// no room for a second one, runs a 256-thread block whatever the size: the sums keep the order of the
+// narrower block (same bits), while the factor's tiles, the cones' lists and the sparse products spread
+// over all four sub-partitions. Not when the caller fixed the threads, and not where several CTAs
+// share an SM: narrow blocks use its FP64 units better there.
+static void shapeBlock(const cxg_batch* B, Group& g) {
+  auto occupancyOf = [&](int block) {
+    int occ = 0;
+    return (ipmOccupancy(&occ, block, g.smem, g.fp32) != cudaSuccess || occ < 1) ? 1 : occ;
+  };
+  g.block = B->wide ? 256 : g.sumThreads;
+  g.occupancy = occupancyOf(g.block);
+  if (g.occupancy == 1 && g.block < 256 && B->st.threads_per_instance == 0) {
+    g.block = 256;
+    g.occupancy = occupancyOf(g.block);
   }
 }
 
@@ -366,7 +387,7 @@ static int buildGroups(cxg_batch* B) {
       L.mMax = std::max(L.mMax, D.m);
       L.nrMax = std::max(L.nrMax, D.nr);
       L.nsocMax = std::max(L.nsocMax, D.nsoc);
-      g.work += (double)D.nr;  // scaled by the launch shape's sharing in partitionGrids
+      g.work += 96.0 + (double)D.nr;  // scaled by the launch shape's sharing in partitionGrids
     }
     const int64_t redBytes = (128 + 32) * 8;
     const int64_t vecBytes = vecDoubles(L.nMax, L.mMax, L.nrMax, L.nsocMax) * 8;
@@ -398,12 +419,7 @@ static int buildGroups(cxg_batch* B) {
     L.total = used;
     g.smem = (size_t)used;
     g.sumThreads = gridMode ? 256 : chooseBlock(L.nrMax, B->st.threads_per_instance);
-    // A batch with an SM for every instance runs 256-thread blocks whatever the size: the sums keep
-    // the order of the narrower block (same bits), while the factor's tiles, the cones' lists and the
-    // sparse products spread over all four sub-partitions. Not when the caller fixed the threads, and
-    // not with more instances than SMs, where the narrow blocks share an SM's FP64 units better.
     B->wide = N <= numSM && B->st.threads_per_instance == 0;
-    g.block = B->wide ? 256 : g.sumThreads;
     // per-instance scratch layout (relative to the CTA base); the FP64 root is needed when the
     // root is not in shared memory (FP64 precision) or for the mixed-precision fallback.
     const bool needRoot64 = !L.root64InSmem;
@@ -431,6 +447,7 @@ static int buildGroups(cxg_batch* B) {
     int occ = 0;
     if (gridMode) {
       // cooperative launch: every CTA resident; only CTA 0 holds an instance (and scratch)
+      g.block = 256;
       CX_CUDA(ipmGridOccupancy(&occ, g.smem, fp32));
       if (occ * numSM < 2) return setErr(CXG_E_UNSUPPORTED, "the whole-GPU root needs two resident CTAs");
       g.grid = occ * numSM;
@@ -438,11 +455,9 @@ static int buildGroups(cxg_batch* B) {
       g.scratchOff = scratchTotal;
       scratchTotal += g.stride;
     } else {
-      const cudaError_t oe = ipmOccupancy(&occ, g.block, g.smem, fp32);
-      if (oe != cudaSuccess || occ < 1) occ = 1;
-      g.grid = std::max(1, std::min(g.count, occ * numSM));
+      shapeBlock(B, g);
+      g.grid = std::max(1, std::min(g.count, g.occupancy * numSM));
       g.gridAlone = g.grid;
-      g.occupancy = occ;
       g.scratchOff = scratchTotal;
       scratchTotal += g.stride * g.grid;
     }
@@ -1071,9 +1086,9 @@ static int enqueueReorder(cxg_batch* B, cudaStream_t s) {
 }
 
 // Enqueues the device-side solve sequence on `s`: queue resets, then one persistent launch per
-// size bucket, each on its own stream forked from and joined back into `s`, so the buckets run
-// concurrently and the batch waits for its slowest instance once rather than once per bucket;
-// then the queues are re-ordered for the next solve (history-ordered queues, above).
+// size bucket, each allowed to start while those before it run, so the buckets run concurrently and
+// the batch waits for its slowest instance once rather than once per bucket; then the queues are
+// re-ordered for the next solve (history-ordered queues, above).
 static int enqueueSolve(cxg_batch* B, cudaStream_t s) {
   const DevSettings ds = makeDevSettings(B->st, B->kktSt);
   CX_CUDA(cudaMemsetAsync(B->dCounters, 0, sizeof(int) * (B->groups.size() + 1), s));
@@ -1105,26 +1120,22 @@ static int enqueueSolve(cxg_batch* B, cudaStream_t s) {
     B->lastLaunches = 1;
     return CXG_OK;
   }
-  CX_CUDA(cudaEventRecord(B->forkJoin[0], s));
-  // Launch order: by shared memory per CTA, largest first. The grids are apportioned so that all
-  // of them can be resident at once (partitionGrids); the block scheduler spreads each launch's
-  // CTAs over the SMs with room left, so the largest CTAs must be placed before the small ones
-  // scatter over every SM and leave no SM with room for a large one (first fit, decreasing).
+  // Launch order: by shared memory per CTA, largest first, each launch when every CTA of the one before
+  // is on an SM. The grids are apportioned so that all of them can be resident at once
+  // (partitionGrids); the block scheduler spreads each launch's CTAs over the SMs with room left, so
+  // the largest CTAs must be placed before the small ones scatter over every SM and leave no SM with
+  // room for a large one (first fit, decreasing). With a stream of its own for each launch, ordered by
+  // priority alone, the order was kept in most solves but not in all: some of the buckets that need a
+  // whole SM then found only two thirds of theirs free.
   std::vector<size_t> launchOrder(G);
   std::iota(launchOrder.begin(), launchOrder.end(), size_t(0));
   std::stable_sort(launchOrder.begin(), launchOrder.end(),
                    [&](size_t a_, size_t b_) { return B->groups[a_].smem > B->groups[b_].smem; });
   for (size_t rank = 0; rank < G; ++rank) {
-    const size_t gi = launchOrder[rank];
-    const Group& g = B->groups[gi];
-    cudaStream_t gs = (G == 1) ? s : B->groupStreams[rank];
-    if (G > 1) CX_CUDA(cudaStreamWaitEvent(gs, B->forkJoin[0], 0));
-    const LaunchArgs a = solveArgs(B, g, ds, B->dCounters + g.counterIdx, B->dScratch + g.scratchOff);
-    CX_CUDA(launchIpm(a, g.grid, g.block, g.smem, g.fp32, gs));
-    if (G > 1) {
-      CX_CUDA(cudaEventRecord(B->forkJoin[gi + 1], gs));
-      CX_CUDA(cudaStreamWaitEvent(s, B->forkJoin[gi + 1], 0));
-    }
+    const Group& g = B->groups[launchOrder[rank]];
+    LaunchArgs a = solveArgs(B, g, ds, B->dCounters + g.counterIdx, B->dScratch + g.scratchOff);
+    a.after = rank > 0;
+    CX_CUDA(launchIpm(a, g.grid, g.block, g.smem, g.fp32, s));
   }
   int rc = enqueueReorder(B, s);
   if (rc) return rc;
@@ -1397,11 +1408,8 @@ extern "C" int cxg_batch_autotune(cxg_batch* B, int trials, char* report, int re
     rep += line;
     for (int b : kCand) {
       if (b < 64 && g.lay.nrMax > 64) continue;  // one warp only for small roots
-      int occ = 0;
       g.sumThreads = b;
-      g.block = B->wide ? 256 : b;
-      if (ipmOccupancy(&occ, g.block, g.smem, g.fp32) != cudaSuccess || occ < 1) occ = 1;
-      g.occupancy = occ;
+      shapeBlock(B, g);
       float med = 0.0f;
       if ((rc = timeSolve(med))) break;
       std::snprintf(line, sizeof(line), " %d threads %.3f ms;", b, med);
@@ -1413,12 +1421,7 @@ extern "C" int cxg_batch_autotune(cxg_batch* B, int trials, char* report, int re
     }
     if (rc) break;
     g.sumThreads = bestBlock;
-    g.block = B->wide ? 256 : bestBlock;
-    {
-      int occ = 0;
-      if (ipmOccupancy(&occ, g.block, g.smem, g.fp32) != cudaSuccess || occ < 1) occ = 1;
-      g.occupancy = occ;
-    }
+    shapeBlock(B, g);
     std::snprintf(line, sizeof(line), " -> %d\n", bestBlock);
     rep += line;
   }

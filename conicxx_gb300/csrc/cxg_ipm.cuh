@@ -3146,6 +3146,8 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) ipmKernel(LaunchArgs 
   __shared__ int sRedi[4];
   __shared__ Ctx c;
   double* scratch = a.scratch + (int64_t)blockIdx.x * a.scratchStride;
+  // the next size bucket's launch may begin once every CTA of this one is on an SM (LaunchArgs::after)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   for (;;) {
     if (threadIdx.x == 0) sInst = atomicAdd(a.counter, 1);
     __syncthreads();
@@ -3158,6 +3160,8 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) ipmKernel(LaunchArgs 
     loadInstance(c, a);
     solveInstance<FT>(c, a, inst);
   }
+  // what follows the last bucket in the stream must find all of them finished
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Whole-GPU form for one large instance (a.grid set): a cooperative launch with one CTA per SM.
@@ -3279,8 +3283,17 @@ cudaError_t launchIpmFormT(const LaunchArgs& a, int grid, int block, size_t smem
   void (*k)(LaunchArgs) = ipmKernel<FT, kMaxThreads, kMinBlocks>;
   cudaError_t e = raiseDynSmem((const void*)k, smem);
   if (e != cudaSuccess) return e;
-  k<<<grid, block, smem, stream>>>(a);
-  return cudaGetLastError();
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = a.after ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k, a);
 }
 
 template <typename FT, int kMaxThreads, int kMinBlocks>

@@ -97,6 +97,9 @@ struct LaunchArgs {
   double* scratch;        // gridDim.x * scratchStride doubles
   int64_t scratchStride;
   int sumThreads;         // threads whose sums the block has (<= block size; FOR_V)
+  // this launch may begin while the one before it in the stream runs, once all of that one's CTAs are
+  // resident (programmatic stream serialisation): the size buckets of a batch
+  bool after = false;
   DevSettings st;
   SmemLayout lay;
   struct GridCtl* grid;   // whole-GPU form of one instance (cooperative launch), else null

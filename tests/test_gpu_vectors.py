@@ -88,3 +88,22 @@ def test_wide_blocks_give_the_narrow_blocks_bits(contacts, threads, precision):
         got.append((x, s, z, infos["iterations"], infos["refine_steps"]) + B.backward(np.ones(B.n_total)))
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [0, 1])
+def test_wide_blocks_where_a_cta_has_its_sm_alone(precision):
+    """More instances than SMs: a bucket whose shared memory leaves one CTA per SM (here 42
+    contacts, 120 KB) runs 256-thread blocks, the other bucket (10 contacts) narrow ones; both give the
+    bits of the block sizes asked for by hand."""
+    qps = [generators.contact_qp(s, contacts=42 if s % 2 else 10) for s in range(320)]
+    got = []
+    for t in (0, 128, 32):
+        B = BatchSolver(qps, precision=precision, warm_start=0, threads_per_instance=t)
+        x, s, z, infos = B.solve()
+        got.append((B.split(x, s, z), infos["iterations"]))
+    for i in range(len(qps)):
+        ref = got[1] if i % 2 else got[2]
+        assert got[0][1][i] == ref[1][i]
+        for a, b in zip(got[0][0][i], ref[0][i]):
+            assert np.array_equal(a, b), i
