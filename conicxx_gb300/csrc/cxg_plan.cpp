@@ -172,32 +172,58 @@ static int64_t pushOffsets(std::vector<int>& pool, const std::vector<int64_t>& v
   return off;
 }
 
-// A sparse matrix's rows (CSR: rowPtr, and per entry col and src) as a warp reads them, 32 rows at a
-// time: the rows are sorted by length, longest first (perm: slot -> row; rowPtr becomes the slots'),
-// and in each slice of 32 slots the entries are laid out first entries first, without padding. At
-// level k the slots with more than k entries are the first ones, so a slice's entries of one level are
+// A sparse matrix's rows (CSR: rowPtr) as a warp reads them, 32 rows at a time: the rows are sorted by
+// length, longest first (perm: slot -> row; rowPtr becomes the slots'), and in each slice of 32 slots the
+// entries are laid out first entries first, without padding; returns the entries in that order. At level k
+// the slots with more than k entries are the first ones, so a slice's entries of one level are
 // consecutive, in slot order, and a slice starts at its first slot's rowPtr.
-static void sliceRows(std::vector<int>& rowPtr, std::vector<int>& col, std::vector<int>& src, std::vector<int>& perm) {
+static std::vector<int> sliceRows(std::vector<int>& rowPtr, std::vector<int>& perm) {
   const int rows = (int)rowPtr.size() - 1;
   auto len = [&](int r) { return rowPtr[(size_t)r + 1] - rowPtr[(size_t)r]; };
+  int longest = 0;
+  for (int r = 0; r < rows; ++r) longest = std::max(longest, len(r));
+  std::vector<int> at((size_t)longest + 2, 0);  // counting sort by descending length, stable
+  for (int r = 0; r < rows; ++r) at[(size_t)(longest - len(r)) + 1]++;
+  for (int k = 0; k <= longest; ++k) at[(size_t)k + 1] += at[(size_t)k];
   perm.resize((size_t)rows);
-  std::iota(perm.begin(), perm.end(), 0);
-  std::stable_sort(perm.begin(), perm.end(), [&](int a, int b) { return len(a) > len(b); });
-  std::vector<int> p2(1, 0), c2, s2;
-  c2.reserve(col.size());
-  s2.reserve(src.size());
-  for (int t = 0; t < rows; ++t) p2.push_back(p2.back() + len(perm[(size_t)t]));
+  for (int r = 0; r < rows; ++r) perm[(size_t)at[(size_t)(longest - len(r))]++] = r;
+  std::vector<int> p2((size_t)rows + 1, 0), order((size_t)rowPtr[(size_t)rows]);
+  for (int t = 0; t < rows; ++t) p2[(size_t)t + 1] = p2[(size_t)t] + len(perm[(size_t)t]);
+  size_t out = 0;
   for (int t0 = 0; t0 < rows; t0 += 32) {
-    const int t1 = std::min(rows, t0 + 32), longest = len(perm[(size_t)t0]);
-    for (int k = 0; k < longest; ++k)
-      for (int t = t0; t < t1 && len(perm[(size_t)t]) > k; ++t) {
-        c2.push_back(col[(size_t)(rowPtr[(size_t)perm[(size_t)t]] + k)]);
-        s2.push_back(src[(size_t)(rowPtr[(size_t)perm[(size_t)t]] + k)]);
-      }
+    int base[32], active = std::min(32, rows - t0);
+    for (int i = 0; i < active; ++i) base[i] = rowPtr[(size_t)perm[(size_t)(t0 + i)]];
+    for (int k = 0;; ++k) {
+      while (active > 0 && p2[(size_t)(t0 + active)] - p2[(size_t)(t0 + active - 1)] <= k) --active;
+      if (active == 0) break;
+      for (int i = 0; i < active; ++i) order[out++] = base[i] + k;
+    }
   }
   rowPtr.swap(p2);
-  col.swap(c2);
-  src.swap(s2);
+  return order;
+}
+
+// v in the order given: v[order[0]], v[order[1]], ...
+static std::vector<int> inOrder(const std::vector<int>& v, const std::vector<int>& order) {
+  std::vector<int> w(order.size());
+  for (size_t i = 0; i < order.size(); ++i) w[i] = v[(size_t)order[i]];
+  return w;
+}
+
+// The indices 0 .. keys.size() - 1 sorted by key, stably (radix sort by 11 bits; keys are >= 0).
+static std::vector<int> sortedByKey(const std::vector<int64_t>& keys) {
+  std::vector<int> idx(keys.size()), next(keys.size());
+  std::iota(idx.begin(), idx.end(), 0);
+  int64_t top = 0;
+  for (int64_t k : keys) top = std::max(top, k);
+  for (int sh = 0; sh < 63 && (top >> sh) > 0; sh += 11) {
+    std::vector<int> at(2049, 0);
+    for (int64_t k : keys) at[(size_t)((k >> sh) & 2047) + 1]++;
+    for (int i = 0; i < 2048; ++i) at[(size_t)i + 1] += at[(size_t)i];
+    for (int i : idx) next[(size_t)at[(size_t)((keys[(size_t)i] >> sh) & 2047)]++] = i;
+    idx.swap(next);
+  }
+  return idx;
 }
 
 void planInstance(const cxg_problem& pr, const cxg_settings& st, Pools& pools) {
@@ -214,32 +240,47 @@ void planInstance(const cxg_problem& pr, const cxg_settings& st, Pools& pools) {
   std::vector<int>& I = pools.ipool;
 
   // ---- P: full symmetric CSR over the upper entries, diagonal sources, lower root scatter ----
-  std::vector<std::vector<std::pair<int, int>>> rows((size_t)n);
   std::vector<int> pdiag((size_t)n, -1), plowSrc;
   std::vector<int64_t> plowIdx;
+  std::vector<int> psRow((size_t)n + 1, 0);
   for (int c = 0; c < n; ++c)
     for (int k = pr.Pp[c]; k < pr.Pp[c + 1]; ++k) {
       const int r = pr.Pi[k];
       if (r > c) continue;  // below the diagonal: ignored, as the reference does
-      rows[(size_t)r].push_back({c, k});
-      if (r != c) {
-        rows[(size_t)c].push_back({r, k});
-        plowIdx.push_back(rootIdx(nr, c, r));
-        plowSrc.push_back(k);
-      } else if (pdiag[(size_t)c] < 0) {
-        pdiag[(size_t)c] = k;
-      }
+      psRow[(size_t)r + 1]++;
+      if (r != c) psRow[(size_t)c + 1]++;
     }
-  std::vector<int> psRow((size_t)n + 1, 0), psCol, psSrc;
-  for (int r = 0; r < n; ++r) {
-    std::sort(rows[(size_t)r].begin(), rows[(size_t)r].end());
-    for (auto& e : rows[(size_t)r]) { psCol.push_back(e.first); psSrc.push_back(e.second); }
-    psRow[(size_t)r + 1] = (int)psCol.size();
+  for (int r = 0; r < n; ++r) psRow[(size_t)r + 1] += psRow[(size_t)r];
+  D.nnzPs = psRow[(size_t)n];
+  std::vector<std::pair<int, int>> ps((size_t)D.nnzPs);  // (column, source) by rows
+  {
+    std::vector<int> fill(psRow.begin(), psRow.end() - 1);
+    for (int c = 0; c < n; ++c)
+      for (int k = pr.Pp[c]; k < pr.Pp[c + 1]; ++k) {
+        const int r = pr.Pi[k];
+        if (r > c) continue;
+        ps[(size_t)fill[(size_t)r]++] = {c, k};
+        if (r != c) {
+          ps[(size_t)fill[(size_t)c]++] = {r, k};
+          plowIdx.push_back(rootIdx(nr, c, r));
+          plowSrc.push_back(k);
+        } else if (pdiag[(size_t)c] < 0) {
+          pdiag[(size_t)c] = k;
+        }
+      }
+    for (int r = 0; r < n; ++r) {
+      const auto r0 = ps.begin() + psRow[(size_t)r], r1 = ps.begin() + psRow[(size_t)r + 1];
+      if (!std::is_sorted(r0, r1)) std::sort(r0, r1);  // rows of sorted columns come out in order
+    }
   }
-  D.nnzPs = (int)psCol.size();
   D.nPlow = (int)plowIdx.size();
   std::vector<int> psPerm;
-  sliceRows(psRow, psCol, psSrc, psPerm);
+  const std::vector<int> psOrder = sliceRows(psRow, psPerm);
+  std::vector<int> psCol((size_t)D.nnzPs), psSrc((size_t)D.nnzPs);
+  for (size_t i = 0; i < psOrder.size(); ++i) {
+    psCol[i] = ps[(size_t)psOrder[i]].first;
+    psSrc[i] = ps[(size_t)psOrder[i]].second;
+  }
   D.iPsPerm = pushInts(I, psPerm);
   D.iPp = pushInts(I, std::vector<int>(pr.Pp, pr.Pp + n + 1));
   D.iPi = pushInts(I, std::vector<int>(pr.Pi, pr.Pi + D.nnzPu));
@@ -277,17 +318,15 @@ void planInstance(const cxg_problem& pr, const cxg_settings& st, Pools& pools) {
   D.iAi = pushInts(I, ai);
   {
     // both orders of A as the products read them (sliceRows); the plain ones serve the planning below
-    std::vector<int> rp(arRow), rc(arCol), rs(arSrc), rperm, cp(ap), cc(ai), cs((size_t)D.nnzA), cperm;
-    std::iota(cs.begin(), cs.end(), 0);
-    sliceRows(rp, rc, rs, rperm);
-    sliceRows(cp, cc, cs, cperm);
+    std::vector<int> rp(arRow), rperm, cp(ap), cperm;
+    const std::vector<int> ro = sliceRows(rp, rperm), co = sliceRows(cp, cperm);
     D.iArRow = pushInts(I, rp);
-    D.iArCol = pushInts(I, rc);
-    D.iArSrc = pushInts(I, rs);
+    D.iArCol = pushInts(I, inOrder(arCol, ro));
+    D.iArSrc = pushInts(I, inOrder(arSrc, ro));
     D.iArPerm = pushInts(I, rperm);
     D.iAcRow = pushInts(I, cp);
-    D.iAcCol = pushInts(I, cc);
-    D.iAcSrc = pushInts(I, cs);
+    D.iAcCol = pushInts(I, inOrder(ai, co));
+    D.iAcSrc = pushInts(I, co);
     D.iAcPerm = pushInts(I, cperm);
   }
   D.iAZIdx = pushOffsets(I, azIdx);
@@ -304,58 +343,59 @@ void planInstance(const cxg_problem& pr, const cxg_settings& st, Pools& pools) {
   const int nUnits = l + nsoc;
   D.nUnits = nUnits;
   std::vector<int> unitAd((size_t)nUnits + 1, 0), unitSup((size_t)nUnits + 1, 0), sup, adSrc;
-  std::vector<std::pair<int64_t, int>> tgtContrib;  // (root element offset, contribution id)
-  std::vector<int> contrib;                     // 3 per contribution
+  std::vector<int64_t> target;        // per contribution: root element offset
+  std::vector<int> cA, cB, cD;        // per contribution: its two columns in the densified A, rows
+  std::vector<int> S, at;
   for (int u = 0; u < nUnits; ++u) {
     const int r0 = (u < l) ? p + u : socOff[(size_t)(u - l)];
     const int d = (u < l) ? 1 : socDim[(size_t)(u - l)];
-    std::vector<int> S;
+    S.clear();
     for (int r = r0; r < r0 + d; ++r)
       for (int k = arRow[(size_t)r]; k < arRow[(size_t)r + 1]; ++k) S.push_back(arCol[(size_t)k]);
-    std::sort(S.begin(), S.end());
+    if (!std::is_sorted(S.begin(), S.end())) std::sort(S.begin(), S.end());
     S.erase(std::unique(S.begin(), S.end()), S.end());
     const int s = (int)S.size();
     const int adBase = (int)adSrc.size();
+    // each row's columns ascend: one walk along them (the first of equal columns counts)
+    at.assign(arRow.begin() + r0, arRow.begin() + r0 + d);
     for (int pc = 0; pc < s; ++pc)
       for (int rr = 0; rr < d; ++rr) {
-        const int r = r0 + rr;
-        int src = -1;
-        for (int k = arRow[(size_t)r]; k < arRow[(size_t)r + 1]; ++k)
-          if (arCol[(size_t)k] == S[(size_t)pc]) { src = arSrc[(size_t)k]; break; }
-        adSrc.push_back(src);
+        int& k = at[(size_t)rr];
+        const int end = arRow[(size_t)(r0 + rr) + 1];
+        while (k < end && arCol[(size_t)k] < S[(size_t)pc]) ++k;
+        adSrc.push_back(k < end && arCol[(size_t)k] == S[(size_t)pc] ? arSrc[(size_t)k] : -1);
       }
     for (int pi = 0; pi < s; ++pi)
       for (int pj = 0; pj <= pi; ++pj) {
-        const int cid = (int)(contrib.size() / 3);
-        contrib.push_back(adBase + pi * d);
-        contrib.push_back(adBase + pj * d);
-        contrib.push_back(d);
-        tgtContrib.push_back({rootIdx(nr, S[(size_t)pi], S[(size_t)pj]), cid});
+        cA.push_back(adBase + pi * d);
+        cB.push_back(adBase + pj * d);
+        cD.push_back(d);
+        target.push_back(rootIdx(nr, S[(size_t)pi], S[(size_t)pj]));
       }
     sup.insert(sup.end(), S.begin(), S.end());
     unitAd[(size_t)u + 1] = (int)adSrc.size();
     unitSup[(size_t)u + 1] = (int)sup.size();
   }
-  std::stable_sort(tgtContrib.begin(), tgtContrib.end(),
-                   [](const std::pair<int64_t, int>& a, const std::pair<int64_t, int>& b) { return a.first < b.first; });
   // The targets as rows of contributions, for sliceRows: those with most contributions first, so that
   // the 32 targets a warp takes together are alike; each target's contributions keep their order.
+  const std::vector<int> byTarget = sortedByKey(target);
   std::vector<int64_t> tgtIdx, tgtAll;
-  std::vector<int> tgtBeg(1, 0), cid, unused, tperm;
-  for (size_t t = 0; t < tgtContrib.size(); ++t) {
-    if (t == 0 || tgtContrib[t].first != tgtContrib[t - 1].first) {
-      tgtAll.push_back(tgtContrib[t].first);
+  std::vector<int> tgtBeg(1, 0), tperm;
+  for (size_t t = 0; t < byTarget.size(); ++t) {
+    const int64_t at64 = target[(size_t)byTarget[t]];
+    if (t == 0 || at64 != tgtAll.back()) {
+      tgtAll.push_back(at64);
       tgtBeg.push_back(tgtBeg.back());
     }
-    cid.push_back(tgtContrib[t].second);
     tgtBeg.back()++;
   }
-  unused = cid;
-  sliceRows(tgtBeg, cid, unused, tperm);
+  const std::vector<int> cid = inOrder(byTarget, sliceRows(tgtBeg, tperm));
+  tgtIdx.reserve(tperm.size());
   for (int t : tperm) tgtIdx.push_back(tgtAll[(size_t)t]);
   std::vector<int> contribSorted;
-  for (int f = 0; f < 3; ++f)
-    for (int id : cid) contribSorted.push_back(contrib[(size_t)id * 3 + (size_t)f]);
+  contribSorted.reserve(3 * cid.size());
+  for (const std::vector<int>* f : {&cA, &cB, &cD})
+    for (int id : cid) contribSorted.push_back((*f)[(size_t)id]);
   // the columns of the SOC blocks' densified A: block and offset of each
   std::vector<int> scUnit, scOff;
   for (int b = 0; b < nsoc; ++b)
