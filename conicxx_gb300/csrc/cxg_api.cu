@@ -115,10 +115,11 @@ struct Group {
   SmemLayout lay{};
   size_t smem = 0;
   int64_t stride = 0;        // scratch doubles per CTA
+  int64_t fixedStride = 0;   // of them, what counts against the fixed scratch (solve_device_noalloc)
   int64_t scratchOff = 0;    // offset of this group's scratch in the batch scratch buffer
   int occupancy = 1;         // resident CTAs per SM of this bucket's launch shape
   int gridAlone = 1;         // persistent grid when the bucket runs alone (occupancy x SMs, capped by count)
-  double work = 0.0;         // estimated SM time per iteration: sum over its instances of nr
+  double work = 0.0;         // estimated SM time per iteration: sum over its instances of 96 + nr
   int counterIdx = 0;
 };
 
@@ -423,7 +424,7 @@ static int buildGroups(cxg_batch* B) {
     // per-instance scratch layout (relative to the CTA base); the FP64 root is needed when the
     // root is not in shared memory (FP64 precision) or for the mixed-precision fallback.
     const bool needRoot64 = !L.root64InSmem;
-    int64_t stride = 0;
+    int64_t stride = 0, fixedStride = 0;
     for (int t = s; t < e; ++t) {
       InstanceDesc& D = B->pools.desc[(size_t)idx[(size_t)t]];
       int64_t o = 0;
@@ -441,8 +442,13 @@ static int buildGroups(cxg_batch* B) {
       D.sSlice = o; o += (gridMode && fp32) ? r2((dfSliceBytes(D.nr) + 7) / 8) : 0;
       D.scratchDoubles = o;
       stride = std::max(stride, o);
+      // what the fixed scratch's limit is held against (solve_device_noalloc): without A's two copies in
+      // the products' orders and the ninth double of a second-order block's scaling
+      fixedStride = std::max(fixedStride, o - (r2(3 * (int64_t)D.nnzA) - r2(D.nnzA)) -
+                                              (L.vecInSmem ? 0 : r2(9 * (int64_t)L.nsocMax) - 8 * (int64_t)L.nsocMax));
     }
     g.stride = std::max<int64_t>(r2(stride), 2);
+    g.fixedStride = std::max<int64_t>(r2(fixedStride), 2);
     // persistent grid: resident CTAs for this configuration, capped by the group size
     int occ = 0;
     if (gridMode) {
@@ -1695,12 +1701,12 @@ extern "C" int cxg_batch_solve_device_noalloc(cxg_batch* B, double* x, double* s
   if ((int64_t)(G * sizeof(int)) > kNoallocCounterBytes) return setErr(CXG_E_INTERNAL, "too many size buckets");
   const int64_t capDoubles = (CXG_NOALLOC_SCRATCH_BYTES - kNoallocCounterBytes) / (int64_t)sizeof(double);
   for (const Group& g : B->groups)
-    if (g.stride > capDoubles) {
+    if (g.fixedStride > capDoubles) {
       char msg[256];
       std::snprintf(msg, sizeof(msg),
                     "an instance of this batch needs %lld bytes of working memory per CTA (bucket nr <= %d); "
                     "the fixed scratch holds %lld",
-                    (long long)(g.stride * 8), g.lay.nrMax, (long long)(capDoubles * 8));
+                    (long long)(g.fixedStride * 8), g.lay.nrMax, (long long)(capDoubles * 8));
       return setErr(CXG_E_UNSUPPORTED, msg);
     }
   unsigned char* arena = nullptr;
@@ -1734,12 +1740,16 @@ extern "C" int cxg_batch_solve_device_noalloc(cxg_batch* B, double* x, double* s
     a.warmZ = B->dWz;
     a.haveWarm = B->dHaveWarm;
     a.bwd = B->dBwd;
-    a.scratch = scratch;
+    // an instance within the limit whose copies of A do not fit beside the rest (a root of 33 MB) works in
+    // the batch's own scratch, which its set-up allocated
+    const bool own = g.stride > capDoubles;
+    a.scratch = own ? B->dScratch + g.scratchOff : scratch;
     a.scratchStride = g.stride;
     a.sumThreads = g.sumThreads;
     a.st = ds;
     a.lay = g.lay;
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(g.gridAlone, capDoubles / g.stride));
+    const int grid = own ? std::min(g.gridAlone, g.grid)
+                         : (int)std::max<int64_t>(1, std::min<int64_t>(g.gridAlone, capDoubles / g.stride));
     CX_CUDA(launchIpm(a, grid, g.block, g.smem, g.fp32, st));
   }
   // history-ordered queues for the next solve, as the other solve entry points keep them (the
