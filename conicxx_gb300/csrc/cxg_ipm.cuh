@@ -207,6 +207,12 @@ __device__ __noinline__ void blockSum(double (&v)[K], double* red, int vb) {
   }
 }
 
+// One of four values by the lowest two bits of k.
+__device__ __forceinline__ double pick4(int k, double a, double b, double c, double d) {
+  const double t = (k & 1) ? b : a, u = (k & 1) ? d : c;
+  return (k & 2) ? u : t;
+}
+
 __device__ __forceinline__ double blockMin(double v, double* red) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
@@ -690,12 +696,12 @@ __device__ __forceinline__ df64 shflXorT(df64 v, int m) {
   return df64(__shfl_xor_sync(0xffffffffu, v.hi, m), __shfl_xor_sync(0xffffffffu, v.lo, m));
 }
 
-// Largest split s in {1, 2, 4, 8} of a 32-term dot product such that rows * s threads fit in
+// log2 of the largest split s in {1, 2, 4, 8} of a 32-term dot product such that rows * s threads fit in
 // one pass of a block of vb threads (rows is a multiple of 32, so each warp holds whole groups of s lanes).
 __device__ __forceinline__ int dotSplit(int rows, int vb) {
-  int s = 1;
-  while (s < 8 && rows * s * 2 <= vb) s *= 2;
-  return s;
+  int ls = 0;
+  while (ls < 3 && (rows << (ls + 1)) <= vb) ++ls;
+  return ls;
 }
 
 // Sum of a dot-product partial over the s consecutive lanes of a group (s a power of two <= 8).
@@ -712,93 +718,71 @@ __device__ __forceinline__ T groupSum(T v, int s) {
 // reduction area first, so that a step takes two barriers. (Half of the warps on the chain of
 // diagonal tiles and half on the rows beyond, with one barrier, was slower by a third: the chain
 // is bound by the issue of its double-float operations, not by the barriers.)
-template <typename T>
-__device__ void denseSolve(Ctx& c, const T* M, T* y) {
-  const int Tn = rootTiles(c.nr);
-  const int nth = blockDim.x;
-  const int sd = dotSplit(32, c.vb), wd = 32 / sd;
-  const int di = (int)threadIdx.x / sd, dp = (int)threadIdx.x % sd;  // row and part in a diagonal product
+// (Split and row index are powers of two and shifts: a division by the split cost as much as a product.)
+template <typename T, bool kForward>
+__device__ __forceinline__ void denseSolvePass(Ctx& c, const T* M, T* y) {
+  const int Tn = rootTiles(c.nr), tid = threadIdx.x, nth = blockDim.x;
+  const int lsd = dotSplit(32, c.vb), wd = 32 >> lsd;
+  const int di = tid >> lsd, d0 = (tid & ((1 << lsd) - 1)) * wd;  // row and first column in a diagonal product
   T* x = reinterpret_cast<T*>(c.red);
-  // forward: y_J = Linv_JJ y_J, then y_I -= L_IJ y_J for I > J
-  for (int J = 0; J < Tn; ++J) {
+#pragma unroll 1
+  for (int q = 0; q < Tn; ++q) {
+    const int J = kForward ? q : Tn - 1 - q;
     const T* Ajj = M + tileBase(Tn, J, J);
     T* yJ = y + J * 32;
-    if ((int)threadIdx.x < 32 * sd) {
+    if (tid < (32 << lsd)) {
+      // forward: Linv_JJ y_J, backward: Linv_JJ' y_J (Linv(r, k) at r * ld + k)
+      const T* Ad = Ajj + (kForward ? di * kTileLd + d0 : d0 * kTileLd + di);
       T acc = (T)0;
 #pragma unroll 1
-      for (int c0 = dp * wd; c0 < (dp + 1) * wd; c0 += 4)
+      for (int k = 0; k < wd; k += 4) {
 #pragma unroll
-        for (int col = c0; col < c0 + 4; ++col) {
-          const T l = Ajj[di * kTileLd + col];
-          acc = accT(acc, col < di ? l : (T)0, yJ[col]);
+        for (int u = 0; u < 4; ++u) {
+          const T l = Ad[kForward ? u : u * kTileLd];
+          const int at = d0 + k + u;
+          acc = accT(acc, (kForward ? at < di : at > di) ? l : (T)0, yJ[at]);
         }
-      const T tot = groupSum(accEnd(acc), sd);
-      if (dp == 0) x[di] = yJ[di] + tot;
+        Ad += kForward ? 4 : 4 * kTileLd;
+      }
+      const T tot = groupSum(accEnd(acc), 1 << lsd);
+      if (d0 == 0) x[di] = yJ[di] + tot;
     }
     __syncthreads();
-    if (threadIdx.x < 32) yJ[threadIdx.x] = x[threadIdx.x];
-    const int rows = (Tn - J - 1) * 32;
+    if (tid < 32) yJ[tid] = x[tid];
+    const int rows = (kForward ? Tn - J - 1 : J) * 32;
     if (rows > 0) {
-      const int s = dotSplit(rows, c.vb), w = 32 / s;
+      const int ls = dotSplit(rows, c.vb), w = 32 >> ls;
 #pragma unroll 1
-      for (int t = threadIdx.x; t < rows * s; t += nth) {
-        const int row = t / s, p = t % s;
-        const int I = J + 1 + row / 32, rr = row % 32;
-        const T* Lij = M + tileBase(Tn, I, J);
+      for (int t = tid; t < rows << ls; t += nth) {
+        const int row = t >> ls, p = (t & ((1 << ls) - 1)) * w, rr = row & 31;
+        const int I = (kForward ? J + 1 : 0) + (row >> 5);
+        const T* L = kForward ? M + tileBase(Tn, I, J) + p * kTileLd + rr : M + tileBase(Tn, J, I) + rr * kTileLd + p;
         T acc = (T)0;
 #pragma unroll 1
-        for (int c0 = p * w; c0 < (p + 1) * w; c0 += 4)
+        for (int k = 0; k < w; k += 4) {
 #pragma unroll
-          for (int col = c0; col < c0 + 4; ++col) acc = accT(acc, Lij[col * kTileLd + rr], x[col]);
-        acc = groupSum(accEnd(acc), s);
+          for (int u = 0; u < 4; ++u) acc = accT(acc, L[kForward ? u * kTileLd : u], x[p + k + u]);
+          L += kForward ? 4 * kTileLd : 4;
+        }
+        acc = groupSum(accEnd(acc), 1 << ls);
         if (p == 0) y[I * 32 + rr] -= acc;
       }
     }
     __syncthreads();
   }
+}
+
+template <typename T>
+__device__ void denseSolve(Ctx& c, const T* M, T* y) {
+  const int Tn = rootTiles(c.nr);
+  denseSolvePass<T, true>(c, M, y);   // y_J = Linv_JJ y_J, then y_I -= L_IJ y_J for I > J
 #pragma unroll 1
-  for (int t = threadIdx.x; t < Tn * 32; t += nth) {
+  for (int t = threadIdx.x; t < Tn * 32; t += blockDim.x) {
     const int J = t / 32, rr = t % 32;
     y[t] /= M[tileBase(Tn, J, J) + rr * kTileLd + rr];
   }
   __syncthreads();
-  // backward: x_J = Linv_JJ^T y_J, then y_K -= L_JK^T x_J for K < J
-  for (int J = Tn - 1; J >= 0; --J) {
-    const T* Ajj = M + tileBase(Tn, J, J);
-    T* yJ = y + J * 32;
-    if ((int)threadIdx.x < 32 * sd) {
-      T acc = (T)0;
-#pragma unroll 1
-      for (int r0 = dp * wd; r0 < (dp + 1) * wd; r0 += 4)
-#pragma unroll
-        for (int row = r0; row < r0 + 4; ++row) {
-          const T l = Ajj[row * kTileLd + di];
-          acc = accT(acc, row > di ? l : (T)0, yJ[row]);
-        }
-      const T tot = groupSum(accEnd(acc), sd);
-      if (dp == 0) x[di] = yJ[di] + tot;
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) yJ[threadIdx.x] = x[threadIdx.x];
-    const int rows = J * 32;
-    if (rows > 0) {
-      const int s = dotSplit(rows, c.vb), w = 32 / s;
-#pragma unroll 1
-      for (int t = threadIdx.x; t < rows * s; t += nth) {
-        const int row = t / s, p = t % s;
-        const int K = row / 32, cc = row % 32;
-        const T* Ljk = M + tileBase(Tn, J, K);
-        T acc = (T)0;
-#pragma unroll 1
-        for (int r0 = p * w; r0 < (p + 1) * w; r0 += 4)
-#pragma unroll
-          for (int r2 = r0; r2 < r0 + 4; ++r2) acc = accT(acc, Ljk[cc * kTileLd + r2], x[r2]);
-        acc = groupSum(accEnd(acc), s);
-        if (p == 0) y[K * 32 + cc] -= acc;
-      }
-    }
-    __syncthreads();
-  }
+  denseSolvePass<T, false>(c, M, y);  // x_J = Linv_JJ^T y_J, then y_K -= L_JK^T x_J for K < J
 }
 
 // ------------------------------------------------------------------------------------------
@@ -2815,13 +2799,27 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       dbz = v[3];
       dsz = v[4];
       dxPx = v[5];
-      rtau = dqx + dbz + kappa + dxPx / tau;
-      // the scalars' products are fused into their sums as written out here and below (the root's
-      // arithmetic decides one of them), whatever the compiler finds around them
-      const double mu = fma(tau, kappa, dsz) / (double)(degree + 1);
-      const double nrx = sqrt(v[0]) / tau, nrz = sqrt(v[1]) / tau;
-      const double pobj = (0.5 * dxPx / tau + dqx) / tau;
-      const double dobj = (-0.5 * dxPx / tau - dbz) / tau;
+      // The quotients of this stage side by side in the lanes of one division each (a division holds the
+      // FP64 unit for some 600 cycles, whatever the number of lanes that want one). The scalars'
+      // products are fused into their sums as written out here and below (the root's arithmetic decides
+      // one of them), whatever the compiler finds around them.
+      const int lane = threadIdx.x & 31;
+      const double dkrA = __dmul_rn(tau, kappa);
+      double quo;
+      {
+        const double root = sqrt((lane & 7) == 3 ? v[1] : v[0]), half = 0.5 * dxPx;
+        const double num = (lane & 4) ? pick4(lane, half, tau, kappa, dkrA)
+                                      : pick4(lane, dxPx, fma(tau, kappa, dsz), root, root);
+        const double den = (lane & 4) ? pick4(lane, tau, fmax(kappa, 1e-30), tau, tau)
+                                      : pick4(lane, tau, (double)(degree + 1), tau, tau);
+        quo = num / den;
+      }
+      auto quotient = [&](int k) { return __shfl_sync(0xffffffffu, quo, k); };
+      rtau = dqx + dbz + kappa + quotient(0);
+      const double mu = quotient(1), nrx = quotient(2), nrz = quotient(3), halfTau = quotient(4);
+      const double ratio = quotient(5), kappaTau = quotient(6), dkrTau = quotient(7);
+      quo = ((lane & 1) ? -halfTau - dbz : halfTau + dqx) / tau;
+      const double pobj = quotient(0), dobj = quotient(1);
       // 4. convergence / infeasibility (solver_impl.cpp checkConvergence / checkInfeasibility)
       if (trow && threadIdx.x == 0) {
         trow[0] = mu; trow[1] = nrx; trow[2] = nrz; trow[3] = pobj; trow[4] = dobj; trow[8] = tau; trow[9] = kappa;
@@ -2829,7 +2827,6 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       const double gapAbs = fabs(pobj - dobj);
       const double gapTol = st.tol_gap_abs + st.tol_gap_rel * fmax(fabs(pobj), fabs(dobj));
       if (nrx < st.tol_feas && nrz < st.tol_feas && gapAbs < gapTol && tau > 1e-6) { status = 1; break; }
-      const double ratio = tau / fmax(kappa, 1e-30);
       if (ratio <= st.tol_infeas) {
         double w[2] = {0.0, 0.0};
         FOR_V(r, m, c.vb) w[0] += c.z[r] * c.z[r];
@@ -2851,7 +2848,7 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       }
       FOR_V(r, m, c.vb) td[1] += c.bs[r] * c.z1[r];
       blockSum<4>(td, c.red, c.vb);
-      const double tauDen = kappa / tau - td[0] - td[1] + td[2] - td[3];
+      const double tauDen = kappaTau - td[0] - td[1] + td[2] - td[3];
 
       // 5. affine step: rhs (rx, s - rz)
       FOR_T(j, n) c.rhs[j] = c.rx[j];
@@ -2867,8 +2864,7 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       }
       FOR_V(r, m, c.vb) tn3[1] += c.bs[r] * c.sol[n + r];
       blockSum<4>(tn3, c.red, c.vb);
-      const double dkrA = tau * kappa;
-      const double tauNumA = rtau - dkrA / tau + tn3[0] + tn3[1] + 2.0 * tn3[2];
+      const double tauNumA = rtau - dkrTau + tn3[0] + tn3[1] + 2.0 * tn3[2];
       if (tauDen == 0.0 || !isfinite(tauNumA) || !isfinite(tauDen)) { status = 5; break; }
       const double dtauA = tauNumA / tauDen;
       FOR_T(j, n) c.dx[j] = c.sol[j] + dtauA * c.x1[j];
@@ -2877,8 +2873,9 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       coneApply(c, kHs, 0.0, c.dz, c.tm);
       FOR_T(r, m) c.ds[r] = -(c.tm[r] + c.s[r]);
       __syncthreads();
-      const double dkappaA =
-          -(sizeof(FT) == 8 ? fma(tau, kappa, __dmul_rn(kappa, dtauA)) : fma(kappa, dtauA, dkrA)) / tau;
+      const double dkappaNum = -(sizeof(FT) == 8 ? fma(tau, kappa, __dmul_rn(kappa, dtauA)) : fma(kappa, dtauA, dkrA));
+      quo = ((lane & 1) ? -tau : dkappaNum) / ((lane & 1) ? dtauA : tau);
+      const double dkappaA = quotient(0), toTau = quotient(1);
       {
         int bad = !finiteBits(dtauA) || !finiteBits(dkappaA);
         FOR_T(j, n) bad |= !finiteBits(c.dx[j]);
@@ -2887,7 +2884,7 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       }
       // 6. affine step length (no fraction), mu_aff, sigma
       double aaff = 1.0;
-      if (dtauA < 0) aaff = fmin(aaff, -tau / dtauA);
+      if (dtauA < 0) aaff = fmin(aaff, toTau);
       if (dkappaA < 0) aaff = fmin(aaff, -kappa / dkappaA);
       aaff = coneMaxStep2(c, aaff);
       double sa[2] = {0.0, 0.0};
@@ -2938,7 +2935,8 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       coneApply(c, kHs, 0.0, c.dz, c.tm);
       FOR_T(r, m) c.ds[r] = -(c.tm[r] + c.dcon[r]);
       __syncthreads();
-      const double dkappa = -fma(kappa, dtau, dkrC) / tau;
+      quo = ((lane & 1) ? -tau : -fma(kappa, dtau, dkrC)) / ((lane & 1) ? dtau : tau);
+      const double dkappa = quotient(0), toTauC = quotient(1);
       {
         int bad = !finiteBits(dtau) || !finiteBits(dkappa);
         FOR_T(j, n) bad |= !finiteBits(c.dx[j]);
@@ -2947,7 +2945,7 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       }
       // 8. step length with the fraction-to-boundary factor
       double alpha = 1.0;
-      if (dtau < 0) alpha = fmin(alpha, -tau / dtau);
+      if (dtau < 0) alpha = fmin(alpha, toTauC);
       if (dkappa < 0) alpha = fmin(alpha, -kappa / dkappa);
       alpha = coneMaxStep2(c, alpha);
       alpha *= st.max_step_fraction;
