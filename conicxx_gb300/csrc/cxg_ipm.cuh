@@ -363,8 +363,9 @@ static __device__ __noinline__ void coneUpdateScaling(Ctx& c, const DevSettings&
   __syncthreads();
 }
 
-// out = f(W) x on every cone row (Zero rows: 0, or eps * x for kHsEps).
-static __device__ __noinline__ void coneApply(Ctx& c, int f, double eps, const double* x, double* out) {
+// out = f(W) x on every cone row (Zero rows: 0, or eps * x for kHsEps). `sync`: with a barrier at the end.
+static __device__ __noinline__ void coneApply(Ctx& c, int f, double eps, const double* x, double* out,
+                                               bool sync = true) {
   FOR_T(r, c.p) out[r] = (f == kHsEps) ? eps * x[r] : 0.0;
   FOR_T(t, c.l + c.nsoc) {  // the longer SOC units first, packed into as few warps as they fill
     if (t >= c.nsoc) {
@@ -376,7 +377,7 @@ static __device__ __noinline__ void coneApply(Ctx& c, int f, double eps, const d
       socApply(c.sp[b], c.cu + off, d, f, eps, x + off, out + off);
     }
   }
-  __syncthreads();
+  if (sync) __syncthreads();
 }
 
 // out = G x on the cone rows with the G eigenvalues prepared at factorisation (Zero rows: 0, or left as
@@ -546,20 +547,22 @@ static __device__ __noinline__ double kktResidualImpl(Ctx& c, const DevSettings&
   const double* xs = sol;
   const double* zs = sol + n;
   double acc2[2] = {0.0, 0.0};
+  // (Hs + epsA I) z, then the products, with one barrier for both: warps without cone units go ahead
+  coneApply(c, kHsEps, st.static_reg_A, zs, c.tm2, false);
   kktProducts(c, xs, zs, c.tn, c.dx, res + n);  // dx: free during a solve
-  FOR_T(t, n) {
-    // the product with the small regularisation rounded first (not fused into the sum)
-    const double acc = __dadd_rn(__dmul_rn(st.static_reg_P, xs[t]), c.tn[t]) + c.dx[t];
-    res[t] = rhs[t] - acc;
+  // the residual and its norm in one pass, each thread the elements that it sums
+  FOR_V(t, n + m, c.vb) {
+    double r;
+    if (t < n) {
+      // the product with the small regularisation rounded first (not fused into the sum)
+      r = rhs[t] - (__dadd_rn(__dmul_rn(st.static_reg_P, xs[t]), c.tn[t]) + c.dx[t]);
+    } else {
+      r = (rhs[t] - res[t]) + c.tm2[t - n];
+    }
+    res[t] = r;
+    acc2[0] += r * r;
+    if (first) acc2[1] += rhs[t] * rhs[t];
   }
-  FOR_T(r, m) res[n + r] = rhs[n + r] - res[n + r];
-  __syncthreads();
-  // + (Hs + epsA I) z on the cone rows
-  coneApply(c, kHsEps, st.static_reg_A, zs, c.tm2);
-  FOR_T(r, m) res[n + r] += c.tm2[r];
-  __syncthreads();
-  FOR_V(t, n + m, c.vb) acc2[0] += res[t] * res[t];
-  if (first) FOR_V(t, n + m, c.vb) acc2[1] += rhs[t] * rhs[t];
   // both norms and the quotient by one warp: a square root and a division hold the FP64 unit for
   // some 600 cycles each
   if (c.vb & (c.vb - 1)) {
@@ -588,11 +591,12 @@ static __device__ __noinline__ void kktApply(Ctx& c, const DevSettings& st, cons
   const int n = c.n, m = c.m;
   const double* xs = sol;
   const double* zs = sol + n;
+  coneApply(c, kHsEps, st.static_reg_A, zs, c.tm2, false);
   kktProducts(c, xs, zs, c.tn, c.dx, y + n);
-  FOR_T(t, n) y[t] = __dadd_rn(__dmul_rn(st.static_reg_P, xs[t]), c.tn[t]) + c.dx[t];
-  __syncthreads();
-  coneApply(c, kHsEps, st.static_reg_A, zs, c.tm2);
-  FOR_T(r, m) y[n + r] -= c.tm2[r];
+  FOR_T(t, n + m) {
+    if (t < n) y[t] = __dadd_rn(__dmul_rn(st.static_reg_P, xs[t]), c.tn[t]) + c.dx[t];
+    else y[t] -= c.tm2[t - n];
+  }
   __syncthreads();
 }
 
