@@ -499,31 +499,77 @@ enum {
   kProdColsF32 = 32, kProdColsDf = 64  // atz is an array of float / df64
 };
 
-// The products asked for, the slices of all of them as one list of tasks, the long rows of P first. One
-// function for every product of the iteration: each inlined copy of sliceDot was 5 to 11 KB of code.
-static __device__ __noinline__ void sliceProducts(Ctx& c, int what, const double* x, const double* z, double* px,
-                                                  void* atz, double* ax, const double* init) {
-  const int sn = slices(c.n);
+// Products to form: `what`, the vectors and where the results go.
+struct ProductJob {
+  int what;
+  const double *x, *z;
+  double* px;
+  void* atz;
+  double* ax;
+  const double* init;
+};
+
+__device__ __forceinline__ int productTasks(const Ctx& c, int what) {
+  return ((what & kProdP) ? slices(c.n) : 0) + ((what & kProdCols) ? slices(c.n) : 0) +
+         ((what & kProdRows) ? slices(c.m) : 0);
+}
+
+// The products asked for, the slices of all of them as one list of tasks, the long rows of P first: the
+// CTA's warps take them all (`first` < 0), or warp `first`'s of `count` over the grid. One function for
+// every product of the iteration: each inlined copy of sliceDot was 5 to 11 KB of code.
+static __device__ __noinline__ void sliceTasks(const Ctx& c, const ProductJob& p, int first, int count) {
+  const int what = p.what, sn = slices(c.n), end = productTasks(c, what);
   const int eP = (what & kProdP) ? sn : 0, eC = eP + ((what & kProdCols) ? sn : 0);
-  const int end = eC + ((what & kProdRows) ? slices(c.m) : 0);
   const bool add = what & kProdInit;
 #pragma unroll 1
-  for (int q, i = 0; i * (int)(blockDim.x >> 5) < end; ++i) {
-    q = snakeTask(i);
+  for (int i = 0;; ++i) {
+    const int base = i * (first < 0 ? (int)(blockDim.x >> 5) : count);
+    if (base >= end) break;
+    const int q = first < 0 ? snakeTask(i) : base + first;
     if (q >= end) continue;
     const int kind = (q >= eP) + (q >= eC);
     const Sliced& A = kind == 0 ? c.sP : kind == 1 ? c.sAc : c.sAr;
     int row;
     const double v = sliceDot(A, kind == 0 || (kind == 1 && (what & kProdColsFour)), q - (kind == 0 ? 0 : kind == 1 ? eP : eC),
-                              kind == 1 ? z : x, row, add ? init : nullptr, kind == 2, add && kind == 1 ? c.p : 0);
+                              kind == 1 ? p.z : p.x, row, add ? p.init : nullptr, kind == 2, add && kind == 1 ? c.p : 0);
     if (row < 0) continue;
-    if (kind == 0) px[row] = v;
-    else if (kind == 2) { if (!add || row >= c.p) ax[row] = v; }
-    else if (what & kProdColsF32) reinterpret_cast<float*>(atz)[row] = (float)v;
-    else if (what & kProdColsDf) reinterpret_cast<df64*>(atz)[row] = (df64)v;
-    else reinterpret_cast<double*>(atz)[row] = v;
+    if (kind == 0) p.px[row] = v;
+    else if (kind == 2) { if (!add || row >= c.p) p.ax[row] = v; }
+    else if (what & kProdColsF32) reinterpret_cast<float*>(p.atz)[row] = (float)v;
+    else if (what & kProdColsDf) reinterpret_cast<df64*>(p.atz)[row] = (df64)v;
+    else reinterpret_cast<double*>(p.atz)[row] = v;
   }
+}
+
+#ifdef CXG_GRID_KERNELS
+// Whole-GPU kernels: products of more than four tasks a warp go to the other CTAs (two grid barriers,
+// about 5 us, against 15 us and more for CTA 0 alone), which leaves CTA 0 free until productsEnd.
+static __device__ bool gridProductsPost(Ctx& c, const ProductJob& p);
+static __device__ void gridProductsWait(Ctx& c);
+__device__ __forceinline__ bool productsBegin(Ctx& c, const ProductJob& p) {
+  if (!c.grid || productTasks(c, p.what) <= 4 * (int)(blockDim.x >> 5)) return false;
+  gridProductsPost(c, p);
+  return true;
+}
+#else
+__device__ __forceinline__ bool productsBegin(Ctx&, const ProductJob&) { return false; }
+#endif
+// Ends with a barrier. `begun`: productsBegin's answer.
+__device__ __forceinline__ void productsEnd(Ctx& c, const ProductJob& p, bool begun) {
+#ifdef CXG_GRID_KERNELS
+  if (begun) {
+    gridProductsWait(c);
+    return;
+  }
+#endif
+  (void)begun;
+  sliceTasks(c, p, -1, 0);
   __syncthreads();
+}
+__device__ __forceinline__ void sliceProducts(Ctx& c, int what, const double* x, const double* z, double* px, void* atz,
+                                              double* ax, const double* init) {
+  const ProductJob p{what, x, z, px, atz, ax, init};
+  productsEnd(c, p, productsBegin(c, p));
 }
 
 // y = P_sym x (full symmetric P)
@@ -532,9 +578,8 @@ static __device__ __forceinline__ void pmul(Ctx& c, const double* x, double* y) 
 }
 
 // px = P x, atz = A'z (interleaved sums) and ax = A x
-static __device__ __forceinline__ void kktProducts(Ctx& c, const double* x, const double* z, double* px, double* atz,
-                                                   double* ax) {
-  sliceProducts(c, kProdP | kProdCols | kProdRows | kProdColsFour, x, z, px, atz, ax, nullptr);
+__device__ __forceinline__ ProductJob kktProducts(const double* x, const double* z, double* px, double* atz, double* ax) {
+  return {kProdP | kProdCols | kProdRows | kProdColsFour, x, z, px, atz, ax, nullptr};
 }
 
 // res = rhs - K sol for the statically-regularised K (the matrix refinement targets,
@@ -548,8 +593,10 @@ static __device__ __noinline__ double kktResidualImpl(Ctx& c, const DevSettings&
   const double* zs = sol + n;
   double acc2[2] = {0.0, 0.0};
   // (Hs + epsA I) z, then the products, with one barrier for both: warps without cone units go ahead
+  const ProductJob prod = kktProducts(xs, zs, c.tn, c.dx, res + n);  // dx: free during a solve
+  const bool begun = productsBegin(c, prod);
   coneApply(c, kHsEps, st.static_reg_A, zs, c.tm2, false);
-  kktProducts(c, xs, zs, c.tn, c.dx, res + n);  // dx: free during a solve
+  productsEnd(c, prod, begun);
   // the residual and its norm in one pass, each thread the elements that it sums
   FOR_V(t, n + m, c.vb) {
     double r;
@@ -591,8 +638,10 @@ static __device__ __noinline__ void kktApply(Ctx& c, const DevSettings& st, cons
   const int n = c.n, m = c.m;
   const double* xs = sol;
   const double* zs = sol + n;
+  const ProductJob prod = kktProducts(xs, zs, c.tn, c.dx, y + n);
+  const bool begun = productsBegin(c, prod);
   coneApply(c, kHsEps, st.static_reg_A, zs, c.tm2, false);
-  kktProducts(c, xs, zs, c.tn, c.dx, y + n);
+  productsEnd(c, prod, begun);
   FOR_T(t, n + m) {
     if (t < n) y[t] = __dadd_rn(__dmul_rn(st.static_reg_P, xs[t]), c.tn[t]) + c.dx[t];
     else y[t] -= c.tm2[t - n];
@@ -798,7 +847,7 @@ __device__ void denseSolve(Ctx& c, const T* M, T* y) {
 // CTA runs with it. Jobs are the same tile operations in the same order per tile as the
 // single-CTA root, spread over the warps of the grid, with a grid barrier between dependent
 // steps of the factor (two per tile column); the triangular passes hand solved tiles over by flags.
-enum { kGridOpFactor = 1, kGridOpSolve = 2, kGridOpExit = 3 };
+enum { kGridOpFactor = 1, kGridOpSolve = 2, kGridOpExit = 3, kGridOpProducts = 4 };
 
 constexpr int kGridMaxTiles = 131072 / kTile;  // of the largest whole-GPU root
 
@@ -814,6 +863,7 @@ struct GridCtl {
   double ep, ea;     // regularisation bumps of the assembly
   int64_t stageOff;  // byte offset of the tile staging area in dynamic shared memory
   unsigned long long waitNs;  // longest barrier wait; 0 = kGridWaitNs
+  ProductJob prod;   // products job
   Ctx ctx;           // CTA 0's instance context (pointers into global memory only)
   int flags[2 * kGridMaxTiles];  // job whose forward / backward pass has solved the tile
 };
@@ -875,6 +925,25 @@ static __device__ __noinline__ bool gridSync(GridCtl* g) {
   __syncthreads();
   return sOk != 0;
 }
+
+#ifdef CXG_GRID_KERNELS
+// The products job on CTAs 1 ..: the tasks go round the CTAs first, so that few of them share an SM. After
+// a failed barrier the results are not used: the next root job fails as well.
+static __device__ __forceinline__ void gridProductsShare(GridCtl* g) {
+  if (blockIdx.x > 0) {
+    const int ctas = (int)gridDim.x - 1, w = threadIdx.x >> 5;
+    sliceTasks(g->ctx, g->prod, (int)blockIdx.x - 1 + ctas * w, ctas * (int)(blockDim.x >> 5));
+  }
+}
+static __device__ bool gridProductsPost(Ctx& c, const ProductJob& p) {
+  if (threadIdx.x == 0) {
+    c.grid->op = kGridOpProducts;
+    c.grid->prod = p;
+  }
+  return gridSync(c.grid);
+}
+static __device__ void gridProductsWait(Ctx& c) { gridSync(c.grid); }
+#endif
 
 // The cone-unit contributions added to the root, slices of 32 targets (one a lane), warp w0 of nw: a
 // target's contributions in their order, A_u' (G_u A_u) as d multiply-adds each. Four contributions'
@@ -2219,6 +2288,13 @@ __device__ __noinline__ void gridWorker(GridCtl* g, const DevSettings& st) {
     volatile GridCtl* vg = g;
     const int op = vg->op, arith = vg->arith;
     if (op == kGridOpExit) return;
+#ifdef CXG_GRID_KERNELS
+    if (op == kGridOpProducts) {
+      gridProductsShare(g);
+      if (!gridSync(g)) return;
+      continue;
+    }
+#endif
     bool ok;
     if constexpr (sizeof(FT) == 4)
       ok = (arith == 1) ? gridJobT<float>(g, st, op, nullptr) : gridJobT<df64>(g, st, op, nullptr);

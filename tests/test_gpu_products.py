@@ -67,3 +67,21 @@ def test_grid_solve_at_the_edges_of_its_runs(nr, arith, tol):
     x = _probe(K, nx, b, arith, -1)[2]
     ref = np.linalg.solve(K, b)
     assert np.linalg.norm(x - ref) <= tol * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("n,zero,nonneg,soc", [(352, 2, 309, (6, 3)), (352, 2, 310, (6, 3)), (1025, 3, 40, (4, 5))])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_whole_gpu_products_agree_with_one_cta(n, zero, nonneg, soc, precision):
+    """The whole-GPU form hands products of more than 32 slices to the other CTAs: 32 and 33 slices in a
+    KKT residual, and 33 in a product with P alone, against the one-CTA form."""
+    from conicxx_gb300 import Solver
+
+    qp = ragged_qp(5, n, zero, nonneg, soc)
+    got = []
+    for whole in (-1, 1):
+        S = Solver()
+        assert S.setup(qp, precision=precision, warm_start=0, whole_gpu_root=whole)
+        sol = S.solve()
+        assert int(sol.status) == 1
+        got.append(np.asarray(sol.x))
+    assert np.linalg.norm(got[0] - got[1]) <= X_TOL * max(1.0, np.linalg.norm(got[0]))
