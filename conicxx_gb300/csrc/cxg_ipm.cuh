@@ -847,7 +847,7 @@ __device__ void denseSolve(Ctx& c, const T* M, T* y) {
 // CTA runs with it. Jobs are the same tile operations in the same order per tile as the
 // single-CTA root, spread over the warps of the grid, with a grid barrier between dependent
 // steps of the factor (two per tile column); the triangular passes hand solved tiles over by flags.
-enum { kGridOpFactor = 1, kGridOpSolve = 2, kGridOpExit = 3, kGridOpProducts = 4 };
+enum { kGridOpFactor = 1, kGridOpSolve = 2, kGridOpExit = 3, kGridOpProducts = 4, kGridOpSave = 5 };
 
 constexpr int kGridMaxTiles = 131072 / kTile;  // of the largest whole-GPU root
 
@@ -859,7 +859,7 @@ struct GridCtl {
   int arith;         // root arithmetic of the job: 0 FP64, 1 FP32, 2 double-float
   int epoch;         // number of the job (tile flags of the triangular solves)
   void* M;           // root of the job
-  void* y;           // solve vector (root arithmetic), rootTiles(nr) * 32 entries
+  void* y;           // solve vector (root arithmetic), rootTiles(nr) * 32 entries; save: FP64 copy of the root
   double ep, ea;     // regularisation bumps of the assembly
   int64_t stageOff;  // byte offset of the tile staging area in dynamic shared memory
   unsigned long long waitNs;  // longest barrier wait; 0 = kGridWaitNs
@@ -943,6 +943,34 @@ static __device__ bool gridProductsPost(Ctx& c, const ProductJob& p) {
   return gridSync(c.grid);
 }
 static __device__ void gridProductsWait(Ctx& c) { gridSync(c.grid); }
+
+// The factored root as FP64, for the adjoint: this CTA's share. CTA 0 alone took 32 ms for the 147 MB of a
+// 5940-row root, a tenth of the whole solve.
+template <typename T>
+__device__ __forceinline__ void gridSaveShare(GridCtl* g) {
+  const T* R = reinterpret_cast<const T*>(g->M);
+  double* out = reinterpret_cast<double*>(g->y);
+  const int64_t rs = rootSize(g->ctx.nr), step = (int64_t)gridDim.x * blockDim.x;
+#pragma unroll 4
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < rs; t += step) out[t] = (double)R[t];
+}
+static __device__ __forceinline__ void gridSaveJob(GridCtl* g) {
+  const int arith = g->arith;
+  if (arith == 0) gridSaveShare<double>(g);
+  else if (arith == 1) gridSaveShare<float>(g);
+  else gridSaveShare<df64>(g);
+}
+static __device__ void gridSaveRoot(Ctx& c, int arith, void* M, double* out) {
+  if (threadIdx.x == 0) {
+    c.grid->op = kGridOpSave;
+    c.grid->arith = arith;
+    c.grid->M = M;
+    c.grid->y = out;
+  }
+  if (!gridSync(c.grid)) return;
+  gridSaveJob(c.grid);
+  gridSync(c.grid);
+}
 #endif
 
 // The cone-unit contributions added to the root, slices of 32 targets (one a lane), warp w0 of nw: a
@@ -2294,6 +2322,11 @@ __device__ __noinline__ void gridWorker(GridCtl* g, const DevSettings& st) {
       if (!gridSync(g)) return;
       continue;
     }
+    if (op == kGridOpSave) {
+      gridSaveJob(g);
+      if (!gridSync(g)) return;
+      continue;
+    }
 #endif
     bool ok;
     if constexpr (sizeof(FT) == 4)
@@ -3073,6 +3106,12 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
     double* Bs = a.bwd + D.bwdOff;
     const BwdLayout bl = bwdLayout(c.nr, n, m, c.nsoc);
     const int64_t rs = rootSize(c.nr);
+#ifdef CXG_GRID_KERNELS
+    if constexpr (G) {
+      if (fs.use64) gridSaveRoot(c, ArithOf<typename HighT<FT>::type>::v, c.root64, Bs + bl.root);
+      else gridSaveRoot(c, ArithOf<FT>::v, c.root, Bs + bl.root);
+    } else
+#endif
     if (sizeof(FT) == 8) {
       const double* R = fs.use64 ? c.root64 : reinterpret_cast<const double*>(c.root);
 #pragma unroll 1
