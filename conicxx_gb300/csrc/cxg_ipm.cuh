@@ -1074,7 +1074,9 @@ __device__ __forceinline__ void copyTileAsync(T* dst, const T* src, int t, int n
 // memory; warp w takes columns 4 w .. 4 w + 3, a lane one row, with the tile routine's operations in its
 // order. Single tiles rather than 128x128 super-blocks: a super-block holds one SM's FP64 units for
 // 127 us (24 us of FP32 issue in double-float) while a root of some thousand rows has fewer
-// super-blocks than the GPU has SMs; a tile takes 9 us (2 us).
+// super-blocks than the GPU has SMs; a tile takes 9 us (2 us). FP64 factor of 1020 rows in an iteration
+// 5.4 -> 1.9 ms, of 6400 rows 111 -> 89 ms (its FP64 issue alone 72 ms); double-float of 1100 rows
+// 1.64 -> 1.31 ms.
 template <typename T>
 __device__ __noinline__ void gridTileUpdate(T* M, int Tn, int J, T* sm) {
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, c0 = 4 * (tid >> 5);
@@ -1974,7 +1976,9 @@ __device__ __noinline__ bool gridLdltSteps(GridCtl* g, int nr, int nx, const Dev
 // Roots of at least this many tile columns factor over column pairs (gridLdltPairs): half the C
 // traffic of the trailing update, but a longer serial chain per pair. Below it, one column at a
 // time (gridLdltSteps: FP32 on the tensor cores, double-float on the CUDA cores). The thresholds
-// are the measured crossovers of the two forms on GB300.
+// were the measured crossovers of the two forms on GB300. Pairs win earlier now (double-float 5.6
+// against 4.8 ms at 3072 rows, 2.8 against 3.1 ms at 2048; FP32 13.7 against 12.2 ms at 8192), but below
+// the thresholds the one-column products' smaller error stays what it was.
 constexpr int kPairMinTilesF32 = 352;  // 11264 rows
 constexpr int kPairMinTilesDf = 160;   // 5120 rows
 template <typename T>
