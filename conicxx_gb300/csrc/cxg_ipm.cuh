@@ -2990,7 +2990,9 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
       coneApply(c, kHs, 0.0, c.dz, c.tm);
       FOR_T(r, m) c.ds[r] = -(c.tm[r] + c.s[r]);
       __syncthreads();
-      const double dkappaNum = -(sizeof(FT) == 8 ? fma(tau, kappa, __dmul_rn(kappa, dtauA)) : fma(kappa, dtauA, dkrA));
+      // the batched FP64 kernel fuses the other product of the two
+      const double dkappaNum =
+          -((sizeof(FT) == 8 && !G) ? fma(tau, kappa, __dmul_rn(kappa, dtauA)) : fma(kappa, dtauA, dkrA));
       quo = ((lane & 1) ? -tau : dkappaNum) / ((lane & 1) ? dtauA : tau);
       const double dkappaA = quotient(0), toTau = quotient(1);
       {
