@@ -5,7 +5,8 @@
 //  - batched form (ipmKernel): persistent CTAs take instances from an atomic queue per size
 //    bucket; iterates in shared memory when they fit, the problem data in HBM/L2;
 //  - whole-GPU form (ipmGridKernel): one large instance, CTA 0 running the iteration on vectors in
-//    its scratch while every SM joins the root assembly, LDL' and triangular solves (gridSync).
+//    its scratch while every SM joins the root assembly, LDL', triangular solves and the larger
+//    products with P and A (gridSync).
 //
 // Precision: cone scaling, residuals, refinement residuals, step lengths and termination are
 // FP64. The dense root LDL' (see cxg_layout.h) is FP32 (MIXED) or FP64. In MIXED mode a KKT
