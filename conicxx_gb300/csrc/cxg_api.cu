@@ -166,6 +166,8 @@ struct cxg_batch {
   bool bwdDropped = false;                  // differentiable asked for, not kept (whole-GPU root > 8192 rows)
   bool bwdStale = false;                    // instances replaced since the last solve: no saved states
   void* dGridCtl = nullptr;                 // its control block
+  int gridFaultJob = 0;                     // cxg_batch_grid_fault: the job CTA 1 leaves at (0: none)
+  unsigned long long gridFaultWaitNs = 0;   // and the limit of every wait
   double* dTrace = nullptr;                 // record_timings: iteration traces (count x traceRows rows)
   int traceRows = 0;
 
@@ -1121,6 +1123,8 @@ static int enqueueSolve(cxg_batch* B, cudaStream_t s) {
   if (B->gridMode) {
     const Group& g = B->groups[0];
     CX_CUDA(cudaMemsetAsync(B->dGridCtl, 0, gridCtlBytes(), s));
+    if (B->gridFaultJob > 0)
+      CX_CUDA(setGridFault(reinterpret_cast<GridCtl*>(B->dGridCtl), B->gridFaultJob, B->gridFaultWaitNs, s));
     const LaunchArgs a = solveArgs(B, g, ds, B->dCounters, B->dScratch + g.scratchOff);
     CX_CUDA(launchIpmGrid(a, reinterpret_cast<GridCtl*>(B->dGridCtl), g.grid, g.smem, g.fp32, s));
     B->lastLaunches = 1;
@@ -1250,6 +1254,15 @@ extern "C" int cxg_batch_solve_device(cxg_batch* B, double* x, double* s, double
     CX_CUDA(cudaStreamSynchronize(st));
     return fetchInfo(B, info, 0.0);
   }
+  return CXG_OK;
+}
+
+extern "C" int cxg_batch_grid_fault(cxg_batch* B, int job, double timeout_s) {
+  if (!B) return setErr(CXG_E_INVALID, "null batch");
+  if (!B->gridMode) return setErr(CXG_E_UNSUPPORTED, "the batch does not run on the whole-GPU root");
+  if (job < 0 || (job > 0 && !(timeout_s >= 1e-3 && timeout_s <= 5.0))) return setErr(CXG_E_INVALID, "bad job or time limit");
+  B->gridFaultJob = job;
+  B->gridFaultWaitNs = (unsigned long long)(timeout_s * 1e9);
   return CXG_OK;
 }
 

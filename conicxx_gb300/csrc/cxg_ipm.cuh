@@ -863,7 +863,8 @@ struct GridCtl {
   void* y;           // solve vector (root arithmetic), rootTiles(nr) * 32 entries; save: FP64 copy of the root
   double ep, ea;     // regularisation bumps of the assembly
   int64_t stageOff;  // byte offset of the tile staging area in dynamic shared memory
-  unsigned long long waitNs;  // longest barrier wait; 0 = kGridWaitNs
+  unsigned long long waitNs;  // longest wait at a barrier or for a tile; 0 = kGridWaitNs
+  int leaveJob;      // tests: CTA 1 leaves the launch at its job of this number, undone (0: none)
   ProductJob prod;   // products job
   Ctx ctx;           // CTA 0's instance context (pointers into global memory only)
   int flags[2 * kGridMaxTiles];  // job whose forward / backward pass has solved the tile
@@ -927,9 +928,15 @@ static __device__ __noinline__ bool gridSync(GridCtl* g) {
   return sOk != 0;
 }
 
+// Whether a wait of this launch has run out (every barrier fails from then on); for a whole CTA.
+static __device__ __forceinline__ bool gridFailed(GridCtl* g) {
+  return __syncthreads_or(threadIdx.x == 0 && reinterpret_cast<volatile GridCtl*>(g)->error != 0) != 0;
+}
+
 #ifdef CXG_GRID_KERNELS
 // The products job on CTAs 1 ..: the tasks go round the CTAs first, so that few of them share an SM. After
-// a failed barrier the results are not used: the next root job fails as well.
+// a failed barrier the results are those of an earlier product: the next root job fails as well, and what
+// was judged from them until then does not count (gridFailed).
 static __device__ __forceinline__ void gridProductsShare(GridCtl* g) {
   if (blockIdx.x > 0) {
     const int ctas = (int)gridDim.x - 1, w = threadIdx.x >> 5;
@@ -945,22 +952,24 @@ static __device__ bool gridProductsPost(Ctx& c, const ProductJob& p) {
 }
 static __device__ void gridProductsWait(Ctx& c) { gridSync(c.grid); }
 
-// The factored root as FP64, for the adjoint: this CTA's share. CTA 0 alone took 32 ms for the 147 MB of a
-// 5940-row root, a tenth of the whole solve.
+// The factored root as FP64, for the adjoint: the share of CTA `cta` of `ctas`. CTA 0 alone took 32 ms for
+// the 147 MB of a 5940-row root, a tenth of the whole solve.
 template <typename T>
-__device__ __forceinline__ void gridSaveShare(GridCtl* g) {
+__device__ __forceinline__ void gridSaveShare(GridCtl* g, int cta, int ctas) {
   const T* R = reinterpret_cast<const T*>(g->M);
   double* out = reinterpret_cast<double*>(g->y);
-  const int64_t rs = rootSize(g->ctx.nr), step = (int64_t)gridDim.x * blockDim.x;
+  const int64_t rs = rootSize(g->ctx.nr), step = (int64_t)ctas * blockDim.x;
 #pragma unroll 4
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < rs; t += step) out[t] = (double)R[t];
+  for (int64_t t = (int64_t)cta * blockDim.x + threadIdx.x; t < rs; t += step) out[t] = (double)R[t];
 }
-static __device__ __forceinline__ void gridSaveJob(GridCtl* g) {
+static __device__ __forceinline__ void gridSaveJob(GridCtl* g, int cta, int ctas) {
   const int arith = g->arith;
-  if (arith == 0) gridSaveShare<double>(g);
-  else if (arith == 1) gridSaveShare<float>(g);
-  else gridSaveShare<df64>(g);
+  if (arith == 0) gridSaveShare<double>(g, cta, ctas);
+  else if (arith == 1) gridSaveShare<float>(g, cta, ctas);
+  else gridSaveShare<df64>(g, cta, ctas);
 }
+// CTA 0. Where a barrier fails (nothing follows this job that would notice), all of it by this CTA: the
+// others write the same values, if any.
 static __device__ void gridSaveRoot(Ctx& c, int arith, void* M, double* out) {
   if (threadIdx.x == 0) {
     c.grid->op = kGridOpSave;
@@ -968,9 +977,12 @@ static __device__ void gridSaveRoot(Ctx& c, int arith, void* M, double* out) {
     c.grid->M = M;
     c.grid->y = out;
   }
-  if (!gridSync(c.grid)) return;
-  gridSaveJob(c.grid);
-  gridSync(c.grid);
+  if (gridSync(c.grid)) {
+    gridSaveJob(c.grid, 0, (int)gridDim.x);
+    if (gridSync(c.grid)) return;
+  }
+  gridSaveJob(c.grid, 0, 1);
+  __syncthreads();
 }
 #endif
 
@@ -2316,11 +2328,12 @@ __device__ bool gridJobT(GridCtl* g, const DevSettings& st, int op, PivotStats* 
 // CTAs 1 .. of a whole-GPU launch: wait for a job, run it, until CTA 0 posts the exit.
 template <typename FT>
 __device__ __noinline__ void gridWorker(GridCtl* g, const DevSettings& st) {
-  for (;;) {
+  for (int job = 1;; ++job) {
     if (!gridSync(g)) return;
     volatile GridCtl* vg = g;
     const int op = vg->op, arith = vg->arith;
     if (op == kGridOpExit) return;
+    if (blockIdx.x == 1 && vg->leaveJob == job) return;
 #ifdef CXG_GRID_KERNELS
     if (op == kGridOpProducts) {
       gridProductsShare(g);
@@ -2328,7 +2341,7 @@ __device__ __noinline__ void gridWorker(GridCtl* g, const DevSettings& st) {
       continue;
     }
     if (op == kGridOpSave) {
-      gridSaveJob(g);
+      gridSaveJob(g, (int)blockIdx.x, (int)gridDim.x);
       if (!gridSync(g)) return;
       continue;
     }
@@ -3095,6 +3108,11 @@ __device__ __noinline__ void solveInstance(Ctx& c, const LaunchArgs& a, int inst
     }
   }
   if (trow && threadIdx.x == 0) trow[10] = c.sc[SC_ITREL];  // the last row, whichever way it ended
+
+  // a wait that ran out: products may be old ones, whatever was concluded from them
+  if constexpr (G) {
+    if (gridFailed(c.grid)) status = 5;
+  }
 
   // finalizeSolution (solver_impl.cpp:342-365 of the reference numbering)
   const bool infeas = (status == 2 || status == 3);

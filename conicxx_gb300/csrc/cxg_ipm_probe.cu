@@ -233,6 +233,16 @@ cudaError_t launchGridBarrierTest(int skip, int rounds, double timeoutS, int* er
   return e;
 }
 
+__global__ void gridFaultKernel(GridCtl* g, int job, unsigned long long waitNs) {
+  g->leaveJob = job;
+  g->waitNs = waitNs;
+}
+
+cudaError_t setGridFault(GridCtl* ctl, int job, unsigned long long waitNs, cudaStream_t stream) {
+  gridFaultKernel<<<1, 1, 0, stream>>>(ctl, job, waitNs);
+  return cudaGetLastError();
+}
+
 size_t denseProbeSmem(int arith, int nr) {
   const size_t elem = (arith == 1) ? 4 : 8;
   return (size_t)(rootSize(nr) + (int64_t)rootTiles(nr) * kTile) * elem;

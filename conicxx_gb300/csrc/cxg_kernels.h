@@ -111,6 +111,9 @@ cudaError_t launchIpm(const LaunchArgs& a, int grid, int block, size_t smem, boo
 size_t gridCtlBytes();
 cudaError_t launchIpmGrid(const LaunchArgs& a, GridCtl* ctl, int grid, size_t smem, bool fp32, cudaStream_t stream);
 cudaError_t ipmGridOccupancy(int* blocksPerSM, size_t smem, bool fp32);
+// Tests: in the launch after it on `stream`, CTA 1 leaves at its job number `job` and every wait ends
+// after waitNs.
+cudaError_t setGridFault(GridCtl* ctl, int job, unsigned long long waitNs, cudaStream_t stream);
 // One adjoint solve per instance with the saved final factorisation (same launch shape as the
 // forward groups).
 cudaError_t launchAdjoint(const LaunchArgs& a, int grid, int block, size_t smem, cudaStream_t stream);

@@ -330,6 +330,12 @@ int cxg_dense_ldlt(int nr, int nx, const double* K, const double* b, int arith, 
  * out), max_rounds_passed (most barriers any CTA got through), elapsed_s (launch time). */
 int cxg_grid_barrier_selftest(int skip_cta, int rounds, double timeout_s, int* error_flag, int* max_rounds_passed,
                               double* elapsed_s);
+/* Diagnostic, no reference counterpart: from now on, in every solve of a whole-GPU instance, one of the
+ * other CTAs leaves the launch at its job number `job` (1 ..; a factorisation, a triangular solve, a
+ * product or the copy of the root for backward), that job undone, and every wait ends after timeout_s
+ * (1e-3..5 s). The solve then ends with NumericalError, unless the job left out is the copy for backward
+ * (made by the first CTA then) or no such job comes. job = 0 ends this. */
+int cxg_batch_grid_fault(cxg_batch* batch, int job, double timeout_s);
 /* Host equilibration of the set-up path (Equilibration::compute, src/conicxx/kkt/equilibration.cpp:8-100):
  * d (n), e (m), c. No GPU needed. */
 int cxg_equilibration(const cxg_problem* problem, const cxg_settings* settings, double* d, double* e, double* c);
