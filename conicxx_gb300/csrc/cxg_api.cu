@@ -1420,28 +1420,44 @@ extern "C" int cxg_batch_autotune(cxg_batch* B, int trials, char* report, int re
   for (size_t gi = 0; gi < B->groups.size() && rc == CXG_OK; ++gi) {
     Group& g = B->groups[gi];
     const int start = g.sumThreads;
-    int bestBlock = start;
+    int best = start;
     float bestMs = 0.0f;
     char line[256];
     std::snprintf(line, sizeof(line), "bucket nr<=%d (%d instances):", g.lay.nrMax, g.count);
     rep += line;
-    for (int b : kCand) {
-      if (b < 64 && g.lay.nrMax > 64) continue;  // one warp only for small roots
-      g.sumThreads = b;
+    // the block sizes that the candidates come to, the present one first. A candidate that comes to one of
+    // them again (a CTA with its SM alone runs 256 threads whatever is asked for, shapeBlock) would differ
+    // from it in the order of its sums alone, and be chosen by the noise of its timing.
+    std::vector<int> cand(1, start), blocks;
+    for (int b : kCand)
+      if (b != start && !(b < 64 && g.lay.nrMax > 64)) cand.push_back(b);  // one warp only for small roots
+    for (size_t i = 0; i < cand.size();) {
+      g.sumThreads = cand[i];
+      shapeBlock(B, g);
+      if (std::find(blocks.begin(), blocks.end(), g.block) != blocks.end()) {
+        cand.erase(cand.begin() + (std::ptrdiff_t)i);
+      } else {
+        blocks.push_back(g.block);
+        ++i;
+      }
+    }
+    for (size_t i = 0; i < cand.size() && cand.size() > 1; ++i) {
+      g.sumThreads = cand[i];
       shapeBlock(B, g);
       float med = 0.0f;
       if ((rc = timeSolve(med))) break;
-      std::snprintf(line, sizeof(line), " %d threads %.3f ms;", b, med);
+      std::snprintf(line, sizeof(line), " %d threads %.3f ms;", g.block, med);
       rep += line;
       if (bestMs == 0.0f || med < bestMs) {
         bestMs = med;
-        bestBlock = b;
+        best = cand[i];
       }
     }
     if (rc) break;
-    g.sumThreads = bestBlock;
+    g.sumThreads = best;
     shapeBlock(B, g);
-    std::snprintf(line, sizeof(line), " -> %d\n", bestBlock);
+    if (cand.size() == 1) rep += " one shape";
+    std::snprintf(line, sizeof(line), " -> %d threads\n", g.block);
     rep += line;
   }
   cudaEventDestroy(e0);

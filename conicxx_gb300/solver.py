@@ -282,8 +282,8 @@ class BatchSolver:
               "cxg_batch_update_values_device")
 
     def autotune(self, trials=3):
-        """Pick threads per instance for every size bucket by timing each bucket's launch alone
-        (cxg_batch_autotune); returns the per-bucket report."""
+        """Pick the size buckets' edges and the threads per instance of every bucket whose instances share
+        SMs, by timing whole solves (cxg_batch_autotune); returns the report."""
         buf = C.create_string_buffer(8192)
         check(lib().cxg_batch_autotune(self._h, int(trials), buf, len(buf)), "cxg_batch_autotune")
         return buf.value.decode()

@@ -275,7 +275,8 @@ int cxg_batch_solve_device_noalloc(cxg_batch* batch, double* x, double* s, doubl
  * timed solves after one warm-up each, median kept): (1) the size-bucket edges on the root size,
  * from five candidate sets (finer and coarser than the built-in one), each planned with its SM
  * shares and working memory; (2) then, one bucket at a time, 32 (roots of at most 64 rows), 64,
- * 128 or 256 threads per instance. The fastest choices are kept for later solves. The trials
+ * 128 or 256 threads per instance, where several instances share an SM (an instance with an SM of
+ * its own runs on 256 threads, and nothing is tried). The fastest choices are kept for later solves. The trials
  * solve the current values with warm start off and overwrite the last solution (solve again to
  * read one). Allocates device memory. report (may be NULL) receives one line per edge set and
  * one line per bucket with the measured times. */
