@@ -445,9 +445,8 @@ static int buildGroups(cxg_batch* B) {
       D.scratchDoubles = o;
       stride = std::max(stride, o);
       // what the fixed scratch's limit is held against (solve_device_noalloc): without A's two copies in
-      // the products' orders and the ninth double of a second-order block's scaling
-      fixedStride = std::max(fixedStride, o - (r2(3 * (int64_t)D.nnzA) - r2(D.nnzA)) -
-                                              (L.vecInSmem ? 0 : r2(9 * (int64_t)L.nsocMax) - 8 * (int64_t)L.nsocMax));
+      // the products' orders
+      fixedStride = std::max(fixedStride, o - (r2(3 * (int64_t)D.nnzA) - r2(D.nnzA)));
     }
     g.stride = std::max<int64_t>(r2(stride), 2);
     g.fixedStride = std::max<int64_t>(r2(fixedStride), 2);

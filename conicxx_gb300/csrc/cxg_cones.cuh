@@ -73,17 +73,19 @@ constexpr double kWMax = 1e8;                      // second_order_cone.cpp:152
 // reference dense form below
 constexpr double kHsRes = 2.220446049250313e-16;
 
-// Per-SOC-block scaling parameters (9 doubles in shared memory): kind (0 identity fallback, 1
-// diagonal, 2 plane, 3 plane with the small eigenvalue of Hs held at the dense form's resolution,
-// hsSmall), beta, lam = lambda (plane) or a = 2v0^2-1 (diagonal), w2 = beta / lambda (plane), the
-// small in-plane eigenvalue of W, kept since a division costs as much as nine multiply-adds and
-// every application needs it, qc, qs (in-plane eigenvector of lambda), and the three eigenvalues of
-// G = (Hs + eps I)^-1 prepared at factorisation time (socPrepareG).
-// The unit vector u is kept in a row-indexed array at rows off+1 .. off+dim-1.
+// Per-SOC-block scaling parameters (8 doubles in shared memory): beta, lam = lambda (plane) or
+// a = 2v0^2-1 (diagonal), w2 = beta / lambda (plane), the small in-plane eigenvalue of W, kept since a
+// division costs as much as nine multiply-adds and every application needs it, qc, qs (in-plane
+// eigenvector of lambda), and the three eigenvalues of G = (Hs + eps I)^-1 prepared at factorisation
+// time (socPrepareG). The unit vector u is kept in a row-indexed array at rows off+1 .. off+dim-1,
+// whose row off holds the block's kind (socKind): 0 identity fallback, 1 diagonal, 2 plane, 3 plane
+// with the small eigenvalue of Hs held at the dense form's resolution (hsSmall). A ninth double for
+// the kind would move the sizes at which the vectors and the root fit in shared memory.
 struct SocScale {
-  long long kind;
   double beta, lam, w2, qc, qs, r0, r1, r2;
 };
+__device__ __forceinline__ int socKind(const double* u) { return __double2loint(u[0]); }
+__device__ __forceinline__ void setSocKind(double* u, int kind) { u[0] = __hiloint2double(0, kind); }
 static_assert(sizeof(SocScale) == 8 * kSocScaleDoubles, "SocScale is kept in arrays of doubles");
 
 // Computes the NT scaling of one SOC block from (s, z) (second_order_cone.cpp:70-159): the same
@@ -133,7 +135,7 @@ __device__ __forceinline__ void socUpdateScalingDim(const double* s, const doubl
   wmax *= beta;
   // Hs = W W has entries up to ~dim * wmax^2: finite whenever W is finite and wmax <= 1e8.
   if (!finite || nanBits(wmax) || lessBits(kWMax, wmax)) {
-    sc.kind = 0;
+    setSocKind(u, 0);
     sc.beta = 1.0;
     sc.lam = 1.0;
     sc.w2 = 1.0;
@@ -144,7 +146,7 @@ __device__ __forceinline__ void socUpdateScalingDim(const double* s, const doubl
   const double n1 = sqrt(n1sq);
   sc.beta = beta;
   if (zeroBits(n1) || d == 1) {
-    sc.kind = 1;
+    setSocKind(u, 1);
     sc.lam = 2.0 * v0 * v0 - 1.0;
     sc.w2 = beta;
     sc.qc = 1.0;
@@ -162,7 +164,7 @@ __device__ __forceinline__ void socUpdateScalingDim(const double* s, const doubl
   double qa, qb;
   if (!lessBits(A, E)) { qa = l1 - E; qb = C; } else { qa = C; qb = l1 - A; }
   const double qn = hypot(qa, qb);
-  sc.kind = 2;
+  setSocKind(u, 2);
   sc.lam = l1;
   sc.w2 = beta / l1;
   sc.qc = qa / qn;
@@ -221,7 +223,7 @@ template <int DIM>
 __device__ __forceinline__ void socApplyDim(const SocScale& sc, const double* u, int dim, int f, double eps,
                                             const double* x, double* y) {
   const int d = DIM ? DIM : dim;
-  const int kind = (int)sc.kind;
+  const int kind = socKind(u);
   if (kind == 0) {
     const double g = wfun(f, 1.0, eps);
     for (int i = 0; i < d; ++i) y[i] = g * x[i];
@@ -257,8 +259,8 @@ __device__ __forceinline__ void socApply(const SocScale& sc, const double* u, in
 }
 
 // G = (Hs + eps I)^-1 of one SOC block as its three eigenvalues (stored in sc.r0..r2).
-__device__ __forceinline__ void socPrepareG(SocScale& sc, double eps) {
-  const int kind = (int)sc.kind;
+__device__ __forceinline__ void socPrepareG(SocScale& sc, const double* u, double eps) {
+  const int kind = socKind(u);
   if (kind == 0) {
     const double g = 1.0 / (1.0 + eps);
     sc.r0 = sc.r1 = sc.r2 = g;
@@ -278,7 +280,7 @@ __device__ __forceinline__ void socPrepareG(SocScale& sc, double eps) {
 template <int DIM>
 __device__ __forceinline__ void socApplyGDim(const SocScale& sc, const double* u, int dim, const double* x, double* y) {
   const int d = DIM ? DIM : dim;
-  const int kind = (int)sc.kind;
+  const int kind = socKind(u);
   if (kind == 0) {
     for (int i = 0; i < d; ++i) y[i] = sc.r0 * x[i];
     return;

@@ -87,7 +87,7 @@ __global__ void coneEvalKernel(int op, int zero, int nn, int nsoc, const int* of
   }
   if (params) {
     for (int b = threadIdx.x; b < nsoc; b += blockDim.x) {
-      params[8 * b + 0] = (double)sp[b].kind;
+      params[8 * b + 0] = (double)socKind(cu + off[b]);
       params[8 * b + 1] = sp[b].beta;
       params[8 * b + 2] = sp[b].lam;
       params[8 * b + 3] = sp[b].qc;

@@ -355,7 +355,7 @@ static __device__ __noinline__ void coneUpdateScaling(Ctx& c, const DevSettings&
   // once a block's dense form has lost its small eigenvalue (the reference's pivot test fails),
   // the instance's blocks take Hs at the dense form's resolution, from this iteration on (sticky)
   const bool floorHs = c.sc[SC_HSFLOOR] != 0.0 || mx > 0;
-  if (floorHs) FOR_T(b, c.nsoc) if (c.sp[b].kind == 2) c.sp[b].kind = 3;
+  if (floorHs) FOR_T(b, c.nsoc) if (socKind(c.cu + c.socOff[b]) == 2) setSocKind(c.cu + c.socOff[b], 3);
   __syncthreads();
   if (threadIdx.x == 0) {
     c.sc[SC_SOCLVL] = (double)mx;
@@ -2394,7 +2394,7 @@ __device__ __noinline__ void assembleFactor(Ctx& c, const DevSettings& st, T* M,
       c.cu[c.p + i] = g;
       for (int k = c.unitAd[i]; k < c.unitAd[i + 1]; ++k) c.T[k] = g * c.Ad[k];
     } else {
-      socPrepareG(c.sp[u], epsA);
+      socPrepareG(c.sp[u], c.cu + c.socOff[u], epsA);
     }
   }
   __syncthreads();

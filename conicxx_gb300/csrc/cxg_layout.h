@@ -99,7 +99,7 @@ struct InstanceDesc {
 };
 
 // Doubles of one SOC block's scaling parameters (SocScale).
-constexpr int kSocScaleDoubles = 9;
+constexpr int kSocScaleDoubles = 8;
 
 // Saved final state of one instance for the adjoint (differentiable batches), in doubles:
 // FP64 root factor, NN/SOC scaling (w, G eigenvalues / u, SOC parameters), normalised iterate
