@@ -115,7 +115,7 @@ struct Group {
   SmemLayout lay{};
   size_t smem = 0;
   int64_t stride = 0;        // scratch doubles per CTA
-  int64_t fixedStride = 0;   // of them, what counts against the fixed scratch (solve_device_noalloc)
+  int64_t fixedStride = 0;   // the same without A's copies in slice order (noallocShape)
   int64_t scratchOff = 0;    // offset of this group's scratch in the batch scratch buffer
   int occupancy = 1;         // resident CTAs per SM of this bucket's launch shape
   int gridAlone = 1;         // persistent grid when the bucket runs alone (occupancy x SMs, capped by count)
@@ -431,7 +431,7 @@ static int buildGroups(cxg_batch* B) {
       InstanceDesc& D = B->pools.desc[(size_t)idx[(size_t)t]];
       int64_t o = 0;
       D.sPv = o; o += r2((int64_t)D.nnzPu + D.nnzPs);
-      D.sAv = o; o += r2(3 * (int64_t)D.nnzA);
+      D.sAv = o; o += r2(D.nnzA);
       D.sAd = o; o += r2(D.nAd);
       D.sT = o; o += r2(D.nAd);
       D.sQ = o; o += r2(D.n);
@@ -442,11 +442,10 @@ static int buildGroups(cxg_batch* B) {
       D.sKry = o; o += gridMode ? krylovDoubles(L.nMax, L.mMax) : 0;
       o = r2(o);  // 16-byte aligned: the slices are read by bulk copies
       D.sSlice = o; o += (gridMode && fp32) ? r2((dfSliceBytes(D.nr) + 7) / 8) : 0;
+      fixedStride = std::max(fixedStride, o);
+      D.sAc = o; o += r2(2 * (int64_t)D.nnzA);
       D.scratchDoubles = o;
       stride = std::max(stride, o);
-      // what the fixed scratch's limit is held against (solve_device_noalloc): without A's two copies in
-      // the products' orders
-      fixedStride = std::max(fixedStride, o - (r2(3 * (int64_t)D.nnzA) - r2(D.nnzA)));
     }
     g.stride = std::max<int64_t>(r2(stride), 2);
     g.fixedStride = std::max<int64_t>(r2(fixedStride), 2);
@@ -1283,16 +1282,42 @@ extern "C" int cxg_batch_footprint(const cxg_batch* B, int64_t* plan, int64_t* v
   return CXG_OK;
 }
 
+// How the allocation-free solve runs a bucket in its fixed array: CTAs, doubles of each one's working
+// memory, and whether they do without A's copies in slice order (2 nnz(A) doubles, up to two thirds of
+// the working memory; reading A through its source indices takes 2% longer). The copies are left out
+// where the array holds no CTA with them, or where a CTA would take more instances one after another
+// (58 instances of 200 variables in FP64 on 58 CTAs 21.3 ms, with the copies on 55 CTAs 32.2 ms; 96 with
+// a dense 400 x 60 A on 57 CTAs 86.4 ms, on 34 CTAs 105.2 ms).
+struct NoallocShape {
+  int grid;
+  int64_t stride;
+  bool gather;
+};
+static constexpr int64_t kNoallocCounterBytes = 256;
+static constexpr int64_t kNoallocDoubles = (CXG_NOALLOC_SCRATCH_BYTES - kNoallocCounterBytes) / (int64_t)sizeof(double);
+static NoallocShape noallocShape(const Group& g) {
+  auto ctas = [&](int64_t stride) { return std::min<int64_t>(g.gridAlone, kNoallocDoubles / stride); };
+  auto rounds = [&](int64_t n) { return (g.count + n - 1) / n; };
+  const int64_t with = ctas(g.stride), without = std::max<int64_t>(ctas(g.fixedStride), 1);
+  NoallocShape s{};
+  s.gather = with < 1 || rounds(without) < rounds(with);
+  s.stride = s.gather ? g.fixedStride : g.stride;
+  s.grid = (int)(s.gather ? without : with);
+  return s;
+}
+
 extern "C" int cxg_batch_describe(const cxg_batch* B, char* buf, int buflen) {
   if (!B || !buf || buflen <= 0) return setErr(CXG_E_INVALID, "bad arguments");
   std::string out;
   for (const Group& g : B->groups) {
     char line[512];
+    const NoallocShape na = noallocShape(g);
     std::snprintf(line, sizeof(line),
                   "group instances=%d nrMax=%d nMax=%d mMax=%d %s block=%d grid=%d smem=%zu vecInSmem=%d "
-                  "rootInSmem=%d root64InSmem=%d scratchPerCTA=%lld wholeGPU=%d\n",
+                  "rootInSmem=%d root64InSmem=%d scratchPerCTA=%lld wholeGPU=%d noallocGrid=%d noallocPerCTA=%lld\n",
                   g.count, g.lay.nrMax, g.lay.nMax, g.lay.mMax, g.fp32 ? "mixed" : "fp64", g.block, g.grid, g.smem,
-                  g.lay.vecInSmem, g.lay.rootInSmem, g.lay.root64InSmem, (long long)g.stride, B->gridMode ? 1 : 0);
+                  g.lay.vecInSmem, g.lay.rootInSmem, g.lay.root64InSmem, (long long)g.stride, B->gridMode ? 1 : 0,
+                  B->gridMode ? 0 : na.grid, (long long)na.stride);
     out += line;
   }
   std::snprintf(buf, (size_t)buflen, "%s", out.c_str());
@@ -1696,7 +1721,6 @@ extern "C" int cxg_batch_backward_device(cxg_batch* B, const double* dL_dx, doub
 // These must be zero when a launch starts, so every call clears them on its stream. The rest is
 // the per-CTA FP64 scratch. The kernel writes scratch before it reads it, so no clearing is needed.
 static __device__ __align__(256) unsigned char g_noallocArena[CXG_NOALLOC_SCRATCH_BYTES];
-constexpr int64_t kNoallocCounterBytes = 256;
 constexpr int kNoallocMaxDevices = 64;
 static unsigned char* g_noallocPtr[kNoallocMaxDevices];
 static std::mutex g_noallocMutex;
@@ -1727,14 +1751,13 @@ extern "C" int cxg_batch_solve_device_noalloc(cxg_batch* B, double* x, double* s
   if (dev != B->device) return setErr(CXG_E_INVALID, "the batch lives on another device: make that device current");
   const size_t G = B->groups.size();
   if ((int64_t)(G * sizeof(int)) > kNoallocCounterBytes) return setErr(CXG_E_INTERNAL, "too many size buckets");
-  const int64_t capDoubles = (CXG_NOALLOC_SCRATCH_BYTES - kNoallocCounterBytes) / (int64_t)sizeof(double);
   for (const Group& g : B->groups)
-    if (g.fixedStride > capDoubles) {
+    if (g.fixedStride > kNoallocDoubles) {
       char msg[256];
       std::snprintf(msg, sizeof(msg),
                     "an instance of this batch needs %lld bytes of working memory per CTA (bucket nr <= %d); "
                     "the fixed scratch holds %lld",
-                    (long long)(g.fixedStride * 8), g.lay.nrMax, (long long)(capDoubles * 8));
+                    (long long)(g.fixedStride * 8), g.lay.nrMax, (long long)(kNoallocDoubles * 8));
       return setErr(CXG_E_UNSUPPORTED, msg);
     }
   unsigned char* arena = nullptr;
@@ -1768,17 +1791,14 @@ extern "C" int cxg_batch_solve_device_noalloc(cxg_batch* B, double* x, double* s
     a.warmZ = B->dWz;
     a.haveWarm = B->dHaveWarm;
     a.bwd = B->dBwd;
-    // an instance within the limit whose copies of A do not fit beside the rest (a root of 33 MB) works in
-    // the batch's own scratch, which its set-up allocated
-    const bool own = g.stride > capDoubles;
-    a.scratch = own ? B->dScratch + g.scratchOff : scratch;
-    a.scratchStride = g.stride;
+    const NoallocShape na = noallocShape(g);
+    a.scratch = scratch;
+    a.scratchStride = na.stride;
+    a.gatherA = na.gather ? 1 : 0;
     a.sumThreads = g.sumThreads;
     a.st = ds;
     a.lay = g.lay;
-    const int grid = own ? std::min(g.gridAlone, g.grid)
-                         : (int)std::max<int64_t>(1, std::min<int64_t>(g.gridAlone, capDoubles / g.stride));
-    CX_CUDA(launchIpm(a, grid, g.block, g.smem, g.fp32, st));
+    CX_CUDA(launchIpm(a, na.grid, g.block, g.smem, g.fp32, st));
   }
   // history-ordered queues for the next solve, as the other solve entry points keep them (the
   // re-ordering kernel uses static shared memory and the batch's own queue array only)

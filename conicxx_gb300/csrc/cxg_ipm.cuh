@@ -48,6 +48,7 @@ struct Sliced {
   const double* val;
   const int *col, *ptr, *perm;  // per entry; slot ptr; slot -> row
   int rows;
+  const int* src;               // kGather: the entries' places in val, or null (val is in slice order)
 };
 
 // Products of the 32 rows of slice `sl` with x, one row a lane (a whole warp calls it); row receives
@@ -61,10 +62,13 @@ struct Sliced {
 // thread in plain CSR order a 189-row P of 9 100 entries took 19 000 cycles, now 11 400; the same order
 // with the loads under their conditions 29 000. One FP64 instruction (64 cycles) per entry of a slice's
 // longest row is 7 000. Inlined: a function would save and restore its registers through L1.
+// kGather: values through their source index, for working memory without A's copies in slice order
+// (LaunchArgs::gatherA); a form of its own, since the second dependent load costs the other one time.
+template <bool kGather>
 __device__ __forceinline__ double sliceDot(const Sliced& A, bool kFour, int sl, const double* x, int& row,
                                            const double* init = nullptr, bool negInit = false, int cmin = 0) {
   const int lane = threadIdx.x & 31, slot = 32 * sl + lane, rows = A.rows;
-  const int *ptr = A.ptr, *col = A.col;
+  const int *ptr = A.ptr, *col = A.col, *src = kGather ? A.src : nullptr;
   const double* val = A.val;
   const bool real = slot < rows;
   const int b0 = ptr[min(slot, rows)], b1 = ptr[min(slot + 1, rows)], r0 = A.perm[min(slot, rows - 1)];
@@ -86,7 +90,7 @@ __device__ __forceinline__ double sliceDot(const Sliced& A, bool kFour, int sl, 
     for (int u = 0; u < 8; ++u) {
       const bool on = k + u < len;
       const int at = on ? base : start;
-      v[u] = val[at];
+      v[u] = val[kGather && src ? src[at] : at];
       ci[u] = col[at];
       base += __popc(__ballot_sync(0xffffffffu, on));
     }
@@ -245,6 +249,7 @@ struct GridCtl;
 struct Ctx {
   int n, m, p, l, nsoc, nr, nUnits;
   int vb;  // threads of the block whose sums the instance has (FOR_V)
+  bool gather;  // no copies of A in slice order: values through their source index (LaunchArgs::gatherA)
   const InstanceDesc* D;
   const int *pdiag, *plowSrc, *ap, *ai, *arSrc;
   const int *azSrc, *socOff, *socDim, *unitAd, *unitSup, *tgtBeg, *contrib, *scUnit, *scOff;
@@ -306,10 +311,11 @@ static __device__ __noinline__ void loadInstance(Ctx& c, const LaunchArgs& a) {
   FOR_T(b2, c.nsoc) c.ev[c.socOff[b2]] = 1.0;
   FOR_T(k, D.nnzPs) c.Pv[k] = c.Pu[psSrc[k]];
   const int* acSrc = a.ipool + D.iAcSrc;
-  FOR_T(k, D.nnzA) {
-    c.Avc[k] = c.Av[acSrc[k]];
-    c.Avr[k] = c.Av[c.arSrc[k]];
-  }
+  if (!c.gather)
+    FOR_T(k, D.nnzA) {
+      c.Avc[k] = c.Av[acSrc[k]];
+      c.Avr[k] = c.Av[c.arSrc[k]];
+    }
   const int* adSrc = a.ipool + D.iAdSrc;
   FOR_T(k, D.nAd) {
     const int src = adSrc[k];
@@ -518,6 +524,7 @@ __device__ __forceinline__ int productTasks(const Ctx& c, int what) {
 // The products asked for, the slices of all of them as one list of tasks, the long rows of P first: the
 // CTA's warps take them all (`first` < 0), or warp `first`'s of `count` over the grid. One function for
 // every product of the iteration: each inlined copy of sliceDot was 5 to 11 KB of code.
+template <bool kGather>
 static __device__ __noinline__ void sliceTasks(const Ctx& c, const ProductJob& p, int first, int count) {
   const int what = p.what, sn = slices(c.n), end = productTasks(c, what);
   const int eP = (what & kProdP) ? sn : 0, eC = eP + ((what & kProdCols) ? sn : 0);
@@ -531,8 +538,9 @@ static __device__ __noinline__ void sliceTasks(const Ctx& c, const ProductJob& p
     const int kind = (q >= eP) + (q >= eC);
     const Sliced& A = kind == 0 ? c.sP : kind == 1 ? c.sAc : c.sAr;
     int row;
-    const double v = sliceDot(A, kind == 0 || (kind == 1 && (what & kProdColsFour)), q - (kind == 0 ? 0 : kind == 1 ? eP : eC),
-                              kind == 1 ? p.z : p.x, row, add ? p.init : nullptr, kind == 2, add && kind == 1 ? c.p : 0);
+    const double v = sliceDot<kGather>(A, kind == 0 || (kind == 1 && (what & kProdColsFour)), q - (kind == 0 ? 0 : kind == 1 ? eP : eC),
+                                       kind == 1 ? p.z : p.x, row, add ? p.init : nullptr, kind == 2,
+                                       add && kind == 1 ? c.p : 0);
     if (row < 0) continue;
     if (kind == 0) p.px[row] = v;
     else if (kind == 2) { if (!add || row >= c.p) p.ax[row] = v; }
@@ -562,9 +570,12 @@ __device__ __forceinline__ void productsEnd(Ctx& c, const ProductJob& p, bool be
     gridProductsWait(c);
     return;
   }
-#endif
+  sliceTasks<false>(c, p, -1, 0);
+#else
   (void)begun;
-  sliceTasks(c, p, -1, 0);
+  if (c.gather) sliceTasks<true>(c, p, -1, 0);
+  else sliceTasks<false>(c, p, -1, 0);
+#endif
   __syncthreads();
 }
 __device__ __forceinline__ void sliceProducts(Ctx& c, int what, const double* x, const double* z, double* px, void* atz,
@@ -940,7 +951,7 @@ static __device__ __forceinline__ bool gridFailed(GridCtl* g) {
 static __device__ __forceinline__ void gridProductsShare(GridCtl* g) {
   if (blockIdx.x > 0) {
     const int ctas = (int)gridDim.x - 1, w = threadIdx.x >> 5;
-    sliceTasks(g->ctx, g->prod, (int)blockIdx.x - 1 + ctas * w, ctas * (int)(blockDim.x >> 5));
+    sliceTasks<false>(g->ctx, g->prod, (int)blockIdx.x - 1 + ctas * w, ctas * (int)(blockDim.x >> 5));
   }
 }
 static __device__ bool gridProductsPost(Ctx& c, const ProductJob& p) {
@@ -3241,11 +3252,12 @@ static __device__ void setupCtx(Ctx& c, const LaunchArgs& a, int inst, unsigned 
   c.Pu = scratch + D.sPv;
   c.Pv = c.Pu + D.nnzPu;
   c.Av = scratch + D.sAv;
-  c.Avc = c.Av + D.nnzA;
-  c.Avr = c.Avc + D.nnzA;
-  c.sP = {c.Pv, I + D.iPsCol, I + D.iPsRow, I + D.iPsPerm, D.n};
-  c.sAc = {c.Avc, I + D.iAcCol, I + D.iAcRow, I + D.iAcPerm, D.n};
-  c.sAr = {c.Avr, I + D.iArCol, I + D.iArRow, I + D.iArPerm, D.m};
+  c.gather = a.gatherA != 0;
+  c.Avc = c.gather ? c.Av : scratch + D.sAc;
+  c.Avr = c.gather ? c.Av : c.Avc + D.nnzA;
+  c.sP = {c.Pv, I + D.iPsCol, I + D.iPsRow, I + D.iPsPerm, D.n, nullptr};
+  c.sAc = {c.Avc, I + D.iAcCol, I + D.iAcRow, I + D.iAcPerm, D.n, I + D.iAcSrc};
+  c.sAr = {c.Avr, I + D.iArCol, I + D.iArRow, I + D.iArPerm, D.m, I + D.iArSrc};
   c.Ad = scratch + D.sAd;
   c.T = scratch + D.sT;
   c.qs = scratch + D.sQ;

@@ -96,6 +96,7 @@ struct LaunchArgs {
   int traceRows;
   double* scratch;        // gridDim.x * scratchStride doubles
   int64_t scratchStride;
+  int gatherA = 0;        // scratch holds no copies of A in slice order (batched forms; Ctx::gather)
   int sumThreads;         // threads whose sums the block has (<= block size; FOR_V)
   // this launch may begin while the one before it in the stream runs, once all of that one's CTAs are
   // resident (programmatic stream serialisation): the size buckets of a batch

@@ -86,13 +86,15 @@ struct InstanceDesc {
   int64_t vPx, vQ, vAx, vB;           // user values (P upper CSC order, q, A CSC order, b)
   int64_t vX, vS, vZ;                 // outputs: x at vQ-like offset (n), s/z at vB-like offset (m)
   // per-instance FP64 scratch offsets (relative to the CTA's scratch base)
-  int64_t sPv, sAv, sAd, sT, sQ, sB;  // scaled P (user order, then slice order), scaled A (CSC order, then
-                                      // by columns and by rows in slice order), Ad, T, q, b
+  int64_t sPv, sAv, sAd, sT, sQ, sB;  // scaled P (user order, then slice order), scaled A (CSC order), Ad,
+                                      // T, q, b
   int64_t sRoot64;                    // FP64 root (fallback / FP64 precision when not in SMEM)
   int64_t sVec;                       // FP64 vectors that do not fit in shared memory
   int64_t sVecG;                      // FP64 vectors always kept in scratch (vecGlobalDoubles)
   int64_t sKry;                       // whole-GPU form: the GMRES Krylov area (krylovDoubles)
   int64_t sSlice;                     // whole-GPU mixed form: the double-float panel slices (dfSliceBytes)
+  int64_t sAc;                        // scaled A by columns, then by rows, in slice order; after all the
+                                      // rest, so that a CTA can do without them (LaunchArgs::gatherA)
   int64_t scratchDoubles;             // total per-CTA scratch this instance needs
   int64_t bwdOff;                     // offset of this instance's saved final state (differentiable)
   double cost;                        // scheduling weight (~ nr^3)
