@@ -3314,8 +3314,10 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) ipmKernel(LaunchArgs 
     loadInstance(c, a);
     solveInstance<FT>(c, a, inst);
   }
-  // what follows the last bucket in the stream must find all of them finished
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // What follows the last bucket in the stream must find all of them finished: a launch ends when its
+  // first CTA has seen the one before it end, and so the last one after all. The other CTAs leave, so
+  // that other streams have their SMs.
+  if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Whole-GPU form for one large instance (a.grid set): a cooperative launch with one CTA per SM.
