@@ -247,9 +247,12 @@ __device__ __forceinline__ int tileLeafPanel(T* A, int b, int J, int nr, int nx,
   __syncwarp();
   if (c0 + 8 < 32) {
     const bool below = r >= c0 + 8;
+    // rows not below: the leaf's last one, without use (their own entries are those that the other warps
+    // write meanwhile, tileInverseSum)
+    const int ru = below ? r : c0 + 7;
     T u[8];
 #pragma unroll
-    for (int t = 0; t < 8; ++t) u[t] = A[(c0 + t) * kTileLd + r];  // rows above: not stored
+    for (int t = 0; t < 8; ++t) u[t] = A[(c0 + t) * kTileLd + ru];
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
 #pragma unroll
@@ -322,9 +325,10 @@ __device__ __forceinline__ int tileLeafPanel(df64* A, int b, int J, int nr, int 
   if (leaf) invD[r] = invMine;
   __syncwarp();
   if (c0 + 8 < 32) {
+    const int ru = r >= c0 + 8 ? r : c0 + 7;  // as above
     df64 u[8];
 #pragma unroll
-    for (int t = 0; t < 8; ++t) u[t] = A[(c0 + t) * kTileLd + r];  // rows above: not stored
+    for (int t = 0; t < 8; ++t) u[t] = A[(c0 + t) * kTileLd + ru];
     dfPanelSteps<7>(u, A, c0, 0, invD);
     dfPanelSteps<3>(u, A, c0, 4, invD);
   }
