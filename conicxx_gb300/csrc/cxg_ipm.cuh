@@ -2116,7 +2116,10 @@ static __device__ __forceinline__ int waitTiles(GridCtl* g, const int* flags, in
     if (in) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(flags + mine) : "memory");
     const unsigned open = ~__ballot_sync(0xffffffffu, v == epoch);
     const int ready = open ? __ffs(open) - 1 : 32;
-    if (ready > 0) return ready;
+    if (ready > 0) {
+      __syncwarp();  // what one lane's flag opens, the others read
+      return ready;
+    }
     if ((spin & 63) == 63) {
       volatile GridCtl* vg = g;
       const unsigned long long now = globalNs();
