@@ -198,12 +198,12 @@ extern "C" int cxg_equilibration(const cxg_problem* pr, const cxg_settings* st, 
   return CXG_OK;
 }
 
-extern "C" int cxg_dense_ldlt(int nr, int nx, const double* K, const double* b, int arith, int threads,
-                              int linear_solver, double* L, double* D, double* x, long long* cycles, int* flags) {
+// threads > 0: one CTA; else the whole-GPU form on `ctas` CTAs (0: every SM's).
+static int denseLdltProbe(int nr, int nx, const double* K, const double* b, int arith, int threads, int ctas,
+                          int linear_solver, double* L, double* D, double* x, long long* cycles, int* flags) {
   using namespace cxg;
-  const bool whole = threads == -1;
-  if (nr < 1 || nx < 0 || nx > nr || !K || !b || arith < 0 || arith > 2 ||
-      (!whole && (threads < 32 || threads > 256 || (threads % 32) != 0))) {
+  const bool whole = threads <= 0;
+  if (nr < 1 || nx < 0 || nx > nr || !K || !b || arith < 0 || arith > 2) {
     lastErrorRef() = "cxg_dense_ldlt: bad arguments";
     return CXG_E_INVALID;
   }
@@ -242,7 +242,8 @@ extern "C" int cxg_dense_ldlt(int nr, int nx, const double* K, const double* b, 
   }
   DG_CUDA(cudaMemcpy(dK, K, nn * 8, cudaMemcpyHostToDevice));
   DG_CUDA(cudaMemcpy(dB, b, (size_t)nr * 8, cudaMemcpyHostToDevice));
-  DG_CUDA(launchDenseProbe(arith, nr, nx, dK, dB, st, threads, dL, dD, dX, dC, dF));
+  if (whole) DG_CUDA(launchDenseProbeGrid(arith, nr, nx, dK, dB, st, ctas, dL, dD, dX, dC, dF));
+  else DG_CUDA(launchDenseProbe(arith, nr, nx, dK, dB, st, threads, dL, dD, dX, dC, dF));
   DG_CUDA(cudaDeviceSynchronize());
   if (L) DG_CUDA(cudaMemcpy(L, dL, nn * 8, cudaMemcpyDeviceToHost));
   if (D) DG_CUDA(cudaMemcpy(D, dD, (size_t)nr * 8, cudaMemcpyDeviceToHost));
@@ -251,6 +252,25 @@ extern "C" int cxg_dense_ldlt(int nr, int nx, const double* K, const double* b, 
   if (flags) DG_CUDA(cudaMemcpy(flags, dF, (whole ? 3 : 2) * sizeof(int), cudaMemcpyDeviceToHost));
   for (void* p : bufs) cudaFree(p);
   return CXG_OK;
+}
+
+extern "C" int cxg_dense_ldlt(int nr, int nx, const double* K, const double* b, int arith, int threads,
+                              int linear_solver, double* L, double* D, double* x, long long* cycles, int* flags) {
+  if (threads != -1 && (threads < 32 || threads > 256 || (threads % 32) != 0)) {
+    lastErrorRef() = "cxg_dense_ldlt: bad arguments";
+    return CXG_E_INVALID;
+  }
+  return denseLdltProbe(nr, nx, K, b, arith, threads, 0, linear_solver, L, D, x, cycles, flags);
+}
+
+extern "C" int cxg_dense_ldlt_grid(int nr, int nx, const double* K, const double* b, int arith, int ctas,
+                                   int linear_solver, double* L, double* D, double* x, long long* nanoseconds,
+                                   int* flags) {
+  if (ctas < 0 || ctas == 1) {
+    lastErrorRef() = "cxg_dense_ldlt_grid: bad arguments";
+    return CXG_E_INVALID;
+  }
+  return denseLdltProbe(nr, nx, K, b, arith, -1, ctas, linear_solver, L, D, x, nanoseconds, flags);
 }
 
 extern "C" int cxg_grid_barrier_selftest(int skip_cta, int rounds, double timeout_s, int* error_flag,

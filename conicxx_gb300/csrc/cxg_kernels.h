@@ -132,5 +132,9 @@ cudaError_t launchGridBarrierTest(int skip, int rounds, double timeoutS, int* er
                                   double* elapsedS);
 cudaError_t launchDenseProbe(int arith, int nr, int nx, const double* K, const double* b, const DevSettings& st,
                              int threads, double* L, double* D, double* x, long long* cyc, int* flags);
+// The same by the whole-GPU form on `ctas` CTAs (0: every SM's): nanoseconds, and a third flag, 1 if a
+// wait ran out (2 s).
+cudaError_t launchDenseProbeGrid(int arith, int nr, int nx, const double* K, const double* b, const DevSettings& st,
+                                 int ctas, double* L, double* D, double* x, long long* cyc, int* flags);
 
 }  // namespace cxg

@@ -323,6 +323,12 @@ int cxg_cones_eval(int op, int zero_dim, int nonneg_dim, int n_soc, const int* s
 int cxg_dense_ldlt(int nr, int nx, const double* K, const double* b, int arith, int threads, int linear_solver,
                    double* L, double* D, double* x, long long* cycles, int* flags);
 
+/* The whole-GPU form of cxg_dense_ldlt (threads = -1) on `ctas` CTAs, 2 .. the SMs (0: all): with few of them
+ * a small matrix takes the paths of one that is too large for every SM's warps at once. CXG_E_CUDA with
+ * more CTAs than the device holds. */
+int cxg_dense_ldlt_grid(int nr, int nx, const double* K, const double* b, int arith, int ctas, int linear_solver,
+                        double* L, double* D, double* x, long long* nanoseconds, int* flags);
+
 /* Diagnostic, no reference counterpart: the bounded wait of the whole-GPU root's grid barrier.
  * One cooperative launch of one CTA per SM passes `rounds` grid barriers; when skip_cta >= 0 that
  * CTA returns without arriving, so the others' first wait runs out after timeout_s (1e-3..5 s),
