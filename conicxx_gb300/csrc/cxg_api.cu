@@ -150,8 +150,9 @@ struct cxg_batch {
   int* dCounters = nullptr;
   int* dOrder = nullptr;
   cudaStream_t stream = nullptr;
-  std::vector<cudaStream_t> groupStreams;   // one per size bucket (forked inside the graph)
-  std::vector<cudaEvent_t> forkJoin;        // fork event + one join event per bucket
+  std::vector<cudaStream_t> groupStreams;   // the adjoint's, one per size bucket (ensureAdjointStreams)
+  std::vector<cudaEvent_t> forkJoin;        // the adjoint's: fork event + one join event per bucket
+  bool solved = false;                      // a solve other than the allocation-free one has been enqueued
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graphExec = nullptr;
   DevSettings graphSettings{};
@@ -1091,17 +1092,11 @@ static int enqueueReorder(cxg_batch* B, cudaStream_t s) {
   return CXG_OK;
 }
 
-// Enqueues the device-side solve sequence on `s`: queue resets, then one persistent launch per
-// size bucket, each allowed to start while those before it run, so the buckets run concurrently and
-// the batch waits for its slowest instance once rather than once per bucket; then the queues are
-// re-ordered for the next solve (history-ordered queues, above).
-static int enqueueSolve(cxg_batch* B, cudaStream_t s) {
-  const DevSettings ds = makeDevSettings(B->st, B->kktSt);
-  CX_CUDA(cudaMemsetAsync(B->dCounters, 0, sizeof(int) * (B->groups.size() + 1), s));
+// Streams and events of the adjoint's launches: one stream per launch rank, the first the highest priority
+// (the block scheduler dispatches pending CTAs by stream priority, so that their placement follows
+// enqueueAdjoint's launch order), and an event to fork from and one per bucket to join.
+static int ensureAdjointStreams(cxg_batch* B) {
   const size_t G = B->groups.size();
-  // one stream per launch rank, the first the highest priority: the block scheduler dispatches
-  // pending CTAs by stream priority, so the placement follows the launch order below even where
-  // the graph submits its independent launches in another order
   if (B->groupStreams.size() < G) {
     int least = 0, greatest = 0;
     CX_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
@@ -1118,6 +1113,17 @@ static int enqueueSolve(cxg_batch* B, cudaStream_t s) {
     CX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     B->forkJoin.push_back(e);
   }
+  return CXG_OK;
+}
+
+// Enqueues the device-side solve sequence on `s`: queue resets, then one persistent launch per
+// size bucket, each allowed to start while those before it run, so the buckets run concurrently and
+// the batch waits for its slowest instance once rather than once per bucket; then the queues are
+// re-ordered for the next solve (history-ordered queues, above).
+static int enqueueSolve(cxg_batch* B, cudaStream_t s) {
+  const DevSettings ds = makeDevSettings(B->st, B->kktSt);
+  CX_CUDA(cudaMemsetAsync(B->dCounters, 0, sizeof(int) * (B->groups.size() + 1), s));
+  const size_t G = B->groups.size();
   if (B->gridMode) {
     const Group& g = B->groups[0];
     CX_CUDA(cudaMemsetAsync(B->dGridCtl, 0, gridCtlBytes(), s));
@@ -1154,7 +1160,11 @@ static int enqueueSolve(cxg_batch* B, cudaStream_t s) {
 // Device-side solve through the captured graph (re-captured when the settings change).
 static int runSolve(cxg_batch* B, cudaStream_t s) {
   if (int rc = ensureTrace(B)) return rc;
+  // here, so that a backward call on a stream under capture creates none
+  if (B->dBwd)
+    if (int rc = ensureAdjointStreams(B)) return rc;
   B->bwdStale = false;
+  B->solved = true;
   // the whole-GPU form is one cooperative launch: enqueued directly, not through a graph
   if (B->gridMode) return enqueueSolve(B, s);
   const DevSettings ds = makeDevSettings(B->st, B->kktSt);
@@ -1169,7 +1179,7 @@ static int runSolve(cxg_batch* B, cudaStream_t s) {
     if (rc) { if (g) cudaGraphDestroy(g); return rc; }
     if (ce != cudaSuccess) return setErr(CXG_E_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
     B->graph = g;
-    CX_CUDA(cudaGraphInstantiate(&B->graphExec, B->graph, cudaGraphInstantiateFlagUseNodePriority));
+    CX_CUDA(cudaGraphInstantiate(&B->graphExec, B->graph, 0));
     B->graphSettings = ds;
     B->graphValid = true;
   }
@@ -1622,9 +1632,12 @@ extern "C" int cxg_solver_backward(cxg_solver* S, const double* dL_dx, double* d
 
 extern "C" int cxg_batch_backward(cxg_batch* B, const double* dL_dx, double* dq, double* db, double* dPx, double* dAx);
 
-// Enqueues the adjoint of every instance (one launch per size bucket, forked like the solve).
+// Enqueues the adjoint of every instance: one launch per size bucket, each on its own stream forked from
+// and joined back into `s`.
 static int enqueueAdjoint(cxg_batch* B, cudaStream_t s, const double* gx, double* gq, double* gb, double* gP,
                           double* gA) {
+  // more buckets since the last solve (cxg_batch_replace, then the allocation-free solve) want more streams
+  if (int rc = ensureAdjointStreams(B)) return rc;
   const DevSettings ds = makeDevSettings(B->st, B->kktSt);
   CX_CUDA(cudaMemsetAsync(B->dCounters, 0, sizeof(int) * (B->groups.size() + 1), s));
   const size_t G = B->groups.size();
@@ -1680,7 +1693,7 @@ static int checkDifferentiable(cxg_batch* B) {
   if (!B->dBwd && B->bwdDropped)
     return setErr(CXG_E_UNSUPPORTED, "backward is offered up to 8192 root rows on the whole-GPU root");
   if (!B->dBwd) return setErr(CXG_E_NOT_SETUP, "backward needs settings.differentiable = 1 at set-up");
-  if (B->forkJoin.empty()) return setErr(CXG_E_NOT_SETUP, "backward before any solve");
+  if (!B->solved) return setErr(CXG_E_NOT_SETUP, "backward before any solve");
   if (B->bwdStale) return setErr(CXG_E_NOT_SETUP, "backward after cxg_batch_replace needs a solve first");
   return CXG_OK;
 }
