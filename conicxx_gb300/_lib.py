@@ -59,6 +59,7 @@ SIGNATURES = {
     "cxg_batch_describe": (C.c_int, [vp, C.c_char_p, C.c_int]),
     "cxg_batch_footprint": (C.c_int, [vp, i64p, i64p, i64p]),
     "cxg_cones_eval": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, ip, dp, dp, dp, dp, C.c_double, dp, dp, dp]),
+    "cxg_soc_ladder_eval": (C.c_int, [C.c_int, C.c_int, dp, dp, C.c_double, C.c_double, C.c_double, C.c_int, ip]),
     "cxg_equilibration": (C.c_int, [PP, SP, dp, dp, dp]),
     "cxg_plan_inspect": (C.c_int, [PP, SP, i64p, i64p, i64p, i64p, C.c_int]),
 }

@@ -528,14 +528,19 @@ static __device__ __noinline__ int socRefLadderDim(const double* s, const double
   return kLadderLevels;
 }
 
-__device__ __forceinline__ int socRefLadderLevel(const double* s, const double* z, int d, double sregA, double deps,
+__device__ __forceinline__ int socRefLadderExact(const double* s, const double* z, int d, double sregA, double deps,
                                                  double delta, int startLevel) {
-  if (d > kRefDenseMaxDim || d < 2) return 0;
-  if (socPivotsPass(s, z, d, sregA, deps)) return startLevel;
   if (d == 2) return socRefLadderDim<2>(s, z, d, sregA, deps, delta, startLevel);
   if (d == 3) return socRefLadderDim<3>(s, z, d, sregA, deps, delta, startLevel);
   if (d == 4) return socRefLadderDim<4>(s, z, d, sregA, deps, delta, startLevel);
   return socRefLadderDim<0>(s, z, d, sregA, deps, delta, startLevel);
+}
+
+__device__ __forceinline__ int socRefLadderLevel(const double* s, const double* z, int d, double sregA, double deps,
+                                                 double delta, int startLevel) {
+  if (d > kRefDenseMaxDim || d < 2) return 0;
+  if (socPivotsPass(s, z, d, sregA, deps)) return startLevel;
+  return socRefLadderExact(s, z, d, sregA, deps, delta, startLevel);
 }
 
 __device__ __forceinline__ double socMargin(const double* x, int d) {

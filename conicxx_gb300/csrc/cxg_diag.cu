@@ -96,6 +96,19 @@ __global__ void coneEvalKernel(int op, int zero, int nn, int nsoc, const int* of
   }
 }
 
+// Per block: the ladder level as the iteration takes it, the level from the dense pivots themselves, and
+// whether the bound let the block through.
+__global__ void socLadderKernel(int count, int dim, const double* s, const double* z, double sregA, double deps,
+                                double delta, int start, int* out) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= count) return;
+  s += (int64_t)b * dim;
+  z += (int64_t)b * dim;
+  out[3 * b] = socRefLadderLevel(s, z, dim, sregA, deps, delta, start);
+  out[3 * b + 1] = socRefLadderExact(s, z, dim, sregA, deps, delta, start);
+  out[3 * b + 2] = socPivotsPass(s, z, dim, sregA, deps) ? 1 : 0;
+}
+
 }  // namespace cxg
 
 using namespace cxg;
@@ -175,6 +188,33 @@ extern "C" int cxg_cones_eval(int op, int zero_dim, int nonneg_dim, int n_soc, c
   if (out) DG_CUDA(cudaMemcpy(out, dO, sizeof(double) * (size_t)m, cudaMemcpyDeviceToHost));
   if (scalars) DG_CUDA(cudaMemcpy(scalars, dSc, sizeof(double) * 2, cudaMemcpyDeviceToHost));
   if (soc_params && n_soc) DG_CUDA(cudaMemcpy(soc_params, dP, sizeof(double) * 8 * (size_t)n_soc, cudaMemcpyDeviceToHost));
+  for (void* p : bufs) cudaFree(p);
+  return CXG_OK;
+}
+
+extern "C" int cxg_soc_ladder_eval(int count, int dim, const double* s, const double* z, double static_reg_A,
+                                   double dynamic_reg_eps, double dynamic_reg_delta, int start_level, int* levels) {
+  if (count < 1 || dim < 2 || dim > kRefDenseMaxDim || !s || !z || !levels || start_level < 0 ||
+      start_level >= kLadderLevels) {
+    lastErrorRef() = "cxg_soc_ladder_eval: bad arguments";
+    return CXG_E_INVALID;
+  }
+  std::vector<void*> bufs;
+  const size_t bytes = sizeof(double) * (size_t)count * (size_t)dim;
+  void *dS = nullptr, *dZ = nullptr, *dL = nullptr;
+  DG_CUDA(cudaMalloc(&dS, bytes));
+  bufs.push_back(dS);
+  DG_CUDA(cudaMalloc(&dZ, bytes));
+  bufs.push_back(dZ);
+  DG_CUDA(cudaMalloc(&dL, sizeof(int) * 3 * (size_t)count));
+  bufs.push_back(dL);
+  DG_CUDA(cudaMemcpy(dS, s, bytes, cudaMemcpyHostToDevice));
+  DG_CUDA(cudaMemcpy(dZ, z, bytes, cudaMemcpyHostToDevice));
+  socLadderKernel<<<(count + 127) / 128, 128>>>(count, dim, (const double*)dS, (const double*)dZ, static_reg_A,
+                                                dynamic_reg_eps, dynamic_reg_delta, start_level, (int*)dL);
+  DG_CUDA(cudaGetLastError());
+  DG_CUDA(cudaDeviceSynchronize());
+  DG_CUDA(cudaMemcpy(levels, dL, sizeof(int) * 3 * (size_t)count, cudaMemcpyDeviceToHost));
   for (void* p : bufs) cudaFree(p);
   return CXG_OK;
 }

@@ -309,6 +309,11 @@ int cxg_batch_describe(const cxg_batch* batch, char* buf, int buflen);
 int cxg_cones_eval(int op, int zero_dim, int nonneg_dim, int n_soc, const int* soc_dims, const double* s,
                    const double* z, const double* u, const double* v, double alpha_or_eps, double* out,
                    double* scalars, double* soc_params);
+/* The regularisation ladder's level of `count` second-order blocks of `dim` rows (2..8; s, z: count x dim), with
+ * the settings given, from start_level on: levels[3 b] as the iteration takes it, [3 b + 1] from the dense
+ * pivots of the block (kkt_system.cpp:152-168, 242-264), [3 b + 2] = 1 where a bound spares the pivots. */
+int cxg_soc_ladder_eval(int count, int dim, const double* s, const double* z, double static_reg_A,
+                        double dynamic_reg_eps, double dynamic_reg_delta, int start_level, int* levels);
 /* Dense root factorisation of the IPM kernel (the reduced KKT root's LDL', QDLDL-style no
  * pivoting with the per-pivot rule of RegularizedLdlt::regularizePivot when linear_solver is
  * CXG_LINSOLVER_REGULARIZED, src/conicxx/kkt/regularized_ldlt.cpp:132-139) on one given dense
