@@ -233,6 +233,11 @@ static const int kBucketEdges[] = {32, 64, 96, 128, 192, 256, 384, 512, 1024, 20
 // every SM (whole_gpu_root = 0), which accepts up to kGridMaxRoot rows. The plan's root scatter
 // maps hold 64-bit element offsets; a 131072-row root is 8.86e9 entries (71 GB of 8-byte
 // entries), and the host planner and tile indices stay within 32 bits up to there.
+// kGridAutoRoot was the crossover of both forms in FP64 with earlier kernels. Now the whole-GPU form is
+// the faster one from about 190 rows in FP64 (192 rows 10.7 against 11.4 ms a solve, 512 rows 31.5 against
+// 140 ms) and from about 360 in mixed precision (320 rows 36.2 against 28.6 ms, 384 rows 34.1 against 42.8).
+// The line stays at 512: below it solves keep the one-CTA form's refinement and its bits, and the
+// other SMs stay free for other streams; whole_gpu_root = 1 asks for the other form.
 static const int kCtaMaxRoot = 4096;
 static const int kGridAutoRoot = 512;
 static const int kGridMaxRoot = 131072;

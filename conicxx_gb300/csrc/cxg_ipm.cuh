@@ -2094,9 +2094,11 @@ __device__ __noinline__ bool gridLdltSteps(GridCtl* g, int nr, int nx, const Dev
 // applies the solved tiles x_j to its rows in order (forward: j ascending, backward: descending), as
 // they are published, solves its own tile when its turn comes and publishes it: within the CTA
 // through shared memory, to the others in y with a flag per tile. Its tiles of the root arrive by
-// asynchronous copies, two ahead of the one in use. So a tile step costs one product and one diagonal
-// solve (about 0.5 us), and only every eighth one a hand-over between SMs; in blocks of four tiles
-// with a grid barrier each it was 17 us a block, mostly tiles read from L2 on the critical path.
+// asynchronous copies, two ahead of the one in use. So a tile step is one product and one diagonal
+// solve, and only every eighth one a hand-over between SMs. Measured a step: FP32 1.5 us, double-float
+// 2.9, FP64 3.4 (1020 rows, 2 x 32 steps: 94, 188 and 219 us; 6400 rows: 0.59, 1.14 and 1.37 ms), of
+// which a product's arithmetic is a small part; in blocks of four tiles with a grid barrier each it was
+// 17 us a block, mostly tiles read from L2 on the critical path.
 // Every y tile takes its updates one source tile at a time in the same order as before.
 constexpr int kSolveRows = 4;   // row tiles a warp owns at a time, at most
 constexpr int kSolveBufs = 3;   // tile buffers of a warp
